@@ -22,6 +22,7 @@ using namespace pic;
 
 constexpr double kFp32Unit = 0x1p-24;  // unit roundoff of FP32 round-to-nearest
 constexpr long kUploadChunk = 1l << 22;  // particles per upload staging round (256 MB)
+constexpr long kFieldChunk = 1l << 22;   // doubles per round of a node field's staging (32 MB)
 constexpr long kSortMovedFraction = 50;   // re-sort a species when 2 % of it left cell order
 
 namespace {
@@ -57,7 +58,7 @@ struct SpeciesHost {
     unsigned long long* id2 = nullptr;
     float* den = nullptr;
     float* den_avg = nullptr;
-    float* mom = nullptr;  // velocity moments, 7 node planes, allocated on first sampleMoments
+    float4* mom = nullptr;  // velocity moments, two float4 per node, allocated on first sampleMoments
     int avg_samples = 0;
     double scale = 1.0;  // fixed-point scale of the density accumulator
     unsigned long long next_id = 0;
@@ -945,6 +946,15 @@ int ensure_upload(pic_world* w, long n) {
     }
     return PIC_OK;
 }
+// the same buffer as FP64 staging of node fields, per_node doubles a node: *nodes of it fit (at most
+// kFieldChunk doubles are used)
+int ensure_field_stage(pic_world* w, int per_node, int* nodes) {
+    const long vals = std::min<long>(kFieldChunk, (long)w->g.nv * per_node);
+    int rc = ensure_upload(w, (vals + 7) / 8);
+    if (rc) return rc;
+    *nodes = (int)(std::min<long>(kFieldChunk, w->upload_cap * 8) / per_node);
+    return PIC_OK;
+}
 }  // namespace
 
 // a pointer the world's device can dereference: its own device memory, or pinned host memory
@@ -1355,8 +1365,8 @@ extern "C" int pic_species_sample_moments(pic_world* w, int sp) {
     CU(cudaSetDevice(w->device));
     SpeciesHost& s = w->sp[sp];
     if (!s.mom) {
-        CU(cudaMalloc((void**)&s.mom, sizeof(float) * 7 * (size_t)w->g.nv));
-        CU(cudaMemsetAsync(s.mom, 0, sizeof(float) * 7 * (size_t)w->g.nv, w->stream));
+        CU(cudaMalloc((void**)&s.mom, sizeof(float4) * 2 * (size_t)w->g.nv));
+        CU(cudaMemsetAsync(s.mom, 0, sizeof(float4) * 2 * (size_t)w->g.nv, w->stream));
     }
     {
         Scope sc(w, "moments", 1);
@@ -1370,40 +1380,36 @@ extern "C" int pic_species_clear_samples(pic_world* w, int sp) {
     if (!valid_sp(w, sp)) return fail(PIC_ERR_ARG, "bad species");
     CU(cudaSetDevice(w->device));
     SpeciesHost& s = w->sp[sp];
-    if (s.mom) CU(cudaMemsetAsync(s.mom, 0, sizeof(float) * 7 * (size_t)w->g.nv, w->stream));
+    if (s.mom) CU(cudaMemsetAsync(s.mom, 0, sizeof(float4) * 2 * (size_t)w->g.nv, w->stream));
     return PIC_OK;
 }
 
-// Species::computeGasProperties (Species.cpp:777-804): vel = nv/n, T = m/(2k) (var_u + var_v + var_w)
+// Species::computeGasProperties (Species.cpp:777-804): vel = nv/n, T = m/(2k) (var_u + var_v + var_w),
+// formed on the device in FP64, a staging buffer of nodes at a time
 extern "C" int pic_species_gas_properties(pic_world* w, int sp, double* vel, double* T) {
     if (!valid_sp(w, sp)) return fail(PIC_ERR_ARG, "bad species");
     CU(cudaSetDevice(w->device));
     SpeciesHost& s = w->sp[sp];
     const int nv = w->g.nv;
-    std::vector<float> m((size_t)7 * nv, 0.f);
-    if (s.mom) {
-        CU(cudaMemcpyAsync(m.data(), s.mom, sizeof(float) * 7 * (size_t)nv, cudaMemcpyDeviceToHost, w->stream));
-        CU(cudaStreamSynchronize(w->stream));
+    if (!s.mom) {  // nothing sampled
+        if (vel) std::fill(vel, vel + 3 * (size_t)nv, 0.0);
+        if (T) std::fill(T, T + nv, 0.0);
+        return PIC_OK;
     }
-    for (int n = 0; n < nv; n++) {
-        double cnt = m[n];
-        double u = cnt > 0 ? m[(size_t)nv + n] / cnt : 0, v = cnt > 0 ? m[(size_t)2 * nv + n] / cnt : 0,
-               ww = cnt > 0 ? m[(size_t)3 * nv + n] / cnt : 0;
-        if (vel) {
-            vel[3 * n] = u;
-            vel[3 * n + 1] = v;
-            vel[3 * n + 2] = ww;
+    int cap = 0;
+    int rc = ensure_field_stage(w, 4, &cap);
+    if (rc) return rc;
+    double *dv = w->upload_buf, *dt = dv + 3 * (size_t)cap;
+    for (int a = 0; a < nv; a += cap) {
+        const int m = std::min(cap, nv - a);
+        {
+            Scope sc(w, "moments", 1);
+            launch_gas_properties(s.mom, a, m, s.mass / (2 * kKb), vel ? dv : nullptr, T ? dt : nullptr, w->stream);
         }
-        if (T) {
-            if (cnt <= 0) {
-                T[n] = 0;
-                continue;
-            }
-            double uu = m[(size_t)4 * nv + n] / cnt - u * u, vv = m[(size_t)5 * nv + n] / cnt - v * v,
-                   wq = m[(size_t)6 * nv + n] / cnt - ww * ww;
-            T[n] = s.mass / (2 * kKb) * (uu + vv + wq);
-        }
+        if (vel) CU(cudaMemcpyAsync(vel + 3 * (size_t)a, dv, sizeof(double) * 3 * m, cudaMemcpyDeviceToHost, w->stream));
+        if (T) CU(cudaMemcpyAsync(T + a, dt, sizeof(double) * m, cudaMemcpyDeviceToHost, w->stream));
     }
+    CU(cudaStreamSynchronize(w->stream));
     return PIC_OK;
 }
 

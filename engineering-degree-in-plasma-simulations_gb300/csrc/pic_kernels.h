@@ -136,7 +136,11 @@ struct DsmcArgs {
 };
 void launch_dsmc(const DsmcArgs& a, cudaStream_t s);
 void launch_sums(SpeciesDev sp, double* out, cudaStream_t s, int grid);
-void launch_sample_moments(const GridDev& g, SpeciesDev sp, float* mom, cudaStream_t s, int grid);
+void launch_sample_moments(const GridDev& g, SpeciesDev sp, float4* mom, cudaStream_t s, int grid);
+// mean velocity (3 per node) and temperature of nodes first .. first + m - 1 from the sampled moments
+// (null outputs are skipped)
+void launch_gas_properties(const float4* mom, int first, int m, double t_scale, double* vel, double* T,
+                           cudaStream_t s);
 void launch_merge(const GridDev& g, SpeciesDev sp, const float4* ef, const int* cell_start, int* list, int* nlist,
                   int min_count, float qm_half_dt, uint2 key, unsigned step, unsigned* err,
                   unsigned long long* stats, cudaStream_t s, int grid);
