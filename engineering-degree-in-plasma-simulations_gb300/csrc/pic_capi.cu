@@ -10,7 +10,9 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
+#include <unistd.h>
 #include <vector>
 #include "../../include/pic_gb300.h"
 #include "pic_kernels.h"
@@ -152,6 +154,7 @@ struct pic_world {
     double time = 0.0;
     double* upload_buf = nullptr;  // particle upload staging (upload_cap particles, at most kUploadChunk)
     long upload_cap = 0;
+    std::mutex stage_mutex;  // held from the first to the last enqueued use of upload_buf in a call
     // bound on the 2-norm of the rounding error of the FP32 residual r (valid with rhs_valid)
     double r_err = 0.0;
     // solver
@@ -772,20 +775,88 @@ extern "C" int pic_world_set_slabs(pic_world* w, int nslabs, const double* phi_l
     return upload_kinds(w, false);
 }
 
+namespace {
+// the particle upload staging buffer holds at least min(n, kUploadChunk) particles; the caller holds
+// stage_mutex while it uses the buffer, so that calls on other host threads keep theirs apart
+int ensure_upload(pic_world* w, long n) {
+    const long want = std::min<long>(kUploadChunk, n);
+    if (w->upload_cap < want) {
+        if (w->upload_buf) CU(cudaFree(w->upload_buf));
+        w->upload_buf = nullptr;
+        w->upload_cap = 0;
+        CU(cudaMalloc(&w->upload_buf, (size_t)want * 8 * sizeof(double)));
+        w->upload_cap = want;
+    }
+    return PIC_OK;
+}
+// the same buffer as FP64 staging of node fields, per_node doubles a node: *nodes of it fit (at most
+// kFieldChunk doubles are used)
+int ensure_field_stage(pic_world* w, int per_node, int* nodes) {
+    const long vals = std::min<long>(kFieldChunk, (long)w->g.nv * per_node);
+    int rc = ensure_upload(w, (vals + 7) / 8);
+    if (rc) return rc;
+    *nodes = (int)(std::min<long>(kFieldChunk, w->upload_cap * 8) / per_node);
+    return PIC_OK;
+}
+// Device bytes to the caller's array, whose every page is written to first: a copy into an untouched
+// allocation faults page by page from the copy's side, which took between 0.08 and 6.6 ms for 8 MB from
+// call to call, against 0.05 ms into touched pages and about 0.25 ms for the faults on the host.  (A
+// read before the write would map the shared zero page first and then replace it, which costs a
+// translation shootdown per page: measured 20 us each.)
+int copy_out(pic_world* w, void* out, const void* dev, size_t bytes) {
+    static const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
+    volatile char* p = static_cast<volatile char*>(out);
+    for (size_t x = 0; x < bytes; x += page) p[x] = 0;
+    if (bytes) p[bytes - 1] = 0;
+    CU(cudaMemcpyAsync(out, dev, bytes, cudaMemcpyDeviceToHost, w->stream));
+    return PIC_OK;
+}
+// a node field of per_node doubles a node to the caller's array, from(first node, nodes, staging)
+// filling the staging buffer on the world's stream
+template <class F>
+int field_out(pic_world* w, int per_node, double* out, F from) {
+    std::lock_guard<std::mutex> lock(w->stage_mutex);
+    int cap = 0;
+    int rc = ensure_field_stage(w, per_node, &cap);
+    if (rc) return rc;
+    for (int a = 0; a < w->g.nv; a += cap) {
+        const int m = std::min(cap, w->g.nv - a);
+        from(a, m, w->upload_buf);
+        rc = copy_out(w, out + (size_t)per_node * a, w->upload_buf, sizeof(double) * per_node * m);
+        if (rc) return rc;
+    }
+    CU(cudaStreamSynchronize(w->stream));
+    return PIC_OK;
+}
+// and from the caller's array, to(first node, nodes, staging) reading the staging buffer
+template <class F>
+int field_in(pic_world* w, int per_node, const double* in, F to) {
+    std::lock_guard<std::mutex> lock(w->stage_mutex);
+    int cap = 0;
+    int rc = ensure_field_stage(w, per_node, &cap);
+    if (rc) return rc;
+    for (int a = 0; a < w->g.nv; a += cap) {
+        const int m = std::min(cap, w->g.nv - a);
+        CU(cudaMemcpyAsync(w->upload_buf, in + (size_t)per_node * a, sizeof(double) * per_node * m,
+                           cudaMemcpyHostToDevice, w->stream));
+        to(a, m, w->upload_buf);
+    }
+    CU(cudaStreamSynchronize(w->stream));
+    CU(cudaGetLastError());
+    return PIC_OK;
+}
+}  // namespace
+
 extern "C" int pic_world_get_field(pic_world* w, int which, double* out) {
     if (!w || !out) return fail(PIC_ERR_ARG, "null argument");
     CU(cudaSetDevice(w->device));
     const GridDev& g = w->g;
     if (which == 0) {
-        std::vector<float2> t(g.nv);
-        CU(cudaMemcpyAsync(t.data(), w->phi, sizeof(float2) * g.nv, cudaMemcpyDeviceToHost, w->stream));
-        CU(cudaStreamSynchronize(w->stream));
-        for (int n = 0; n < g.nv; n++) out[n] = ff_to_double(t[n]);
+        int rc = field_out(w, 1, out, [&](int a, int m, double* st) { launch_phi_out(w->phi + a, m, st, w->stream); });
+        if (rc) return rc;
     } else if (which == 1) {
-        std::vector<float> t(g.nv);
-        CU(cudaMemcpyAsync(t.data(), w->rho, sizeof(float) * g.nv, cudaMemcpyDeviceToHost, w->stream));
-        CU(cudaStreamSynchronize(w->stream));
-        for (int n = 0; n < g.nv; n++) out[n] = t[n];
+        int rc = field_out(w, 1, out, [&](int a, int m, double* st) { launch_f32_out(w->rho + a, m, st, w->stream); });
+        if (rc) return rc;
     } else if (which == 2) {
         // World::computeNodeVolumes: half a cell per non-periodic face (of each stacked instance)
         const int nn[3] = {g.ni, g.nj, g.zslab ? g.zslab : g.nk};
@@ -824,14 +895,8 @@ extern "C" int pic_world_get_field(pic_world* w, int which, double* out) {
                     out[n] = id;
                 }
     } else if (which == 3) {
-        std::vector<float4> t(g.nv);
-        CU(cudaMemcpyAsync(t.data(), w->ef, sizeof(float4) * g.nv, cudaMemcpyDeviceToHost, w->stream));
-        CU(cudaStreamSynchronize(w->stream));
-        for (int n = 0; n < g.nv; n++) {
-            out[3 * n] = t[n].x;
-            out[3 * n + 1] = t[n].y;
-            out[3 * n + 2] = t[n].z;
-        }
+        int rc = field_out(w, 3, out, [&](int a, int m, double* st) { launch_ef_out(w->ef + a, m, st, w->stream); });
+        if (rc) return rc;
     } else {
         return fail(PIC_ERR_ARG, "unknown field %d", which);
     }
@@ -857,26 +922,15 @@ extern "C" int pic_world_potential_energy(pic_world* w, double* pe) {
 extern "C" int pic_world_set_field(pic_world* w, int which, const double* in) {
     if (!w || !in) return fail(PIC_ERR_ARG, "null argument");
     CU(cudaSetDevice(w->device));
-    const GridDev& g = w->g;
     if (which == 0) {
         w->rhs_valid = false;
-        std::vector<float2> t(g.nv);
-        for (int n = 0; n < g.nv; n++) t[n] = ff_pack(in[n]);
-        CU(cudaMemcpyAsync(w->phi, t.data(), sizeof(float2) * g.nv, cudaMemcpyHostToDevice, w->stream));
-        CU(cudaStreamSynchronize(w->stream));
-    } else if (which == 1) {
-        std::vector<float> t(in, in + g.nv);
-        CU(cudaMemcpyAsync(w->rho, t.data(), sizeof(float) * g.nv, cudaMemcpyHostToDevice, w->stream));
-        CU(cudaStreamSynchronize(w->stream));
-    } else if (which == 3) {
-        std::vector<float4> t(g.nv);
-        for (int n = 0; n < g.nv; n++) t[n] = make_float4((float)in[3 * n], (float)in[3 * n + 1], (float)in[3 * n + 2], 0.f);
-        CU(cudaMemcpyAsync(w->ef, t.data(), sizeof(float4) * g.nv, cudaMemcpyHostToDevice, w->stream));
-        CU(cudaStreamSynchronize(w->stream));
-    } else {
-        return fail(PIC_ERR_ARG, "field %d is not settable", which);
+        return field_in(w, 1, in, [&](int a, int m, const double* st) { launch_phi_in(st, m, w->phi + a, w->stream); });
     }
-    return PIC_OK;
+    if (which == 1)
+        return field_in(w, 1, in, [&](int a, int m, const double* st) { launch_f32_in(st, m, w->rho + a, w->stream); });
+    if (which == 3)
+        return field_in(w, 3, in, [&](int a, int m, const double* st) { launch_ef_in(st, m, w->ef + a, w->stream); });
+    return fail(PIC_ERR_ARG, "field %d is not settable", which);
 }
 
 // =====================================================================================
@@ -933,30 +987,6 @@ extern "C" int pic_species_create(pic_world* w, const char* name, double mass, d
     return PIC_OK;
 }
 
-namespace {
-// the particle upload staging buffer holds at least min(n, kUploadChunk) particles
-int ensure_upload(pic_world* w, long n) {
-    const long want = std::min<long>(kUploadChunk, n);
-    if (w->upload_cap < want) {
-        if (w->upload_buf) CU(cudaFree(w->upload_buf));
-        w->upload_buf = nullptr;
-        w->upload_cap = 0;
-        CU(cudaMalloc(&w->upload_buf, (size_t)want * 8 * sizeof(double)));
-        w->upload_cap = want;
-    }
-    return PIC_OK;
-}
-// the same buffer as FP64 staging of node fields, per_node doubles a node: *nodes of it fit (at most
-// kFieldChunk doubles are used)
-int ensure_field_stage(pic_world* w, int per_node, int* nodes) {
-    const long vals = std::min<long>(kFieldChunk, (long)w->g.nv * per_node);
-    int rc = ensure_upload(w, (vals + 7) / 8);
-    if (rc) return rc;
-    *nodes = (int)(std::min<long>(kFieldChunk, w->upload_cap * 8) / per_node);
-    return PIC_OK;
-}
-}  // namespace
-
 // a pointer the world's device can dereference: its own device memory, or pinned host memory
 // mapped into the unified address space (the kernel then reads it over the host link);
 // nullptr for pageable memory
@@ -1002,6 +1032,7 @@ extern "C" int pic_species_add_particles(pic_world* w, int sp, const double* pos
     }
     // through a reusable device staging buffer, kUploadChunk particles at a time (pos, vel, w and
     // ids in FP64 / u64); without ids the device numbers the particles from next_id on
+    std::lock_guard<std::mutex> lock(w->stage_mutex);
     int urc = ensure_upload(w, n);
     if (urc) return urc;
     const long cap = w->upload_cap;
@@ -1396,6 +1427,7 @@ extern "C" int pic_species_gas_properties(pic_world* w, int sp, double* vel, dou
         if (T) std::fill(T, T + nv, 0.0);
         return PIC_OK;
     }
+    std::lock_guard<std::mutex> lock(w->stage_mutex);
     int cap = 0;
     int rc = ensure_field_stage(w, 4, &cap);
     if (rc) return rc;
@@ -1406,8 +1438,8 @@ extern "C" int pic_species_gas_properties(pic_world* w, int sp, double* vel, dou
             Scope sc(w, "moments", 1);
             launch_gas_properties(s.mom, a, m, s.mass / (2 * kKb), vel ? dv : nullptr, T ? dt : nullptr, w->stream);
         }
-        if (vel) CU(cudaMemcpyAsync(vel + 3 * (size_t)a, dv, sizeof(double) * 3 * m, cudaMemcpyDeviceToHost, w->stream));
-        if (T) CU(cudaMemcpyAsync(T + a, dt, sizeof(double) * m, cudaMemcpyDeviceToHost, w->stream));
+        if (vel && (rc = copy_out(w, vel + 3 * (size_t)a, dv, sizeof(double) * 3 * m))) return rc;
+        if (T && (rc = copy_out(w, T + a, dt, sizeof(double) * m))) return rc;
     }
     CU(cudaStreamSynchronize(w->stream));
     return PIC_OK;
@@ -1446,11 +1478,9 @@ extern "C" int pic_charge_density(pic_world* w) {
 extern "C" int pic_species_get_den(pic_world* w, int sp, double* out) {
     if (!valid_sp(w, sp) || !out) return fail(PIC_ERR_ARG, "bad arguments");
     CU(cudaSetDevice(w->device));
-    std::vector<float> t(w->g.nv);
-    CU(cudaMemcpyAsync(t.data(), w->sp[sp].den, sizeof(float) * w->g.nv, cudaMemcpyDeviceToHost, w->stream));
-    CU(cudaStreamSynchronize(w->stream));
-    for (int n = 0; n < w->g.nv; n++) out[n] = t[n];
-    return check_device_error(w);
+    const float* den = w->sp[sp].den;
+    int rc = field_out(w, 1, out, [&](int a, int m, double* st) { launch_f32_out(den + a, m, st, w->stream); });
+    return rc ? rc : check_device_error(w);
 }
 
 extern "C" int pic_species_update_averages(pic_world* w, int sp) {
@@ -1471,11 +1501,8 @@ extern "C" int pic_species_update_averages(pic_world* w, int sp) {
 extern "C" int pic_species_get_den_avg(pic_world* w, int sp, double* out) {
     if (!valid_sp(w, sp) || !out) return fail(PIC_ERR_ARG, "bad arguments");
     CU(cudaSetDevice(w->device));
-    std::vector<float> t(w->g.nv);
-    CU(cudaMemcpyAsync(t.data(), w->sp[sp].den_avg, sizeof(float) * w->g.nv, cudaMemcpyDeviceToHost, w->stream));
-    CU(cudaStreamSynchronize(w->stream));
-    for (int n = 0; n < w->g.nv; n++) out[n] = t[n];
-    return PIC_OK;
+    const float* avg = w->sp[sp].den_avg;
+    return field_out(w, 1, out, [&](int a, int m, double* st) { launch_f32_out(avg + a, m, st, w->stream); });
 }
 
 namespace {
@@ -1500,13 +1527,10 @@ extern "C" int pic_species_sort(pic_world* w, int sp, int32_t* cell_counts) {
     sort_species(w, sp);
     CU(cudaGetLastError());
     if (cell_counts) {
-        // counts per cell = start[c+1] - start[c]; start has nc entries, the total is the count
-        std::vector<int> st(w->g.nc);
-        CU(cudaMemcpyAsync(st.data(), w->cell_start, sizeof(int) * w->g.nc, cudaMemcpyDeviceToHost, w->stream));
-        int n = 0;
-        CU(cudaMemcpyAsync(&n, w->sp[sp].dev.counts, sizeof(int), cudaMemcpyDeviceToHost, w->stream));
+        // the scatter's cursors end at the cell counts
+        int rc = copy_out(w, cell_counts, w->cell_count, sizeof(int) * w->g.nc);
+        if (rc) return rc;
         CU(cudaStreamSynchronize(w->stream));
-        for (int c = 0; c < w->g.nc; c++) cell_counts[c] = (c + 1 < w->g.nc ? st[c + 1] : n) - st[c];
     }
     return PIC_OK;
 }
@@ -2228,6 +2252,7 @@ extern "C" int pic_source_sample(pic_world* w, int source_id) {
     const uint4 ru = philox4x32_10(make_uint4(0xFFFFFFFFu, sa.step, 0x5C000000u + sa.src, 7u), sa.key);
     const long n = (long)(num_micro / s.mpw0 + (double)u01(ru.x));
     if (n <= 0) return PIC_OK;
+    std::lock_guard<std::mutex> lock(w->stage_mutex);
     int rc = ensure_upload(w, n);
     if (rc) return rc;
     const long cap = w->upload_cap;

@@ -103,6 +103,54 @@ __global__ void k_finalize_rho(FinalizeArgs a) {
 }
 void launch_finalize_rho(const FinalizeArgs& a, cudaStream_t s, int grid) { k_finalize_rho<<<grid, 256, 0, s>>>(a); }
 
+// Node fields as the caller's FP64 arrays (a staging buffer of nodes first .. first + m - 1 at a time).
+// The conversions run here, so that the host only copies: converting 16.8 M nodes through host vectors
+// took 13-17 ms a field on one core, the copy alone 0.8 ms into touched and 5.5 ms into fresh pages.
+__global__ void k_phi_out(const float2* __restrict__ phi, int m, double* __restrict__ out) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x)
+        out[x] = ff_to_double(phi[x]);
+}
+__global__ void k_phi_in(const double* __restrict__ in, int m, float2* __restrict__ phi) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) phi[x] = ff_pack(in[x]);
+}
+__global__ void k_f32_out(const float* __restrict__ f, int m, double* __restrict__ out) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) out[x] = (double)f[x];
+}
+__global__ void k_f32_in(const double* __restrict__ in, int m, float* __restrict__ f) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) f[x] = (float)in[x];
+}
+__global__ void k_ef_out(const float4* __restrict__ ef, int m, double* __restrict__ out) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x) {
+        const float4 e = ef[x];
+        out[3 * (size_t)x] = (double)e.x;
+        out[3 * (size_t)x + 1] = (double)e.y;
+        out[3 * (size_t)x + 2] = (double)e.z;
+    }
+}
+__global__ void k_ef_in(const double* __restrict__ in, int m, float4* __restrict__ ef) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += gridDim.x * blockDim.x)
+        ef[x] = make_float4((float)in[3 * (size_t)x], (float)in[3 * (size_t)x + 1], (float)in[3 * (size_t)x + 2], 0.f);
+}
+static int copy_blocks(int m) { return std::max(1, std::min(1216, (m + 255) / 256)); }
+void launch_phi_out(const float2* phi, int m, double* out, cudaStream_t s) {
+    k_phi_out<<<copy_blocks(m), 256, 0, s>>>(phi, m, out);
+}
+void launch_phi_in(const double* in, int m, float2* phi, cudaStream_t s) {
+    k_phi_in<<<copy_blocks(m), 256, 0, s>>>(in, m, phi);
+}
+void launch_f32_out(const float* f, int m, double* out, cudaStream_t s) {
+    k_f32_out<<<copy_blocks(m), 256, 0, s>>>(f, m, out);
+}
+void launch_f32_in(const double* in, int m, float* f, cudaStream_t s) {
+    k_f32_in<<<copy_blocks(m), 256, 0, s>>>(in, m, f);
+}
+void launch_ef_out(const float4* ef, int m, double* out, cudaStream_t s) {
+    k_ef_out<<<copy_blocks(m), 256, 0, s>>>(ef, m, out);
+}
+void launch_ef_in(const double* in, int m, float4* ef, cudaStream_t s) {
+    k_ef_in<<<copy_blocks(m), 256, 0, s>>>(in, m, ef);
+}
+
 // dst += src over n floats, four per thread with 16-byte accesses where n allows
 __global__ void k_add_f32(float* __restrict__ dst, const float* __restrict__ src, int n) {
     const int n4 = n >> 2;

@@ -225,6 +225,13 @@ void launch_pcg_iter_impl(const GridDev& g, SolveWork& w, float* d_in, float* d_
 // phi[dst] = phi[src] for the MIRROR pairs (first n_mirror entries), then the ALIAS pairs
 void launch_fill_aux(const int2* pairs, int n_mirror, int n_alias, float2* phi, cudaStream_t s);
 void launch_den_avg(float* avg, const float* den, int nv, float a, float b, cudaStream_t s, int grid);
+// m nodes of a field to and from FP64 (phi as hi + lo, a float field, the three components of E)
+void launch_phi_out(const float2* phi, int m, double* out, cudaStream_t s);
+void launch_phi_in(const double* in, int m, float2* phi, cudaStream_t s);
+void launch_f32_out(const float* f, int m, double* out, cudaStream_t s);
+void launch_f32_in(const double* in, int m, float* f, cudaStream_t s);
+void launch_ef_out(const float4* ef, int m, double* out, cudaStream_t s);
+void launch_ef_in(const double* in, int m, float4* ef, cudaStream_t s);
 // dst += src (n floats; both 16-byte aligned)
 void launch_add(float* dst, const float* src, int n, cudaStream_t s, int grid);
 
