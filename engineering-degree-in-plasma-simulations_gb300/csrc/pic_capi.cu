@@ -24,6 +24,7 @@ using namespace pic;
 
 constexpr double kFp32Unit = 0x1p-24;  // unit roundoff of FP32 round-to-nearest
 constexpr long kUploadChunk = 1l << 22;  // particles per upload staging round (256 MB)
+constexpr int kClusterMost = 16;         // CTAs of the one-cluster inner solvers
 constexpr long kFieldChunk = 1l << 22;   // doubles per round of a node field's staging (32 MB)
 constexpr long kSortMovedFraction = 50;   // re-sort a species when 2 % of it left cell order
 
@@ -170,6 +171,8 @@ struct pic_world {
     int max_it = 10000;
     double omega = 1.4;
     long n_solves = 0, n_refine = 0, n_inner = 0;
+    // planes per CTA of the one-cluster inner solvers (0: the grid does not fit), valid for cluster_per
+    int sor_planes = 0, pcg_planes = 0, cluster_per = -1;
     LpState* lp = nullptr;  // learned preconditioner, created on first use
     // r (FP32) holds the FP64 residual of phi for rho_prev; the next solve updates it by
     // (rho - rho_prev) / eps0 instead of an FP64 pass.  Cleared when phi, the boundaries or r change.
@@ -557,6 +560,8 @@ SolveWork solve_work(pic_world* w) {
     s.gpart = w->gpart;
     s.gstride = w->gstride;
     s.ticket = w->ticket;
+    s.err = w->err;
+    s.wait_polls = wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls);
     return s;
 }
 
@@ -1724,7 +1729,23 @@ int learned_validation_iters(pic_world* w, const float* r, int cap, int* iters) 
     return rc;
 }
 
+// the one-cluster inner solvers' plans for the world's grid
+void plan_clusters(pic_world* w) {
+    if (w->cluster_per == w->periodic[2]) return;
+    w->sor_planes = plan_sor_cluster(w->g, kClusterMost);
+    w->pcg_planes = plan_pcg_cluster(w->g, kClusterMost);
+    w->cluster_per = w->periodic[2];
+}
+// a bounded wait of an inner solver ran out (flag[2], read into h_flag[2]): the solve ends with an error
+int inner_wait_failed(pic_world* w) {
+    w->rhs_valid = false;
+    CU(cudaMemsetAsync(w->flag, 0, sizeof(int) * 4, w->stream));
+    int rc = check_device_error(w);
+    return rc ? rc : fail(PIC_ERR_DEVICE, "a bounded wait of the Poisson solver expired");
+}
+
 int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
+    plan_clusters(w);
     SolveWork sw = solve_work(w);
     double r2, b2, s2 = 0;
     // an FP32 update of the last full residual when phi is unchanged since; the answer is always
@@ -1777,6 +1798,7 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
             continue;
         }
         if (!(iters < w->max_it && outer < 1000)) break;
+        bool waited = false;
         outer++;
         estimated = false;
         if (w->method == PIC_SOLVER_LEARNED && !use_pcg) {
@@ -1785,7 +1807,12 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
         }
         if (w->method == PIC_SOLVER_RBSOR) {
             int sweeps = std::min(25, w->max_it - iters);
-            {
+            if (w->sor_planes > 0) {
+                Scope sc(w, "poisson", 1);
+                launch_sor_cluster(w->g, sw, (float)w->omega, sweeps, w->sor_planes, w->stream);
+                CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
+                waited = true;  // h_flag[2] is read after the residual's synchronisation
+            } else {
                 Scope sc(w, "poisson", 3 * sweeps);
                 CU(cudaMemsetAsync(w->e, 0, sizeof(float) * w->g.nv, w->stream));
                 launch_rbsor_sweeps(w->g, sw, (float)w->omega, sweeps, w->stream);
@@ -1815,16 +1842,23 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
         } else {
             // inner FP32 flexible PCG to eta = 1e-3 of the current residual (or the final target)
             double target = std::max(1e-6 * r2, kInnerTarget * w->tol * w->tol * bn * bn);
-            {
-                Scope sc(w, "poisson", 1);
-                launch_pcg_init(w->g, sw, w->stream);
-            }
+            // a warm-started refinement of the learned method tries a few Jacobi iterations first
+            const int cap = (w->method == PIC_SOLVER_LEARNED && !use_pcg) ? w->warm_jacobi : w->max_it;
             float* din = w->d;
             float* dout = w->d2;
             int it = 0;
-            // a warm-started refinement of the learned method tries a few Jacobi iterations first
-            const int cap = (w->method == PIC_SOLVER_LEARNED && !use_pcg) ? w->warm_jacobi : w->max_it;
-            for (int nb = 2;; nb = std::min(16, 2 * nb)) {  // growing batches: early exits cost little
+            if (w->pcg_planes > 0) {
+                Scope sc(w, "poisson", 1);
+                launch_pcg_cluster(w->g, sw, target, std::min(cap, w->max_it - iters), w->pcg_planes, w->stream);
+                CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
+                CU(cudaStreamSynchronize(w->stream));
+                if (w->h_flag[2]) return inner_wait_failed(w);
+                iters += w->h_flag[1];
+            } else {
+                Scope sc(w, "poisson", 1);
+                launch_pcg_init(w->g, sw, w->stream);
+            }
+            for (int nb = 2; w->pcg_planes == 0; nb = std::min(16, 2 * nb)) {  // growing batches: early exits cost little
                 int batch = std::min(std::min(nb, w->max_it - iters), cap - it);
                 if (batch <= 0) break;
                 {
@@ -1851,6 +1885,7 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
         }
         rc = residual_norms(w, sw, 1, r2, b2, s2);
         if (rc) return rc;
+        if (waited && w->h_flag[2]) return inner_wait_failed(w);
         bn = stop_scale(w, b2, s2);
         rel = std::sqrt(r2) / bn;
         if (!(rel == rel)) break;  // NaN: diverged

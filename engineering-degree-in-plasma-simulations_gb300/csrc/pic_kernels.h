@@ -178,11 +178,21 @@ struct SolveWork {
     float* z;         // CG preconditioned residual
     double* part;     // per-block partial sums [kParts * nslots]
     double* scal;     // device scalars (slots below)
-    int* flag;        // [0] inner converged, [1] iterations completed
+    int* flag;        // [0] inner converged, [1] iterations completed, [2] a bounded wait ran out
+    unsigned* err;    // the world's device error word
+    long long wait_polls;  // polls of a bounded wait
     double* gpart;    // node-kernel block partials [8][gstride]
     int gstride;
     unsigned* ticket; // last-block counter of the node-kernel reductions
 };
+// Inner solvers on one thread-block cluster (pic_cluster.cu): planes per CTA, 0 when the grid does not
+// fit a cluster of at most `most` CTAs
+int plan_sor_cluster(const GridDev& g, int most);
+int plan_pcg_cluster(const GridDev& g, int most);
+// sweeps from e = 0 (with the seam passes); the whole inner CG solve from e = 0, at most cap iterations
+// (flag[0] converged, flag[1] iterations)
+void launch_sor_cluster(const GridDev& g, SolveWork& w, float omega, int sweeps, int planes, cudaStream_t s);
+void launch_pcg_cluster(const GridDev& g, SolveWork& w, double target_rr, int cap, int planes, cudaStream_t s);
 constexpr int kParts = 1024;
 // Node kernels take a tile of kNodeTile consecutive nodes per block, kNodeTile / blockDim.x per
 // thread, strided by blockDim.x so that every load is coalesced and a thread's loads are
