@@ -171,8 +171,9 @@ struct pic_world {
     int max_it = 10000;
     double omega = 1.4;
     long n_solves = 0, n_refine = 0, n_inner = 0;
-    // planes per CTA of the one-cluster inner solvers (0: the grid does not fit), valid for cluster_per
-    int sor_planes = 0, pcg_planes = 0, cluster_per = -1;
+    // inner solvers that keep the grid on the chip: planes per CTA of the one-cluster form, nodes per CTA
+    // of the whole-GPU form (0: not that form), for the periodic z axis they were planned with
+    int sor_planes = 0, pcg_planes = 0, sor_chunk = 0, pcg_chunk = 0, inner_per = -1;
     LpState* lp = nullptr;  // learned preconditioner, created on first use
     // r (FP32) holds the FP64 residual of phi for rho_prev; the next solve updates it by
     // (rho - rho_prev) / eps0 instead of an FP64 pass.  Cleared when phi, the boundaries or r change.
@@ -1729,12 +1730,15 @@ int learned_validation_iters(pic_world* w, const float* r, int cap, int* iters) 
     return rc;
 }
 
-// the one-cluster inner solvers' plans for the world's grid
-void plan_clusters(pic_world* w) {
-    if (w->cluster_per == w->periodic[2]) return;
+// the form of the inner solvers for the world's grid: one cluster, else the whole GPU, else (0) a launch
+// per pass
+void plan_inner(pic_world* w) {
+    if (w->inner_per == w->periodic[2]) return;
     w->sor_planes = plan_sor_cluster(w->g, kClusterMost);
     w->pcg_planes = plan_pcg_cluster(w->g, kClusterMost);
-    w->cluster_per = w->periodic[2];
+    w->sor_chunk = w->sor_planes ? 0 : plan_sor_grid(w->g, w->sms);
+    w->pcg_chunk = w->pcg_planes ? 0 : plan_pcg_grid(w->g, w->sms);
+    w->inner_per = w->periodic[2];
 }
 // a bounded wait of an inner solver ran out (flag[2], read into h_flag[2]): the solve ends with an error
 int inner_wait_failed(pic_world* w) {
@@ -1745,7 +1749,7 @@ int inner_wait_failed(pic_world* w) {
 }
 
 int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
-    plan_clusters(w);
+    plan_inner(w);
     SolveWork sw = solve_work(w);
     double r2, b2, s2 = 0;
     // an FP32 update of the last full residual when phi is unchanged since; the answer is always
@@ -1807,9 +1811,12 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
         }
         if (w->method == PIC_SOLVER_RBSOR) {
             int sweeps = std::min(25, w->max_it - iters);
-            if (w->sor_planes > 0) {
+            if (w->sor_planes > 0 || w->sor_chunk > 0) {
                 Scope sc(w, "poisson", 1);
-                launch_sor_cluster(w->g, sw, (float)w->omega, sweeps, w->sor_planes, w->stream);
+                if (w->sor_planes > 0)
+                    launch_sor_cluster(w->g, sw, (float)w->omega, sweeps, w->sor_planes, w->stream);
+                else
+                    launch_sor_grid(w->g, sw, (float)w->omega, sweeps, w->sor_chunk, w->stream);
                 CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
                 waited = true;  // h_flag[2] is read after the residual's synchronisation
             } else {
@@ -1847,9 +1854,14 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
             float* din = w->d;
             float* dout = w->d2;
             int it = 0;
-            if (w->pcg_planes > 0) {
+            const bool on_chip = w->pcg_planes > 0 || w->pcg_chunk > 0;  // the whole inner solve in one launch
+            if (on_chip) {
                 Scope sc(w, "poisson", 1);
-                launch_pcg_cluster(w->g, sw, target, std::min(cap, w->max_it - iters), w->pcg_planes, w->stream);
+                const int most = std::min(cap, w->max_it - iters);
+                if (w->pcg_planes > 0)
+                    launch_pcg_cluster(w->g, sw, target, most, w->pcg_planes, w->stream);
+                else
+                    launch_pcg_grid(w->g, sw, target, most, w->pcg_chunk, w->stream);
                 CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
                 CU(cudaStreamSynchronize(w->stream));
                 if (w->h_flag[2]) return inner_wait_failed(w);
@@ -1858,7 +1870,7 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
                 Scope sc(w, "poisson", 1);
                 launch_pcg_init(w->g, sw, w->stream);
             }
-            for (int nb = 2; w->pcg_planes == 0; nb = std::min(16, 2 * nb)) {  // growing batches: early exits cost little
+            for (int nb = 2; !on_chip; nb = std::min(16, 2 * nb)) {  // growing batches: early exits cost little
                 int batch = std::min(std::min(nb, w->max_it - iters), cap - it);
                 if (batch <= 0) break;
                 {

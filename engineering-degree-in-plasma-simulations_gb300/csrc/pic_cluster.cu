@@ -499,6 +499,10 @@ void fill_config(int ctas, int threads, size_t smem, cudaStream_t s, cudaLaunchC
     cfg.numAttrs = 1;
 }
 constexpr size_t kSmemMost = 216 * 1024;  // with the static arrays below the 227 KB of a CTA
+// nodes per CTA up to which one cluster is the faster form: at 45^3 (6075 a CTA) 25 sweeps take 107 us here
+// and 108 us on the whole GPU (pic_persist.cu), a CG iteration 6.7 and 7.4 us; at 31 x 31 x 51 (3844) 75
+// and 104 us, 4.9 and 7.3 us; sweeps of 60^3 (14 400) 161 and 120 us
+constexpr long kOwnMost = 6144;
 int stack_planes(const GridDev& g) { return g.periodic[2] ? g.nk - 1 : g.nk; }
 // whether a cluster of the kernel can be resident (its attributes are set here, before any launch)
 template <class K>
@@ -521,7 +525,7 @@ PcgKernel pcg_kernel(long own, int* threads) {
     if (own <= 1024) return k_pcg_cluster<256, 4>;
     if (own <= 2048) return k_pcg_cluster<256, 8>;
     if (own <= 4096) return k_pcg_cluster<512, 8>;
-    if (own <= 8192) return k_pcg_cluster<512, 16>;
+    if (own <= 6144) return k_pcg_cluster<512, 12>;
     return nullptr;
 }
 // threads of the sweeps: one listed node of a pass each, where that many fit
@@ -534,7 +538,7 @@ int plan_sor_cluster(const GridDev& g, int most) {
     for (int c = most; c >= 1; c >>= 1) {
         const int planes = (nz + c - 1) / c, ctas = (nz + planes - 1) / planes;
         const size_t b = sor_smem(nij, planes);
-        if (b > kSmemMost) return 0;
+        if (b > kSmemMost || nij * planes > kOwnMost) return 0;
         if (fits(k_sor_cluster, ctas, sor_threads(nij * planes), b)) return planes;
     }
     return 0;
@@ -547,7 +551,7 @@ int plan_pcg_cluster(const GridDev& g, int most) {
         const size_t b = pcg_smem(nij, planes);
         int threads;
         PcgKernel k = pcg_kernel(nij * planes, &threads);
-        if (!k || b > kSmemMost) return 0;
+        if (!k || b > kSmemMost || nij * planes > kOwnMost) return 0;
         if (fits(k, ctas, threads, b)) return planes;
     }
     return 0;

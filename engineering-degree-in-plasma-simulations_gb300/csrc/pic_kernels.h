@@ -193,6 +193,11 @@ int plan_pcg_cluster(const GridDev& g, int most);
 // (flag[0] converged, flag[1] iterations)
 void launch_sor_cluster(const GridDev& g, SolveWork& w, float omega, int sweeps, int planes, cudaStream_t s);
 void launch_pcg_cluster(const GridDev& g, SolveWork& w, double target_rr, int cap, int planes, cudaStream_t s);
+// The same over the whole GPU (pic_persist.cu): nodes per CTA, 0 when the grid does not fit its SMs' shared memory
+int plan_sor_grid(const GridDev& g, int sms);
+int plan_pcg_grid(const GridDev& g, int sms);
+void launch_sor_grid(const GridDev& g, SolveWork& w, float omega, int sweeps, int chunk, cudaStream_t s);
+void launch_pcg_grid(const GridDev& g, SolveWork& w, double target_rr, int cap, int chunk, cudaStream_t s);
 constexpr int kParts = 1024;
 // Node kernels take a tile of kNodeTile consecutive nodes per block, kNodeTile / blockDim.x per
 // thread, strided by blockDim.x so that every load is coalesced and a thread's loads are

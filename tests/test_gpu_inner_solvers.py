@@ -1,7 +1,7 @@
 """The Poisson inner solvers that keep a whole grid on the chip: one thread-block cluster for small
-grids.  Every geometry rule that their shared-memory planes restate (halo planes, rings, seams of
-periodic axes with an odd number of nodes, mirror walls, objects, thin and one-plane slabs, the largest
-grids of each register form) is solved and compared with the FP64 oracle's converged answer."""
+grids, a persistent kernel over the whole GPU for mid-size ones.  Every geometry rule that they restate
+(halo planes, rings, seams of periodic axes with an odd number of nodes, mirror walls, objects, thin and
+one-plane slabs, rows of every remainder by four, short rows, the largest grids of each register form) is solved and compared with the FP64 oracle's converged answer."""
 import numpy as np
 import pytest
 
@@ -19,6 +19,10 @@ CASES = {
     "mirror_walls_box": ((19, 15, 23), (0, 0, 0), 0, (((0.5, 0.5, 0.0), (2.0, 2.0, 0.2), 100.0),)),
     "widest_planes": ((60, 61, 40), (0, 0, 0), 1, ()),
     "above_one_cluster": ((67, 66, 45), (1, 0, 0), 1, ()),
+    "rows_of_64": ((64, 60, 50), (1, 1, 0), 1, ()),
+    "rows_of_62_mirror": ((62, 61, 44), (0, 1, 0), 0, (((0.5, 0.5, 0.0), (2.0, 2.0, 0.1), 30.0),)),
+    "short_rows": ((3, 5, 8000), (0, 0, 0), 1, ()),
+    "ring_of_the_grid": ((57, 55, 60), (1, 1, 1), 1, (((0.4, 0.5, 0.5), (0.2, 0.3, 0.3), 40.0),)),
 }
 
 
@@ -56,7 +60,7 @@ def test_converges_to_the_oracles_answer(pic, port, name, method):
     W.close()
 
 
-@pytest.mark.parametrize("name", ["walls_21", "ring_all_seams"])
+@pytest.mark.parametrize("name", ["walls_21", "ring_all_seams", "rows_of_64"])
 @pytest.mark.parametrize("method", ["rbsor", "pcg"])
 def test_wait_that_runs_out_is_reported_and_solver_recovers(pic, port, name, method):
     W, g, kind = setup(pic, port, name)
