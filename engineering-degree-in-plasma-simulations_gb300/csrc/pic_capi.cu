@@ -1679,13 +1679,22 @@ constexpr int kLearnedInnerCap = 400;  // iterations of one learned inner solve 
 // FP32 recurrence of the inner residual, which the following float-float residual then certifies
 constexpr double kInnerTarget = 0.64;
 
+// a bounded wait of an inner solver ran out (flag[2], read into h_flag[2]): the solve ends with an error
+int inner_wait_failed(pic_world* w) {
+    w->rhs_valid = false;
+    CU(cudaMemsetAsync(w->flag, 0, sizeof(int) * 4, w->stream));
+    CU(cudaMemsetAsync(w->ticket, 0, sizeof(unsigned) * 4, w->stream));  // counters of a barrier left half-way
+    int rc = check_device_error(w);
+    return rc ? rc : fail(PIC_ERR_DEVICE, "a bounded wait of the Poisson solver expired");
+}
+
 // FP32 flexible CG with the learned preconditioner on L e = r (w->r), e from zero, until
 // r.r <= target or cap iterations; *done = iterations, *conv = reached the target.  Iterations go
 // out in batches between which the host reads the stop flag (the iterations of a batch after the
 // stop return at once, about 30 us each at 256^3): first_batch, then 2, 4, 4, ...
 int learned_inner(pic_world* w, SolveWork& sw, double target, int cap, int first_batch, int* done, bool* conv) {
     {
-        Scope sc(w, "poisson", 4 + 2 * w->lp->nlev);
+        Scope sc(w, "poisson", lp_apply_launches(*w->lp));
         launch_lpcg_init(w->g, sw, *w->lp, w->stream, w->sms);
     }
     float* din = w->d;
@@ -1696,15 +1705,16 @@ int learned_inner(pic_world* w, SolveWork& sw, double target, int cap, int first
     for (int nb = 0; it < cap; nb++) {
         int batch = std::min(nb == 0 ? std::max(1, first_batch) : std::min(4, 1 << nb), cap - it);
         {
-            Scope sc(w, "poisson", (1 + 2 * w->lp->nlev) * batch);
+            Scope sc(w, "poisson", (2 + lp_apply_launches(*w->lp)) * batch);
             for (int b = 0; b < batch; b++) {
                 launch_lpcg_iter(w->g, sw, *w->lp, din, dout, it, target, w->stream, w->sms);
                 std::swap(din, dout);
                 it++;
             }
         }
-        CU(cudaMemcpyAsync(w->h_flag, w->flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
+        CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
         CU(cudaStreamSynchronize(w->stream));
+        if (w->h_flag[2]) return inner_wait_failed(w);
         if (w->h_flag[0]) {
             *done = w->h_flag[1];  // the batch stopped at iteration flag[1]
             *conv = true;
@@ -1740,14 +1750,6 @@ void plan_inner(pic_world* w) {
     w->pcg_chunk = w->pcg_planes ? 0 : plan_pcg_grid(w->g, w->sms);
     w->inner_per = w->periodic[2];
 }
-// a bounded wait of an inner solver ran out (flag[2], read into h_flag[2]): the solve ends with an error
-int inner_wait_failed(pic_world* w) {
-    w->rhs_valid = false;
-    CU(cudaMemsetAsync(w->flag, 0, sizeof(int) * 4, w->stream));
-    int rc = check_device_error(w);
-    return rc ? rc : fail(PIC_ERR_DEVICE, "a bounded wait of the Poisson solver expired");
-}
-
 int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
     plan_inner(w);
     SolveWork sw = solve_work(w);
@@ -1997,10 +1999,12 @@ extern "C" int pic_learned_apply(pic_world* w, const double* r, double* z) {
     for (int n = 0; n < g.nv; n++) rf[n] = (kind[n] & 3) == kFree ? (float)r[n] : 0.f;
     w->rhs_valid = false;
     CU(cudaMemcpyAsync(w->r, rf.data(), sizeof(float) * g.nv, cudaMemcpyHostToDevice, w->stream));
-    launch_lp_apply(g, *w->lp, w->r, w->z, w->kind, nullptr, nullptr, nullptr, w->stream, w->sms);
+    launch_lp_apply(g, *w->lp, solve_work(w), w->r, w->z, nullptr, false, nullptr, w->stream, w->sms);
     CU(cudaGetLastError());
+    CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
     CU(cudaMemcpyAsync(rf.data(), w->z, sizeof(float) * g.nv, cudaMemcpyDeviceToHost, w->stream));
     CU(cudaStreamSynchronize(w->stream));
+    if (w->h_flag[2]) return inner_wait_failed(w);
     for (int n = 0; n < g.nv; n++) z[n] = rf[n];
     return PIC_OK;
 }

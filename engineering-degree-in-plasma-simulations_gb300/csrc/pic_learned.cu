@@ -11,6 +11,7 @@
 #include <vector>
 #include <cuda_bf16.h>
 #include <cstring>
+#include "pic_grid_sync.cuh"
 #include "pic_learned.h"
 #include "pic_stencil.cuh"
 #include "pic_tc.cuh"
@@ -374,41 +375,278 @@ __global__ void k_lp_up(LView zin, LView cin, LView out, int mode, const float* 
         lp_up_at(zin, cin, out, mode, fold, fold_g, inv_diag, idx);
 }
 
-// The coarse end of the hierarchy in one CTA: the restrictions from level l0 - 1 down to the
-// last level, then the level operators from the last level back up to l0, with a block barrier
-// between levels.  These levels hold a few thousand voxels or fewer, so one kernel instead of a
-// launch per level and direction removes a chain of latency-bound launches; every voxel is
-// computed by the same device functions as k_lp_restrict and k_lp_up.
-struct LpCoarseArgs {
-    int l0, nlev;
-    LView f0;                        // level l0 - 1 (its restricted input; the residual if l0 == 1)
+// ------------------------------------------------------------------------------------
+// The coarse part of the hierarchy, levels m .. nlev - 1, in one cooperative launch (one CTA per SM):
+// the restrictions down from level m - 1, then the level operators from the last level back up to m.
+//
+// As a launch per level and direction, with the coarsest levels in one CTA, this part was a chain of
+// latency-bound kernels: 9.7 + 8.0 (restrictions) + 32 (one CTA) + 10.8 + 10.7 us of the 145 us of an
+// iteration of 63 x 63 x 256 nodes, the same for grids of any size.  One launch takes 28 us.  Here
+//   - a level's voxels are spread over all SMs, with up to 32 lanes per voxel that share its taps (the
+//     64 points of a restriction, the 125 taps and 8 prolongation corners of an operator), so that a
+//     thread has few dependent reads and a level costs about one L2 latency and a grid barrier;
+//   - below level lr (at most kLpRedundant voxels) every CTA restricts for itself in shared memory, and
+//     from level le on (network levels of at most kLpRedundantNet voxels) it applies the operators for
+//     itself too, which needs no grid barrier.  (An operator's 125 taps on the 2048 voxels of the next
+//     level up took one CTA 41 000 cycles; spread over the GPU they take 9500, and a barrier 2700.)
+// ------------------------------------------------------------------------------------
+constexpr int kLpMidThreads = 512;
+constexpr int kLpMidMost = 65536;    // voxels of the first level that joins
+constexpr int kLpRedundant = 4096;   // voxels of the last level that the GPU restricts together
+constexpr int kLpRedundantNet = 512;  // voxels of a network level that every CTA computes for itself
+struct LpMidArgs {
+    int m, lr, le, nlev;
+    LView f0;                        // level m - 1 (its restricted input; the residual if m == 1)
     LView z[kLpMaxLevels], e[kLpMaxLevels];
-    int mode[kLpMaxLevels];          // 1: network level (folded stencils), 2: diagonal scaling
-    const float* fold[kLpMaxLevels];
+    const float* fold[kLpMaxLevels];  // folded stencils of a network level, nullptr: diagonal scaling
     float inv_diag[kLpMaxLevels];
+    unsigned* left;                  // CTAs that have finished (the last one resets the barrier)
+    GridWait wait;
 };
-constexpr int kLpCoarseThreads = 512;
-constexpr int kLpCoarseMaxVox = 8192;    // diagonal levels up to this size join the fused chain
-constexpr int kLpCoarseMaxNetVox = 1024;  // network levels up to this size
-__global__ void __launch_bounds__(kLpCoarseThreads) k_lp_coarse(LpCoarseArgs a, const int* flag) {
-    if (flag && flag[0]) return;
-    __shared__ float fold[kLpFold];
-    for (int l = a.l0; l < a.nlev; l++) {
-        const LView& f = l == a.l0 ? a.f0 : a.z[l - 1];
-        for (unsigned idx = threadIdx.x; idx < (unsigned)a.z[l].nvox; idx += blockDim.x) lp_restrict_at(f, a.z[l], idx);
-        __syncthreads();
+// a value of a level: shared memory, or global memory that other CTAs write (L2)
+template <bool SH>
+__device__ __forceinline__ float lp_ld(const float* p) {
+    return SH ? *p : __ldcg(p);
+}
+// sum over the lanes of a voxel's group of S lanes (in its first lane)
+template <int S>
+__device__ __forceinline__ float lp_group_sum(float v) {
+#pragma unroll
+    for (int o = S / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, S);
+    return v;
+}
+// part `s` of S of (R f) at coarse voxel cc: the fine rows s, s + S, ... of its 16, four points each
+// (index rules of k_lp_restrict; points outside the box count zero)
+template <bool SH, int S>
+__device__ __forceinline__ float lp_restrict_part(const LView& f, const LView& c, const int (&cc)[3], int s) {
+    const float w4[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+    auto map = [&](int ax, int k) {
+        int raw = 2 * cc[ax] + k - 1;
+        if (f.per[ax]) {
+            const int nc2 = 2 * c.n[ax];
+            raw = raw < 0 ? raw + nc2 : (raw >= nc2 ? raw - nc2 : raw);
+        }
+        return (unsigned)raw < (unsigned)f.n[ax] ? raw : -1;
+    };
+    int x[4];
+    float wx[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int u = map(0, k);
+        x[k] = max(u, 0);
+        wx[k] = u >= 0 ? w4[k] : 0.f;
+    }
+    float acc = 0.f;
+#pragma unroll
+    for (int q = 0; q < 16 / S; q++) {
+        const int row = s + q * S, ky = row & 3, kz = row >> 2;
+        const int y = map(1, ky), z = map(2, kz);
+        const bool in = y >= 0 && z >= 0;
+        const float wr = in ? ((ky == 0 || ky == 3) ? 0.25f : 0.75f) * ((kz == 0 || kz == 3) ? 0.25f : 0.75f) : 0.f;
+        const float* p = f.a + (in ? y * f.sy + z * f.sz : 0);
+        float a = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; k++) a += wx[k] * lp_ld<SH>(p + x[k]);
+        acc += wr * a;
+    }
+    return acc;
+}
+// part `s` of S of op(z) + P e at voxel c: the rows s, s + S, ... of the 25 rows of a network level's
+// 5 x 5 x 5 stencil (k5: its interior coefficients, shared; face points take their class's variant)
+// or the scaled value, and the corners s, s + S, ... of the prolongation (e.a null: none).  Taps outside
+// the box read a valid point with weight zero, so that up to five rows of loads are in flight together.
+template <bool ZSH, bool ESH, int S>
+__device__ __forceinline__ float lp_up_part(const LView& z, const LView& e, const float* k5,
+                                            const float* __restrict__ fold, float inv_diag, const int (&c)[3], int s) {
+    // coordinate c + d - 2 along an axis, and whether it lies in the box
+    auto nb = [&](int ax, int d, bool& in) {
+        int u = c[ax] + d - 2;
+        if (z.per[ax]) u = u < 0 ? u + z.n[ax] : (u >= z.n[ax] ? u - z.n[ax] : u);
+        in = (unsigned)u < (unsigned)z.n[ax];
+        return in ? u : c[ax];
+    };
+    constexpr int kCorners = (8 + S - 1) / S;
+    float ev[kCorners], ew[kCorners];
+#pragma unroll
+    for (int q = 0; q < kCorners; q++) {
+        const int k = s + q * S;
+        bool in = e.a && k < 8;
+        float w = 1.f;
+        int u[3];
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) {
+            const int b = (k >> ax) & 1, c0 = c[ax] >> 1;
+            u[ax] = b ? lv_nb(c0, (c[ax] & 1) ? 1 : -1, e.n[ax], e.per[ax]) : c0;
+            in = in && u[ax] >= 0;
+            w *= b ? 0.25f : 0.75f;
+        }
+        ew[q] = w;
+        ev[q] = in ? lp_ld<ESH>(e.a + lv_off(e, u[0], u[1], u[2])) : 0.f;
+    }
+    float acc = 0.f;
+    if (fold) {
+        int cls = 0, mul = 1;
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) {
+            if (!z.per[ax]) cls += mul * (c[ax] == 0 ? 1 : (c[ax] == z.n[ax] - 1 ? 2 : 0));
+            mul *= 3;
+        }
+        const float* kk = cls ? fold + kLpFold + 125 * cls : k5;
+        int x[5];
+        bool bx[5];
+#pragma unroll
+        for (int d = 0; d < 5; d++) x[d] = nb(0, d, bx[d]);
+        constexpr int kRows = (25 + S - 1) / S, kAtOnce = kRows < 5 ? kRows : 5;
+#pragma unroll
+        for (int q0 = 0; q0 < kRows; q0 += kAtOnce) {
+            float v[kAtOnce][5];
+#pragma unroll
+            for (int q = 0; q < kAtOnce; q++) {
+                const int row = s + (q0 + q) * S;
+                const int dz = row / 5, dy = row - 5 * dz;
+                bool iy, iz;
+                const int y = nb(1, dy, iy), zz = nb(2, dz, iz);
+                const bool in = q0 + q < kRows && row < 25 && iy && iz;
+                const float* p = z.a + (in ? y * z.sy + zz * z.sz : 0);
+#pragma unroll
+                for (int d = 0; d < 5; d++) v[q][d] = in && bx[d] ? lp_ld<ZSH>(p + x[d]) : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < kAtOnce; q++) {
+                const float* kr = kk + 5 * min(s + (q0 + q) * S, 24);
+#pragma unroll
+                for (int d = 0; d < 5; d++) acc = fmaf(kr[d], v[q][d], acc);
+            }
+        }
+    } else if (s == 0) {
+        acc = inv_diag * lp_ld<ZSH>(z.a + lv_off(z, c[0], c[1], c[2]));
+    }
+#pragma unroll
+    for (int q = 0; q < kCorners; q++) acc = fmaf(ew[q], ev[q], acc);
+    return acc;
+}
+// lanes per voxel: as many as leave every thread of the grid busy
+__device__ __forceinline__ int lp_split(int nvox, int threads, int most) {
+    int s = 1;
+    while (s < most && nvox * s * 2 <= threads) s *= 2;
+    return s;
+}
+// voxel groups of S lanes over nthr threads, the thread's number t: body(voxel, lane, live) for every voxel,
+// whole warps together
+template <int S, class F>
+__device__ __forceinline__ void lp_voxels(int nvox, int t, int nthr, F body) {
+    for (int v0 = (t & ~31) / S; v0 < nvox; v0 += nthr / S) {
+        const int v = v0 + (t & 31) / S;
+        body(min(v, nvox - 1), (t & 31) % S, v < nvox);
+    }
+}
+template <bool SH>
+__device__ void lp_restrict_level(const LView& f, const LView& c, int t, int nthr) {
+    auto run = [&](auto sc) {
+        constexpr int S = decltype(sc)::value;
+        lp_voxels<S>(c.nvox, t, nthr, [&](int v, int s, bool live) {
+            int cc[3];
+            lv_decode(c, (unsigned)v, cc[0], cc[1], cc[2]);
+            const float a = lp_group_sum<S>(lp_restrict_part<SH, S>(f, c, cc, s));
+            if (s == 0 && live) c.a[v] = a;
+        });
+    };
+    switch (lp_split(c.nvox, nthr, 16)) {
+        case 1: run(std::integral_constant<int, 1>{}); break;
+        case 2: run(std::integral_constant<int, 2>{}); break;
+        case 4: run(std::integral_constant<int, 4>{}); break;
+        case 8: run(std::integral_constant<int, 8>{}); break;
+        default: run(std::integral_constant<int, 16>{}); break;
+    }
+}
+template <bool ZSH, bool ESH>
+__device__ void lp_up_level(const LView& z, const LView& e, const LView& out, const float* k5, const float* fold,
+                            float inv_diag, int t, int nthr) {
+    auto run = [&](auto sc) {
+        constexpr int S = decltype(sc)::value;
+        lp_voxels<S>(out.nvox, t, nthr, [&](int v, int s, bool live) {
+            int c[3];
+            lv_decode(out, (unsigned)v, c[0], c[1], c[2]);
+            const float a = lp_group_sum<S>(lp_up_part<ZSH, ESH, S>(z, e, k5, fold, inv_diag, c, s));
+            if (s == 0 && live) out.a[v] = a;
+        });
+    };
+    switch (lp_split(out.nvox, nthr, 32)) {
+        case 1: run(std::integral_constant<int, 1>{}); break;
+        case 2: run(std::integral_constant<int, 2>{}); break;
+        case 4: run(std::integral_constant<int, 4>{}); break;
+        case 8: run(std::integral_constant<int, 8>{}); break;
+        case 16: run(std::integral_constant<int, 16>{}); break;
+        default: run(std::integral_constant<int, 32>{}); break;
+    }
+}
+__global__ void __launch_bounds__(kLpMidThreads, 1) k_lp_mid(LpMidArgs a, const int* flag) {
+    if (flag && flag[0]) return;  // every CTA alike: written by an earlier launch
+    extern __shared__ __align__(16) float mid_dyn[];
+    __shared__ float k5[kLpNetLevels + 1][125];
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, t = blockIdx.x * kLpMidThreads + tid, nthr = gridDim.x * kLpMidThreads;
+    if (tid == 0) s_fail = 0;
+    for (int l = a.m; l < a.nlev && l <= kLpNetLevels; l++)
+        for (int x = tid; x < 125; x += kLpMidThreads) k5[l][x] = a.fold[l][729 + x];
+    unsigned target = 0;
+    bool ok = true;
+    for (int l = a.m; l <= a.lr && l < a.nlev && ok; l++) {
+        lp_restrict_level<false>(l == a.m ? a.f0 : a.z[l - 1], a.z[l], t, nthr);
+        ok = grid_barrier(a.wait, target, &s_fail);
     }
     LView none{};
     none.a = nullptr;
-    for (int l = a.nlev - 1; l >= a.l0; l--) {
-        if (a.mode[l] == 1) {
-            for (int x = threadIdx.x; x < kLpFold; x += blockDim.x) fold[x] = a.fold[l][x];
-            __syncthreads();
-        }
-        const LView& cin = l + 1 < a.nlev ? a.e[l + 1] : none;
-        for (unsigned idx = threadIdx.x; idx < (unsigned)a.e[l].nvox; idx += blockDim.x)
-            lp_up_at(a.z[l], cin, a.e[l], a.mode[l], fold, a.fold[l], a.inv_diag[l], idx);
+    LView esh = none;  // e of level le in this CTA's shared memory
+    if (ok && a.le < a.nlev) {
+        // z of levels lr .. nlev - 1 in shared memory, one after the other, then e of levels nlev - 1 .. le
+        float* p = mid_dyn;
+        LView zs = a.z[a.lr];
+        zs.a = p;
+        for (int x = tid; x < zs.nvox; x += kLpMidThreads) p[x] = __ldcg(a.z[a.lr].a + x);
+        p += zs.nvox;
         __syncthreads();
+        for (int l = a.lr + 1; l < a.nlev; l++) {
+            LView c = a.z[l];
+            c.a = p;
+            p += c.nvox;
+            lp_restrict_level<true>(zs, c, tid, kLpMidThreads);
+            __syncthreads();
+            zs = c;
+        }
+        for (int l = a.nlev - 1; l >= a.le; l--) {
+            LView out = a.e[l];
+            out.a = p;
+            p += out.nvox;
+            lp_up_level<true, true>(zs, esh, out, k5[min(l, kLpNetLevels)], a.fold[l], a.inv_diag[l], tid, kLpMidThreads);
+            __syncthreads();
+            esh = out;
+            if (l > a.le) {
+                zs = a.z[l - 1];
+                float* q = mid_dyn;  // the z of level l - 1 lies behind those of levels lr .. l - 2
+                for (int k = a.lr; k < l - 1; k++) q += a.z[k].nvox;
+                zs.a = q;
+            }
+        }
+        if (a.le == a.m)  // no level above it here: its e goes out, each CTA its share
+            for (int x = t; x < esh.nvox; x += nthr) a.e[a.m].a[x] = esh.a[x];
+    }
+    for (int l = a.le - 1; l >= a.m && ok; l--) {
+        if (l == a.le - 1)
+            lp_up_level<false, true>(a.z[l], esh, a.e[l], k5[min(l, kLpNetLevels)], a.fold[l], a.inv_diag[l], t, nthr);
+        else
+            lp_up_level<false, false>(a.z[l], a.e[l + 1], a.e[l], k5[min(l, kLpNetLevels)], a.fold[l], a.inv_diag[l], t,
+                                      nthr);
+        if (l > a.m) ok = grid_barrier(a.wait, target, &s_fail);
+    }
+    if (tid == 0) {
+        if (!ok) {
+            set_error(a.wait.err, kErrBarrierTimeout);
+            *a.wait.fail = 1;
+        } else if (atomicAdd(a.left, 1u) == gridDim.x - 1) {
+            *a.left = 0u;  // the last CTA: every other one has passed its last barrier
+            *a.wait.arrived = 0u;
+        }
     }
 }
 
@@ -1096,35 +1334,56 @@ static void launch_restrict(const LView& f, const LView& c, const int* flag, cud
     }
 }
 
-void launch_lp_apply(const GridDev& g, const LpState& L, const float* r, float* z, const uint16_t* kind,
-                     const float* q, const SolveWork* red, const int* flag, cudaStream_t s, int sms) {
-    LView r0 = lp_node_view(g, L, const_cast<float*>(r));
-    // the first level of the fused coarse chain: every level from it down is small, and a network
-    // level only when it is tiny (one CTA is too little parallelism for the folded stencil above)
-    int l0 = L.nlev;
-    while (l0 > 1) {
-        const long nv_l = (long)L.dims[l0 - 1][0] * L.dims[l0 - 1][1] * L.dims[l0 - 1][2];
-        if (nv_l > kLpCoarseMaxVox || (l0 - 1 <= kLpNetLevels && nv_l > kLpCoarseMaxNetVox)) break;
-        l0--;
+int lp_apply_launches(const LpState& L) {
+    int n = 1;
+    for (int l = 1; l < L.nlev; l++) {
+        if (L.dims[l][0] * L.dims[l][1] * L.dims[l][2] <= kLpMidMost) return n + 1;
+        n += 2;
     }
+    return n;
+}
+void launch_lp_apply(const GridDev& g, const LpState& L, const SolveWork& w, const float* r, float* z, const float* q,
+                     bool sums, const int* flag, cudaStream_t s, int sms) {
+    const uint16_t* kind = reinterpret_cast<const uint16_t*>(w.kind);
+    LView r0 = lp_node_view(g, L, const_cast<float*>(r));
+    // levels m .. nlev - 1 in one launch; z below level lr and e from level le on by every CTA for itself
+    LpMidArgs ma{};
+    ma.m = ma.lr = ma.le = L.nlev;
+    for (int l = L.nlev - 1; l >= 1; l--) {
+        const int nv_l = L.dims[l][0] * L.dims[l][1] * L.dims[l][2];
+        if (nv_l <= kLpMidMost) ma.m = l;
+        if (nv_l <= kLpRedundant) ma.lr = l;
+        if (nv_l <= (l <= kLpNetLevels ? kLpRedundantNet : kLpRedundant)) ma.le = l;
+    }
+    const int l0 = ma.m;
     for (int l = 1; l < l0; l++) {
         LView f = l == 1 ? r0 : lp_level_view(L, l - 1, L.z[l - 1]);
         LView c = lp_level_view(L, l, L.z[l]);
         launch_restrict(f, c, flag, s, sms);
     }
     if (l0 < L.nlev) {
-        LpCoarseArgs ca{};
-        ca.l0 = l0;
-        ca.nlev = L.nlev;
-        ca.f0 = l0 == 1 ? r0 : lp_level_view(L, l0 - 1, L.z[l0 - 1]);
+        ma.nlev = L.nlev;
+        ma.f0 = l0 == 1 ? r0 : lp_level_view(L, l0 - 1, L.z[l0 - 1]);
+        size_t smem = 0;
         for (int l = l0; l < L.nlev; l++) {
-            ca.z[l] = lp_level_view(L, l, L.z[l]);
-            ca.e[l] = lp_level_view(L, l, L.e[l]);
-            ca.mode[l] = l <= kLpNetLevels ? 1 : 2;
-            ca.fold[l] = ca.mode[l] == 1 ? L.fold + (l - 1) * kLpFoldStride : nullptr;
-            ca.inv_diag[l] = (float)(1.0 / L.diag[l]);
+            ma.z[l] = lp_level_view(L, l, L.z[l]);
+            ma.e[l] = lp_level_view(L, l, L.e[l]);
+            ma.fold[l] = l <= kLpNetLevels ? L.fold + (l - 1) * kLpFoldStride : nullptr;
+            ma.inv_diag[l] = (float)(1.0 / L.diag[l]);
+            if (l >= ma.lr) smem += 2 * sizeof(float) * ma.z[l].nvox;
         }
-        k_lp_coarse<<<1, kLpCoarseThreads, 0, s>>>(ca, flag);
+        ma.left = w.ticket + 2;
+        ma.wait = GridWait{w.ticket + 1, w.wait_polls, w.err, w.flag + 2};
+        static int dyn_set = -1;  // the device whose attribute is set
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dyn_set != dev) {  // levels that halve only two axes add up to less than twice the first one
+            cudaFuncSetAttribute(k_lp_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (int)sizeof(float) * kLpRedundant);
+            dyn_set = dev;
+        }
+        void* args[] = {&ma, (void*)&flag};
+        cudaLaunchCooperativeKernel((const void*)k_lp_mid, dim3((unsigned)std::max(1, sms)), dim3(kLpMidThreads), args,
+                                    smem, s);
     }
     LView none{};
     none.a = nullptr;
@@ -1156,8 +1415,8 @@ void launch_lp_apply(const GridDev& g, const LpState& L, const float* r, float* 
         }
     }
     LView cin = L.nlev > 1 ? lp_level_view(L, 1, L.e[1]) : none;
-    launch_up0(g, r0, cin, z, kind, L.W + L.lay.s0, q, red ? red->gpart : nullptr, red ? red->gstride : 0,
-               red ? red->ticket : nullptr, red ? red->scal + kS_RZN : nullptr, flag, s, sms);
+    launch_up0(g, r0, cin, z, kind, L.W + L.lay.s0, q, w.gpart, w.gstride, w.ticket, sums ? w.scal + kS_RZN : nullptr,
+               flag, s, sms);
 }
 
 // folded stencils of every network level: M = Wm Wl (C x 27), K27[t][t'] = sum_c Wp[t][c] M[c][t'],
@@ -1445,7 +1704,7 @@ void launch_lpcg_init(const GridDev& g, SolveWork& w, const LpState& L, cudaStre
     cudaMemsetAsync(w.q, 0, sizeof(float) * g.nv, s);
     cudaMemsetAsync(w.d, 0, sizeof(float) * g.nv, s);
     cudaMemsetAsync(w.flag, 0, sizeof(int), s);
-    launch_lp_apply(g, L, w.r, w.z, reinterpret_cast<const uint16_t*>(w.kind), w.q, &w, nullptr, s, sms);
+    launch_lp_apply(g, L, w, w.r, w.z, w.q, true, nullptr, s, sms);
 }
 void launch_lpcg_iter(const GridDev& g, SolveWork& w, const LpState& L, float* d_in, float* d_out, int it,
                       double target_rr, cudaStream_t s, int sms) {
@@ -1454,7 +1713,7 @@ void launch_lpcg_iter(const GridDev& g, SolveWork& w, const LpState& L, float* d
                                            it, target_rr);
     k_lpcg_k2<<<stream_blocks(g), 256, 0, s>>>(g, d_out, w.q, w.e, w.r, kd, w.gpart, w.gstride, w.ticket, w.scal,
                                                   w.flag, it);
-    launch_lp_apply(g, L, w.r, w.z, kd, w.q, &w, w.flag, s, sms);
+    launch_lp_apply(g, L, w, w.r, w.z, w.q, true, w.flag, s, sms);
 }
 // the first kernel of an iteration alone, at iteration 0 (beta = 0: d = z, q = L z on the scratch
 // arrays): what the launch-shape tuner times

@@ -93,11 +93,12 @@ float* lp_train_r(const LpState& L);
 float* lp_train_grad(const LpState& L);
 double* lp_train_red(const LpState& L);
 unsigned* lp_train_err(const LpState& L);
-// z = B r on the node array (r zero off FREE nodes); with red != nullptr the last kernel also
-// sums z.r and z.q into red->scal[kS_RZN], [kS_RZO]; every kernel returns early when flag[0] is
-// set (inner solve converged)
-void launch_lp_apply(const GridDev& g, const LpState& L, const float* r, float* z, const uint16_t* kind,
-                     const float* q, const SolveWork* red, const int* flag, cudaStream_t s, int sms);
+// z = B r on the node array (r zero off FREE nodes); with sums the last kernel also sums z.r and z.q
+// into w.scal[kS_RZN], [kS_RZO]; every kernel returns early when flag[0] is set (inner solve converged);
+// w.flag[2] is set when a bounded wait ran out
+void launch_lp_apply(const GridDev& g, const LpState& L, const SolveWork& w, const float* r, float* z, const float* q,
+                     bool sums, const int* flag, cudaStream_t s, int sms);
+int lp_apply_launches(const LpState& L);  // kernels of one apply
 // flexible CG iteration with the learned preconditioner (see pic_learned.cu)
 void launch_lp_norm2(const float* a, int n, double* part, double* out, cudaStream_t s, int grid);
 void launch_lpcg_init(const GridDev& g, SolveWork& w, const LpState& L, cudaStream_t s, int sms);

@@ -17,6 +17,7 @@
 // The arithmetic of a node is that of k_rbsor and k_pcg_* (pic_fields.cu), in the same order.
 #include <algorithm>
 #include "pic_ff.cuh"
+#include "pic_grid_sync.cuh"
 #include "pic_stencil.cuh"
 
 namespace pic {
@@ -33,31 +34,6 @@ struct GridSync {
     unsigned pad[31];
     float2 part[4][kMostCtas];  // float-float partials: d.q, then the three sums after the update
 };
-struct GridWait {
-    GridSync* sync;
-    long long polls;
-    unsigned* err;
-    int* fail;
-};
-// all CTAs of the grid (co-resident: a cooperative launch); false when they did not arrive in time.
-// Global writes of any thread before it are seen by L2 reads of any thread after it.
-__device__ __forceinline__ bool grid_barrier(const GridWait& w, unsigned& target, int* s_fail) {
-    target += gridDim.x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&w.sync->arrived) : "memory");
-        bool ok = false;
-        for (long long it = 0; it < w.polls && !ok; it++) {
-            unsigned c;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&w.sync->arrived) : "memory");
-            ok = (int)(c - target) >= 0;
-        }
-        if (!ok) *s_fail = 1;
-    }
-    __syncthreads();
-    return *s_fail == 0;
-}
-
 // flags of a node: FREE (1), mirror mask (6 bits), wraps (6 bits: at the low / high end of a periodic
 // axis x, y, z); 0 for a node without an unknown
 __device__ __forceinline__ unsigned node_flags(const GridDev& g, int n, unsigned kd) {
@@ -257,7 +233,8 @@ constexpr unsigned long long kPlain4 = 0x0001000100010001ull, kWrap4 = 0x1F801F8
 template <int K>
 __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __restrict__ e, const float* __restrict__ r,
                                                       float* dg, const uint16_t* __restrict__ kind, FF target_rr,
-                                                      int cap, int chunk, int* flag, GridWait wait) {
+                                                      int cap, int chunk, int* flag, GridSync* sync,
+                                                      GridWait wait) {
     extern __shared__ __align__(16) float sm[];
     float4* D4 = reinterpret_cast<float4*>(sm);
     float4* R4 = D4 + chunk / 4;
@@ -295,8 +272,8 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
         R4[q] = make_float4(rv[0], rv[1], rv[2], rv[3]);
         M4[q] = mm;
     }
-    float2(*part1)[kMostCtas] = wait.sync->part;
-    float2(*part3)[kMostCtas] = wait.sync->part + 1;
+    float2(*part1)[kMostCtas] = sync->part;
+    float2(*part3)[kMostCtas] = sync->part + 1;
     unsigned target = 0;
     FF t1[1], t3[3];
     grid_total<3>(f3, wsum, part3, wait, target, &s_fail, t3);  // r.z
@@ -457,7 +434,8 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
 int chunk_of(const GridDev& g, int sms) { return ((g.nv + sms - 1) / sms + 31) / 32 * 32; }
 size_t sor_bytes(int chunk) { return 12 * (size_t)chunk; }
 size_t pcg_bytes(int chunk) { return 14 * (size_t)chunk; }
-using PcgKernel = void (*)(GridDev, float*, const float*, float*, const uint16_t*, FF, int, int, int*, GridWait);
+using PcgKernel = void (*)(GridDev, float*, const float*, float*, const uint16_t*, FF, int, int, int*, GridSync*,
+                           GridWait);
 PcgKernel pcg_kernel(int chunk) {
     if (chunk <= 4 * kPcgThr) return k_pcg_grid<1>;
     if (chunk <= 8 * kPcgThr) return k_pcg_grid<2>;
@@ -490,8 +468,9 @@ void launch_sor_grid(const GridDev& g, SolveWork& w, float omega, int sweeps, in
     const uint16_t* kd = reinterpret_cast<const uint16_t*>(w.kind);
     const float* r = w.r;
     GridDev gg = g;
-    GridWait gw{reinterpret_cast<GridSync*>(w.gpart), w.wait_polls, w.err, w.flag + 2};
-    cudaMemsetAsync(gw.sync, 0, sizeof(unsigned), s);
+    GridSync* sync = reinterpret_cast<GridSync*>(w.gpart);
+    GridWait gw{&sync->arrived, w.wait_polls, w.err, w.flag + 2};
+    cudaMemsetAsync(sync, 0, sizeof(unsigned), s);
     void* args[] = {&gg, &w.e, &r, &kd, &omega, &sweeps, &chunk, &gw};
     cudaLaunchCooperativeKernel((const void*)k_sor_grid, dim3((g.nv + chunk - 1) / chunk), dim3(kThr), args,
                                 sor_bytes(chunk), s);
@@ -502,10 +481,11 @@ void launch_pcg_grid(const GridDev& g, SolveWork& w, double target_rr, int cap, 
     GridDev gg = g;
     // the shared state lies in the node kernels' partial-sum buffer (kParts x 8 doubles at least)
     static_assert(sizeof(GridSync) <= sizeof(double) * 8 * kParts, "the partial-sum buffer holds the grid's state");
-    GridWait gw{reinterpret_cast<GridSync*>(w.gpart), w.wait_polls, w.err, w.flag + 2};
-    cudaMemsetAsync(gw.sync, 0, sizeof(unsigned), s);
+    GridSync* sync = reinterpret_cast<GridSync*>(w.gpart);
+    GridWait gw{&sync->arrived, w.wait_polls, w.err, w.flag + 2};
+    cudaMemsetAsync(sync, 0, sizeof(unsigned), s);
     FF t = ff_from_double(target_rr);
-    void* args[] = {&gg, &w.e, &r, &w.d, &kd, &t, &cap, &chunk, &w.flag, &gw};
+    void* args[] = {&gg, &w.e, &r, &w.d, &kd, &t, &cap, &chunk, &w.flag, &sync, &gw};
     cudaLaunchCooperativeKernel((const void*)pcg_kernel(chunk), dim3((g.nv + chunk - 1) / chunk), dim3(kPcgThr), args,
                                 pcg_bytes(chunk), s);
 }
