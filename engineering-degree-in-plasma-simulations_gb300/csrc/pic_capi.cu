@@ -476,6 +476,7 @@ void free_lp(pic_world* w) {
     }
     if (L->W) cudaFree(L->W);
     if (L->fold) cudaFree(L->fold);
+    if (L->dense) cudaFree(L->dense);
     lp_free_train(*L);
     delete L;
     w->lp = nullptr;
@@ -518,6 +519,18 @@ int ensure_lp(pic_world* w) {
     lp_layout(L->lay);
     CU(cudaMalloc(&L->W, sizeof(float) * L->lay.total));
     CU(cudaMalloc(&L->fold, sizeof(float) * kLpFoldStride * kLpNetLevels));
+    // the first level small enough for a dense matrix, if any
+    L->dense_level = L->nlev;
+    while (L->dense_level > 1 && L->dims[L->dense_level - 1][0] * L->dims[L->dense_level - 1][1] *
+                                         L->dims[L->dense_level - 1][2] <= kLpDenseMost)
+        L->dense_level--;
+    if (L->dense_level < L->nlev) {
+        const int* d = L->dims[L->dense_level];
+        const size_t n = (size_t)d[0] * d[1] * d[2];
+        L->dense_pitch = (int)(n + 3) / 4 * 4;
+        CU(cudaMalloc(&L->dense, sizeof(float) * n * L->dense_pitch));
+        CU(cudaMemsetAsync(L->dense, 0, sizeof(float) * n * L->dense_pitch, w->stream));  // the rows' padding
+    }
     std::vector<float> hw(L->lay.total);
     lp_init_weights(L->lay, L->diag, L->nlev, hw.data());
     CU(cudaMemcpyAsync(L->W, hw.data(), sizeof(float) * hw.size(), cudaMemcpyHostToDevice, w->stream));
@@ -1693,6 +1706,19 @@ int inner_wait_failed(pic_world* w) {
 // out in batches between which the host reads the stop flag (the iterations of a batch after the
 // stop return at once, about 30 us each at 256^3): first_batch, then 2, 4, 4, ...
 int learned_inner(pic_world* w, SolveWork& sw, double target, int cap, int first_batch, int* done, bool* conv) {
+    if (plan_lpcg_grid(w->g, *w->lp, w->sms)) {
+        // the whole solve in one launch; the residual's partner is the unused one of the two potentials
+        {
+            Scope sc(w, "poisson", 1);
+            launch_lpcg_grid(w->g, sw, *w->lp, w->d2, reinterpret_cast<float*>(sw.phi_alt), target, cap, w->stream, w->sms);
+        }
+        CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
+        CU(cudaStreamSynchronize(w->stream));
+        if (w->h_flag[2]) return inner_wait_failed(w);
+        *done = w->h_flag[1];
+        *conv = w->h_flag[0] != 0;
+        return PIC_OK;
+    }
     {
         Scope sc(w, "poisson", lp_apply_launches(*w->lp));
         launch_lpcg_init(w->g, sw, *w->lp, w->stream, w->sms);

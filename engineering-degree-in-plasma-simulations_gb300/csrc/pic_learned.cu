@@ -11,9 +11,8 @@
 #include <vector>
 #include <cuda_bf16.h>
 #include <cstring>
-#include "pic_grid_sync.cuh"
 #include "pic_learned.h"
-#include "pic_stencil.cuh"
+#include "pic_lp_levels.cuh"
 #include "pic_tc.cuh"
 
 namespace pic {
@@ -103,21 +102,6 @@ LView lp_level_view(const LpState& L, int l, float* a) {
 }
 LView lp_node_view(const GridDev& g, const LpState& L, float* a) {
     return lp_view(a, L.dims[0], g.ni, g.ni * g.nj, L.per);
-}
-
-__device__ __forceinline__ void lv_decode(const LView& v, unsigned idx, int& x, int& y, int& z) {
-    unsigned t = fdiv(idx, v.fx);
-    x = (int)(idx - t * (unsigned)v.n[0]);
-    unsigned zz = fdiv(idx, v.fxy);
-    z = (int)zz;
-    y = (int)(t - zz * (unsigned)v.n[1]);
-}
-__device__ __forceinline__ int lv_off(const LView& v, int x, int y, int z) { return x + y * v.sy + z * v.sz; }
-// coordinate c + d along an axis of extent n (|d| <= 2, n >= 2): wrapped, or -1 outside
-__device__ __forceinline__ int lv_nb(int c, int d, int n, int per) {
-    int u = c + d;
-    if (per) return u < 0 ? u + n : (u >= n ? u - n : u);
-    return (u < 0 || u >= n) ? -1 : u;
 }
 
 // z_coarse = R z_fine at coarse voxel idx
@@ -375,271 +359,23 @@ __global__ void k_lp_up(LView zin, LView cin, LView out, int mode, const float* 
         lp_up_at(zin, cin, out, mode, fold, fold_g, inv_diag, idx);
 }
 
-// ------------------------------------------------------------------------------------
-// The coarse part of the hierarchy, levels m .. nlev - 1, in one cooperative launch (one CTA per SM):
-// the restrictions down from level m - 1, then the level operators from the last level back up to m.
-//
-// As a launch per level and direction, with the coarsest levels in one CTA, this part was a chain of
-// latency-bound kernels: 9.7 + 8.0 (restrictions) + 32 (one CTA) + 10.8 + 10.7 us of the 145 us of an
-// iteration of 63 x 63 x 256 nodes, the same for grids of any size.  One launch takes 28 us.  Here
-//   - a level's voxels are spread over all SMs, with up to 32 lanes per voxel that share its taps (the
-//     64 points of a restriction, the 125 taps and 8 prolongation corners of an operator), so that a
-//     thread has few dependent reads and a level costs about one L2 latency and a grid barrier;
-//   - below level lr (at most kLpRedundant voxels) every CTA restricts for itself in shared memory, and
-//     from level le on (network levels of at most kLpRedundantNet voxels) it applies the operators for
-//     itself too, which needs no grid barrier.  (An operator's 125 taps on the 2048 voxels of the next
-//     level up took one CTA 41 000 cycles; spread over the GPU they take 9500, and a barrier 2700.)
-// ------------------------------------------------------------------------------------
-constexpr int kLpMidThreads = 512;
-constexpr int kLpMidMost = 65536;    // voxels of the first level that joins
-constexpr int kLpRedundant = 4096;   // voxels of the last level that the GPU restricts together
-constexpr int kLpRedundantNet = 512;  // voxels of a network level that every CTA computes for itself
+// the coarse levels as a launch of their own (lp_coarse_levels)
 struct LpMidArgs {
-    int m, lr, le, nlev;
-    LView f0;                        // level m - 1 (its restricted input; the residual if m == 1)
-    LView z[kLpMaxLevels], e[kLpMaxLevels];
-    const float* fold[kLpMaxLevels];  // folded stencils of a network level, nullptr: diagonal scaling
-    float inv_diag[kLpMaxLevels];
-    unsigned* left;                  // CTAs that have finished (the last one resets the barrier)
+    LpCoarseLevels lev;
+    unsigned* left;  // CTAs that have finished (the last one resets the barrier)
     GridWait wait;
 };
-// a value of a level: shared memory, or global memory that other CTAs write (L2)
-template <bool SH>
-__device__ __forceinline__ float lp_ld(const float* p) {
-    return SH ? *p : __ldcg(p);
-}
-// sum over the lanes of a voxel's group of S lanes (in its first lane)
-template <int S>
-__device__ __forceinline__ float lp_group_sum(float v) {
-#pragma unroll
-    for (int o = S / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, S);
-    return v;
-}
-// part `s` of S of (R f) at coarse voxel cc: the fine rows s, s + S, ... of its 16, four points each
-// (index rules of k_lp_restrict; points outside the box count zero)
-template <bool SH, int S>
-__device__ __forceinline__ float lp_restrict_part(const LView& f, const LView& c, const int (&cc)[3], int s) {
-    const float w4[4] = {0.25f, 0.75f, 0.75f, 0.25f};
-    auto map = [&](int ax, int k) {
-        int raw = 2 * cc[ax] + k - 1;
-        if (f.per[ax]) {
-            const int nc2 = 2 * c.n[ax];
-            raw = raw < 0 ? raw + nc2 : (raw >= nc2 ? raw - nc2 : raw);
-        }
-        return (unsigned)raw < (unsigned)f.n[ax] ? raw : -1;
-    };
-    int x[4];
-    float wx[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int u = map(0, k);
-        x[k] = max(u, 0);
-        wx[k] = u >= 0 ? w4[k] : 0.f;
-    }
-    float acc = 0.f;
-#pragma unroll
-    for (int q = 0; q < 16 / S; q++) {
-        const int row = s + q * S, ky = row & 3, kz = row >> 2;
-        const int y = map(1, ky), z = map(2, kz);
-        const bool in = y >= 0 && z >= 0;
-        const float wr = in ? ((ky == 0 || ky == 3) ? 0.25f : 0.75f) * ((kz == 0 || kz == 3) ? 0.25f : 0.75f) : 0.f;
-        const float* p = f.a + (in ? y * f.sy + z * f.sz : 0);
-        float a = 0.f;
-#pragma unroll
-        for (int k = 0; k < 4; k++) a += wx[k] * lp_ld<SH>(p + x[k]);
-        acc += wr * a;
-    }
-    return acc;
-}
-// part `s` of S of op(z) + P e at voxel c: the rows s, s + S, ... of the 25 rows of a network level's
-// 5 x 5 x 5 stencil (k5: its interior coefficients, shared; face points take their class's variant)
-// or the scaled value, and the corners s, s + S, ... of the prolongation (e.a null: none).  Taps outside
-// the box read a valid point with weight zero, so that up to five rows of loads are in flight together.
-template <bool ZSH, bool ESH, int S>
-__device__ __forceinline__ float lp_up_part(const LView& z, const LView& e, const float* k5,
-                                            const float* __restrict__ fold, float inv_diag, const int (&c)[3], int s) {
-    // coordinate c + d - 2 along an axis, and whether it lies in the box
-    auto nb = [&](int ax, int d, bool& in) {
-        int u = c[ax] + d - 2;
-        if (z.per[ax]) u = u < 0 ? u + z.n[ax] : (u >= z.n[ax] ? u - z.n[ax] : u);
-        in = (unsigned)u < (unsigned)z.n[ax];
-        return in ? u : c[ax];
-    };
-    constexpr int kCorners = (8 + S - 1) / S;
-    float ev[kCorners], ew[kCorners];
-#pragma unroll
-    for (int q = 0; q < kCorners; q++) {
-        const int k = s + q * S;
-        bool in = e.a && k < 8;
-        float w = 1.f;
-        int u[3];
-#pragma unroll
-        for (int ax = 0; ax < 3; ax++) {
-            const int b = (k >> ax) & 1, c0 = c[ax] >> 1;
-            u[ax] = b ? lv_nb(c0, (c[ax] & 1) ? 1 : -1, e.n[ax], e.per[ax]) : c0;
-            in = in && u[ax] >= 0;
-            w *= b ? 0.25f : 0.75f;
-        }
-        ew[q] = w;
-        ev[q] = in ? lp_ld<ESH>(e.a + lv_off(e, u[0], u[1], u[2])) : 0.f;
-    }
-    float acc = 0.f;
-    if (fold) {
-        int cls = 0, mul = 1;
-#pragma unroll
-        for (int ax = 0; ax < 3; ax++) {
-            if (!z.per[ax]) cls += mul * (c[ax] == 0 ? 1 : (c[ax] == z.n[ax] - 1 ? 2 : 0));
-            mul *= 3;
-        }
-        const float* kk = cls ? fold + kLpFold + 125 * cls : k5;
-        int x[5];
-        bool bx[5];
-#pragma unroll
-        for (int d = 0; d < 5; d++) x[d] = nb(0, d, bx[d]);
-        constexpr int kRows = (25 + S - 1) / S, kAtOnce = kRows < 5 ? kRows : 5;
-#pragma unroll
-        for (int q0 = 0; q0 < kRows; q0 += kAtOnce) {
-            float v[kAtOnce][5];
-#pragma unroll
-            for (int q = 0; q < kAtOnce; q++) {
-                const int row = s + (q0 + q) * S;
-                const int dz = row / 5, dy = row - 5 * dz;
-                bool iy, iz;
-                const int y = nb(1, dy, iy), zz = nb(2, dz, iz);
-                const bool in = q0 + q < kRows && row < 25 && iy && iz;
-                const float* p = z.a + (in ? y * z.sy + zz * z.sz : 0);
-#pragma unroll
-                for (int d = 0; d < 5; d++) v[q][d] = in && bx[d] ? lp_ld<ZSH>(p + x[d]) : 0.f;
-            }
-#pragma unroll
-            for (int q = 0; q < kAtOnce; q++) {
-                const float* kr = kk + 5 * min(s + (q0 + q) * S, 24);
-#pragma unroll
-                for (int d = 0; d < 5; d++) acc = fmaf(kr[d], v[q][d], acc);
-            }
-        }
-    } else if (s == 0) {
-        acc = inv_diag * lp_ld<ZSH>(z.a + lv_off(z, c[0], c[1], c[2]));
-    }
-#pragma unroll
-    for (int q = 0; q < kCorners; q++) acc = fmaf(ew[q], ev[q], acc);
-    return acc;
-}
-// lanes per voxel: as many as leave every thread of the grid busy
-__device__ __forceinline__ int lp_split(int nvox, int threads, int most) {
-    int s = 1;
-    while (s < most && nvox * s * 2 <= threads) s *= 2;
-    return s;
-}
-// voxel groups of S lanes over nthr threads, the thread's number t: body(voxel, lane, live) for every voxel,
-// whole warps together
-template <int S, class F>
-__device__ __forceinline__ void lp_voxels(int nvox, int t, int nthr, F body) {
-    for (int v0 = (t & ~31) / S; v0 < nvox; v0 += nthr / S) {
-        const int v = v0 + (t & 31) / S;
-        body(min(v, nvox - 1), (t & 31) % S, v < nvox);
-    }
-}
-template <bool SH>
-__device__ void lp_restrict_level(const LView& f, const LView& c, int t, int nthr) {
-    auto run = [&](auto sc) {
-        constexpr int S = decltype(sc)::value;
-        lp_voxels<S>(c.nvox, t, nthr, [&](int v, int s, bool live) {
-            int cc[3];
-            lv_decode(c, (unsigned)v, cc[0], cc[1], cc[2]);
-            const float a = lp_group_sum<S>(lp_restrict_part<SH, S>(f, c, cc, s));
-            if (s == 0 && live) c.a[v] = a;
-        });
-    };
-    switch (lp_split(c.nvox, nthr, 16)) {
-        case 1: run(std::integral_constant<int, 1>{}); break;
-        case 2: run(std::integral_constant<int, 2>{}); break;
-        case 4: run(std::integral_constant<int, 4>{}); break;
-        case 8: run(std::integral_constant<int, 8>{}); break;
-        default: run(std::integral_constant<int, 16>{}); break;
-    }
-}
-template <bool ZSH, bool ESH>
-__device__ void lp_up_level(const LView& z, const LView& e, const LView& out, const float* k5, const float* fold,
-                            float inv_diag, int t, int nthr) {
-    auto run = [&](auto sc) {
-        constexpr int S = decltype(sc)::value;
-        lp_voxels<S>(out.nvox, t, nthr, [&](int v, int s, bool live) {
-            int c[3];
-            lv_decode(out, (unsigned)v, c[0], c[1], c[2]);
-            const float a = lp_group_sum<S>(lp_up_part<ZSH, ESH, S>(z, e, k5, fold, inv_diag, c, s));
-            if (s == 0 && live) out.a[v] = a;
-        });
-    };
-    switch (lp_split(out.nvox, nthr, 32)) {
-        case 1: run(std::integral_constant<int, 1>{}); break;
-        case 2: run(std::integral_constant<int, 2>{}); break;
-        case 4: run(std::integral_constant<int, 4>{}); break;
-        case 8: run(std::integral_constant<int, 8>{}); break;
-        case 16: run(std::integral_constant<int, 16>{}); break;
-        default: run(std::integral_constant<int, 32>{}); break;
-    }
-}
-__global__ void __launch_bounds__(kLpMidThreads, 1) k_lp_mid(LpMidArgs a, const int* flag) {
+__global__ void __launch_bounds__(kLvThr, 1) k_lp_mid(const __grid_constant__ LpMidArgs a, const int* flag) {
     if (flag && flag[0]) return;  // every CTA alike: written by an earlier launch
     extern __shared__ __align__(16) float mid_dyn[];
-    __shared__ float k5[kLpNetLevels + 1][125];
+    LevelSmem& sm = *reinterpret_cast<LevelSmem*>(mid_dyn);
     __shared__ int s_fail;
-    const int tid = threadIdx.x, t = blockIdx.x * kLpMidThreads + tid, nthr = gridDim.x * kLpMidThreads;
-    if (tid == 0) s_fail = 0;
-    for (int l = a.m; l < a.nlev && l <= kLpNetLevels; l++)
-        for (int x = tid; x < 125; x += kLpMidThreads) k5[l][x] = a.fold[l][729 + x];
+    if (threadIdx.x == 0) s_fail = 0;
+    lp_load_levels(sm, a.lev, a.lev.m, a.lev.ld, kLvThr);
+    __syncthreads();
     unsigned target = 0;
-    bool ok = true;
-    for (int l = a.m; l <= a.lr && l < a.nlev && ok; l++) {
-        lp_restrict_level<false>(l == a.m ? a.f0 : a.z[l - 1], a.z[l], t, nthr);
-        ok = grid_barrier(a.wait, target, &s_fail);
-    }
-    LView none{};
-    none.a = nullptr;
-    LView esh = none;  // e of level le in this CTA's shared memory
-    if (ok && a.le < a.nlev) {
-        // z of levels lr .. nlev - 1 in shared memory, one after the other, then e of levels nlev - 1 .. le
-        float* p = mid_dyn;
-        LView zs = a.z[a.lr];
-        zs.a = p;
-        for (int x = tid; x < zs.nvox; x += kLpMidThreads) p[x] = __ldcg(a.z[a.lr].a + x);
-        p += zs.nvox;
-        __syncthreads();
-        for (int l = a.lr + 1; l < a.nlev; l++) {
-            LView c = a.z[l];
-            c.a = p;
-            p += c.nvox;
-            lp_restrict_level<true>(zs, c, tid, kLpMidThreads);
-            __syncthreads();
-            zs = c;
-        }
-        for (int l = a.nlev - 1; l >= a.le; l--) {
-            LView out = a.e[l];
-            out.a = p;
-            p += out.nvox;
-            lp_up_level<true, true>(zs, esh, out, k5[min(l, kLpNetLevels)], a.fold[l], a.inv_diag[l], tid, kLpMidThreads);
-            __syncthreads();
-            esh = out;
-            if (l > a.le) {
-                zs = a.z[l - 1];
-                float* q = mid_dyn;  // the z of level l - 1 lies behind those of levels lr .. l - 2
-                for (int k = a.lr; k < l - 1; k++) q += a.z[k].nvox;
-                zs.a = q;
-            }
-        }
-        if (a.le == a.m)  // no level above it here: its e goes out, each CTA its share
-            for (int x = t; x < esh.nvox; x += nthr) a.e[a.m].a[x] = esh.a[x];
-    }
-    for (int l = a.le - 1; l >= a.m && ok; l--) {
-        if (l == a.le - 1)
-            lp_up_level<false, true>(a.z[l], esh, a.e[l], k5[min(l, kLpNetLevels)], a.fold[l], a.inv_diag[l], t, nthr);
-        else
-            lp_up_level<false, false>(a.z[l], a.e[l + 1], a.e[l], k5[min(l, kLpNetLevels)], a.fold[l], a.inv_diag[l], t,
-                                      nthr);
-        if (l > a.m) ok = grid_barrier(a.wait, target, &s_fail);
-    }
-    if (tid == 0) {
+    const bool ok = lp_coarse_levels(sm.lev, sm, a.wait, target, &s_fail);
+    if (threadIdx.x == 0) {
         if (!ok) {
             set_error(a.wait.err, kErrBarrierTimeout);
             *a.wait.fail = 1;
@@ -648,6 +384,71 @@ __global__ void __launch_bounds__(kLpMidThreads, 1) k_lp_mid(LpMidArgs a, const 
             *a.wait.arrived = 0u;
         }
     }
+}
+
+// columns of the dense operator of level ld: op_ld + P (op_ld+1 + ...) R applied to the unit vectors, a
+// column per CTA and turn, all levels in shared memory
+struct LpDenseArgs {
+    LpCoarseLevels lev;  // from ld on
+    float* dense;
+    int pitch;
+};
+__global__ void __launch_bounds__(kLvThr, 1) k_lp_dense(const __grid_constant__ LpDenseArgs a) {
+    extern __shared__ __align__(16) float den_dyn[];
+    LevelSmem& sm = *reinterpret_cast<LevelSmem*>(den_dyn);
+    float* base = den_dyn + sizeof(LevelSmem) / 4;
+    const int ld = a.lev.m, nlev = a.lev.nlev, tid = threadIdx.x, n = a.lev.z[ld].nvox;
+    lp_load_levels(sm, a.lev, ld, nlev, kLvThr);
+    for (int col = blockIdx.x; col < n; col += gridDim.x) {
+        __syncthreads();
+        // z of levels ld .. nlev - 1 one after the other, then two e's that alternate
+        float* p = base;
+        LView zs = sm.lev.z[ld];
+        zs.a = p;
+        for (int x = tid; x < n; x += kLvThr) p[x] = x == col ? 1.f : 0.f;
+        p += n;
+        __syncthreads();
+        for (int l = ld + 1; l < nlev; l++) {
+            LView c = sm.lev.z[l];
+            c.a = p;
+            p += c.nvox;
+            lp_restrict_level<true>(zs, c, 0, 1);
+            __syncthreads();
+            zs = c;
+        }
+        LView up{};
+        for (int l = nlev - 1; l >= ld; l--) {
+            LView out = sm.lev.e[l];
+            out.a = p;
+            p += out.nvox;
+            LView zl = sm.lev.z[l];
+            zl.a = base;
+            for (int k = ld; k < l; k++) zl.a += sm.lev.z[k].nvox;
+            lp_up_level<true, true>(zl, up, out, l, sm.lev.fold[l], sm.lev.inv_diag[l], sm, 0, 1);
+            __syncthreads();
+            up = out;
+        }
+        for (int x = tid; x < n; x += kLvThr) a.dense[(size_t)x * a.pitch + col] = up.a[x];
+    }
+}
+void lp_build_dense(const LpState& L, cudaStream_t s) {
+    if (L.dense_valid || !L.dense) return;
+    LpDenseArgs a;
+    lp_coarse_setup(L, L.dense_level, LView{}, a.lev);
+    a.dense = L.dense;
+    a.pitch = L.dense_pitch;
+    size_t smem = sizeof(LevelSmem);
+    for (int l = L.dense_level; l < L.nlev; l++) smem += 2 * sizeof(float) * a.lev.z[l].nvox;
+    static int dyn_set = -1;  // the device whose attribute is set
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dyn_set != dev) {  // levels that halve only two axes add up to less than twice the first one
+        cudaFuncSetAttribute(k_lp_dense, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(LevelSmem) + 4 * (int)sizeof(float) * kLpDenseMost);
+        dyn_set = dev;
+    }
+    k_lp_dense<<<std::min(a.lev.z[L.dense_level].nvox, 1216), kLvThr, smem, s>>>(a);
+    L.dense_valid = true;
 }
 
 // level 0 on the node array: z = mask * (S0 * r + P e_1); with out != nullptr also z.r -> out[0]
@@ -687,14 +488,6 @@ __global__ void __launch_bounds__(kNodeThreads) k_lp_up0(GridDev g, LView rin, L
 
 constexpr int kUp0X = 32, kUp0Y = 8, kUp0Z = 8;
 constexpr int kUp0HX = kUp0X + 2, kUp0HY = kUp0Y + 2, kUp0HZ = kUp0Z + 2;
-__device__ __forceinline__ int lv_map(int u, int n, int per) {
-    if ((unsigned)u < (unsigned)n) return u;
-    if (!per) return -1;
-    // a tile past the end of a short periodic axis can reach beyond one period: reduce fully so
-    // that every staged read stays on the grid
-    const int m = u % n;
-    return m < 0 ? m + n : m;
-}
 // Stages a halo tile of HX x R values (R rows of HX) in shared memory: element e = hx + HX row
 // reads src[mx[hx] + myz[row]] (0 when either offset is -1).  The trip count is a constant, so
 // every load of a thread is issued before its first shared store.
@@ -1116,16 +909,6 @@ __global__ void __launch_bounds__(kNetX * kNetY, 2) k_lp_up_net_tiled(LView zin,
     plane(I4{}, I4{}, 11);
 }
 
-// index rule of the restriction along one axis (k_lp_restrict): fine point raw of coarse level c,
-// wrapped once by the coarse period on a periodic axis; -1 outside the fine box
-__device__ __forceinline__ int rs_map(int raw, const LView& f, const LView& c, int ax) {
-    if (f.per[ax]) {
-        const int nc2 = 2 * c.n[ax];
-        raw = raw < 0 ? raw + nc2 : (raw >= nc2 ? raw - nc2 : raw);
-        return raw < f.n[ax] ? raw : -1;
-    }
-    return (raw >= 0 && raw < f.n[ax]) ? raw : -1;
-}
 // z_coarse = R z_fine, one warp per column of 32 x 4 x 4 coarse voxels, all in registers.  Lane l
 // owns coarse x = cx0 + l.  The warp marches through the column's ten fine planes; in each it
 // reads the ten fine rows of the column, lane l taking fine x 2cx and 2cx + 1 as one float2 (a
@@ -1334,6 +1117,15 @@ static void launch_restrict(const LView& f, const LView& c, const int* flag, cud
     }
 }
 
+void lp_refresh_k5(const LpState& L, cudaStream_t s) {
+    if (L.k5_valid) return;
+    const int nnet = std::min(kLpNetLevels, L.nlev - 1);
+    for (int l = 1; l <= nnet; l++)
+        cudaMemcpyAsync(L.k5_host[l - 1], L.fold + (l - 1) * kLpFoldStride + 729, sizeof(float) * 125,
+                        cudaMemcpyDeviceToHost, s);
+    cudaStreamSynchronize(s);
+    L.k5_valid = true;
+}
 int lp_apply_launches(const LpState& L) {
     int n = 1;
     for (int l = 1; l < L.nlev; l++) {
@@ -1346,55 +1138,34 @@ void launch_lp_apply(const GridDev& g, const LpState& L, const SolveWork& w, con
                      bool sums, const int* flag, cudaStream_t s, int sms) {
     const uint16_t* kind = reinterpret_cast<const uint16_t*>(w.kind);
     LView r0 = lp_node_view(g, L, const_cast<float*>(r));
-    // levels m .. nlev - 1 in one launch; z below level lr and e from level le on by every CTA for itself
-    LpMidArgs ma{};
-    ma.m = ma.lr = ma.le = L.nlev;
-    for (int l = L.nlev - 1; l >= 1; l--) {
-        const int nv_l = L.dims[l][0] * L.dims[l][1] * L.dims[l][2];
-        if (nv_l <= kLpMidMost) ma.m = l;
-        if (nv_l <= kLpRedundant) ma.lr = l;
-        if (nv_l <= (l <= kLpNetLevels ? kLpRedundantNet : kLpRedundant)) ma.le = l;
-    }
-    const int l0 = ma.m;
+    // levels l0 .. nlev - 1 in one launch
+    int l0 = L.nlev;
+    while (l0 > 1 && L.dims[l0 - 1][0] * L.dims[l0 - 1][1] * L.dims[l0 - 1][2] <= kLpMidMost) l0--;
     for (int l = 1; l < l0; l++) {
         LView f = l == 1 ? r0 : lp_level_view(L, l - 1, L.z[l - 1]);
         LView c = lp_level_view(L, l, L.z[l]);
         launch_restrict(f, c, flag, s, sms);
     }
     if (l0 < L.nlev) {
-        ma.nlev = L.nlev;
-        ma.f0 = l0 == 1 ? r0 : lp_level_view(L, l0 - 1, L.z[l0 - 1]);
-        size_t smem = 0;
-        for (int l = l0; l < L.nlev; l++) {
-            ma.z[l] = lp_level_view(L, l, L.z[l]);
-            ma.e[l] = lp_level_view(L, l, L.e[l]);
-            ma.fold[l] = l <= kLpNetLevels ? L.fold + (l - 1) * kLpFoldStride : nullptr;
-            ma.inv_diag[l] = (float)(1.0 / L.diag[l]);
-            if (l >= ma.lr) smem += 2 * sizeof(float) * ma.z[l].nvox;
-        }
+        LpMidArgs ma;
+        lp_build_dense(L, s);
+        lp_coarse_setup(L, l0, l0 == 1 ? r0 : lp_level_view(L, l0 - 1, L.z[l0 - 1]), ma.lev);
         ma.left = w.ticket + 2;
         ma.wait = GridWait{w.ticket + 1, w.wait_polls, w.err, w.flag + 2};
         static int dyn_set = -1;  // the device whose attribute is set
         int dev = 0;
         cudaGetDevice(&dev);
-        if (dyn_set != dev) {  // levels that halve only two axes add up to less than twice the first one
-            cudaFuncSetAttribute(k_lp_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (int)sizeof(float) * kLpRedundant);
+        if (dyn_set != dev) {
+            cudaFuncSetAttribute(k_lp_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LevelSmem));
             dyn_set = dev;
         }
         void* args[] = {&ma, (void*)&flag};
-        cudaLaunchCooperativeKernel((const void*)k_lp_mid, dim3((unsigned)std::max(1, sms)), dim3(kLpMidThreads), args,
-                                    smem, s);
+        cudaLaunchCooperativeKernel((const void*)k_lp_mid, dim3((unsigned)std::max(1, sms)), dim3(kLvThr), args,
+                                    sizeof(LevelSmem), s);
     }
     LView none{};
     none.a = nullptr;
-    if (!L.k5_valid) {
-        const int nnet = std::min(kLpNetLevels, L.nlev - 1);
-        for (int l = 1; l <= nnet; l++)
-            cudaMemcpyAsync(L.k5_host[l - 1], L.fold + (l - 1) * kLpFoldStride + 729, sizeof(float) * 125,
-                            cudaMemcpyDeviceToHost, s);
-        cudaStreamSynchronize(s);
-        L.k5_valid = true;
-    }
+    lp_refresh_k5(L, s);
     for (int l = l0 - 1; l >= 1; l--) {
         LView zin = lp_level_view(L, l, L.z[l]);
         LView cin = l + 1 < L.nlev ? lp_level_view(L, l + 1, L.e[l + 1]) : none;
@@ -1476,7 +1247,7 @@ __global__ void k_lp_fold(const float* __restrict__ W, LpLayout lay, float* fold
     }
 }
 void launch_lp_fold(const LpState& L, cudaStream_t s) {
-    L.k5_valid = false;
+    L.k5_valid = L.dense_valid = false;
     int nnet = std::min(kLpNetLevels, L.nlev - 1);
     if (nnet > 0) k_lp_fold<<<nnet, 256, 0, s>>>(L.W, L.lay, L.fold);
 }

@@ -35,6 +35,7 @@ struct LpLayout {
     int wm[kLpNetLevels + 1];     // mix   [C][C] (out, in)
     int wp[kLpNetLevels + 1];     // proj  [27][C]
 };
+constexpr int kLpDenseMost = 2048;  // voxels of the level that is applied as a dense matrix, all below it included
 constexpr int kLpFold = 729 + 125;  // per network level: K27 [27][27] then K5 [125] (staged in shared memory)
 // then the 27 face-class variants of K5 [27][125] (class cx + 3 cy + 9 cz per axis: 0 away from a
 // non-periodic face, 1 on its low face, 2 on its high face; variant 0 is K5)
@@ -52,6 +53,11 @@ struct LpState {
     LpLayout lay{};
     float* W = nullptr;     // parameters (FP32 master copy)
     float* fold = nullptr;  // folded stencils, kLpFoldStride per network level (index l-1)
+    // the dense operator of level dense_level and all below it (rows of dense_pitch floats), formed on the
+    // first apply after a fold
+    float* dense = nullptr;
+    int dense_level = 0, dense_pitch = 0;
+    mutable bool dense_valid = false;
     LpTrain* train = nullptr;
     // host copy of every network level's K5, passed to the tiled level kernel as a parameter
     // (the constant bank feeds the FMAs directly); refreshed on the first apply after a fold
@@ -68,6 +74,7 @@ void lp_init_weights(const LpLayout& lay, const double* diag, int nlev, float* h
 void lp_galerkin_diag(const double c[3], int nlev, double* diag);
 
 void launch_lp_fold(const LpState& L, cudaStream_t s);
+void lp_build_dense(const LpState& L, cudaStream_t s);  // when the weights changed since the last call
 void lp_free_train(LpState& L);
 // training (see pic_learned.cu): allocation, bf16 operand copies, one loss + gradient evaluation,
 // a white-noise sample pair, one Adam step (followed by the bf16 copies and the folds)
@@ -98,12 +105,18 @@ unsigned* lp_train_err(const LpState& L);
 // w.flag[2] is set when a bounded wait ran out
 void launch_lp_apply(const GridDev& g, const LpState& L, const SolveWork& w, const float* r, float* z, const float* q,
                      bool sums, const int* flag, cudaStream_t s, int sms);
+void lp_refresh_k5(const LpState& L, cudaStream_t s);  // k5_host after a fold
 int lp_apply_launches(const LpState& L);  // kernels of one apply
 // flexible CG iteration with the learned preconditioner (see pic_learned.cu)
 void launch_lp_norm2(const float* a, int n, double* part, double* out, cudaStream_t s, int grid);
 void launch_lpcg_init(const GridDev& g, SolveWork& w, const LpState& L, cudaStream_t s, int sms);
 void launch_lpcg_iter(const GridDev& g, SolveWork& w, const LpState& L, float* d_in, float* d_out, int it,
                       double target_rr, cudaStream_t s, int sms);
+// the whole inner solve in one launch (pic_lpcg.cu): whether the grid takes it; e from zero, at most cap
+// iterations (w.flag[0] converged, [1] iterations, [2] a wait ran out); d2, r2: node arrays, scratch
+bool plan_lpcg_grid(const GridDev& g, const LpState& L, int sms);
+void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d2, float* r2, double target_rr, int cap,
+                      cudaStream_t s, int sms);
 void launch_lpcg_k1_probe(const GridDev& g, SolveWork& w, float* d_in, float* d_out, cudaStream_t s);
 
 }  // namespace pic

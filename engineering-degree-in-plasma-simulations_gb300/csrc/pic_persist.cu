@@ -25,15 +25,8 @@ namespace {
 
 constexpr int kThr = 1024;     // threads of the sweeps
 constexpr int kPcgThr = 512;   // threads of the CG: 128 registers hold a group's neighbour rows
-constexpr int kMostCtas = 512;             // partial sums held per slot
 constexpr size_t kSmemMost = 216 * 1024;   // dynamic shared memory of a CTA
 
-// what the CTAs of a launch share, the counter zero at launch
-struct GridSync {
-    unsigned arrived;
-    unsigned pad[31];
-    float2 part[4][kMostCtas];  // float-float partials: d.q, then the three sums after the update
-};
 // flags of a node: FREE (1), mirror mask (6 bits), wraps (6 bits: at the low / high end of a periodic
 // axis x, y, z); 0 for a node without an unknown
 __device__ __forceinline__ unsigned node_flags(const GridDev& g, int n, unsigned kd) {
@@ -155,74 +148,6 @@ __global__ void __launch_bounds__(kThr, 1) k_sor_grid(GridDev g, float* __restri
 // ------------------------------------------------------------------------------------
 // the whole inner CG solve of L e = r from e = 0 (the iteration of k_pcg_k1 / k_pcg_k2)
 // ------------------------------------------------------------------------------------
-// a + t, the high parts by TwoSum, the low parts collected (normalised once at the end of a sum)
-__device__ __forceinline__ FF ff_gather(FF a, FF t) {
-    const FF s = two_sum(a.hi, t.hi);
-    return FF{s.hi, a.lo + (t.lo + s.lo)};
-}
-constexpr int kAtOnce = 5;  // partials a lane reads at once: 152 CTAs in one go
-// Sums of N per-thread values over the grid, in every lane of warp 0 of every CTA: FP32 within a warp,
-// float-float over the warps and the CTAs, in a fixed order; passes one grid barrier (false: it failed).
-// part: the N slots of this sum, not read by anyone since the last barrier but one.
-template <int N>
-__device__ __forceinline__ bool grid_total(const float (&v)[N], float (*wsum)[kPcgThr / 32], float2 (*part)[kMostCtas],
-                                           const GridWait& w, unsigned& target, int* s_fail, FF (&out)[N]) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    float x[N];
-#pragma unroll
-    for (int c = 0; c < N; c++) x[c] = v[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < N; c++) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
-    if (lane == 0)
-#pragma unroll
-        for (int c = 0; c < N; c++) wsum[c][wp] = x[c];
-    auto tree = [&]() {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int c = 0; c < N; c++)
-                out[c] = ff_gather(out[c], FF{__shfl_xor_sync(0xffffffffu, out[c].hi, o),
-                                              __shfl_xor_sync(0xffffffffu, out[c].lo, o)});
-#pragma unroll
-        for (int c = 0; c < N; c++) out[c] = two_sum(out[c].hi, out[c].lo);
-    };
-    __syncthreads();
-    if (wp == 0) {
-#pragma unroll
-        for (int c = 0; c < N; c++) out[c] = FF{lane < kPcgThr / 32 ? wsum[c][lane] : 0.f, 0.f};
-        tree();
-        if (lane == 0)
-#pragma unroll
-            for (int c = 0; c < N; c++) __stcg(&part[c][blockIdx.x], make_float2(out[c].hi, out[c].lo));
-    }
-    const bool ok = grid_barrier(w, target, s_fail);
-    if (wp == 0) {
-#pragma unroll
-        for (int c = 0; c < N; c++) out[c] = FF{0.f, 0.f};
-        for (int b0 = lane; b0 < (int)gridDim.x; b0 += 32 * kAtOnce) {
-            float2 t[kAtOnce][N];  // every load in flight before the first is used: one L2 latency
-#pragma unroll
-            for (int u = 0; u < kAtOnce; u++)
-#pragma unroll
-                for (int c = 0; c < N; c++)
-                    t[u][c] = b0 + 32 * u < (int)gridDim.x ? __ldcg(&part[c][b0 + 32 * u]) : make_float2(0.f, 0.f);
-#pragma unroll
-            for (int u = 0; u < kAtOnce; u++)
-#pragma unroll
-                for (int c = 0; c < N; c++) out[c] = ff_gather(out[c], FF{t[u][c].x, t[u][c].y});
-        }
-        tree();
-    }
-    return ok;
-}
-__device__ __forceinline__ float ff_ratio(FF a, FF b) {  // a / b rounded to FP32
-    const float q = a.hi / b.hi;
-    const float rem = fmaf(-q, b.hi, a.hi) + (a.lo - q * b.lo);
-    return q + rem / b.hi;
-}
-
 // flag[0]: converged (r.r <= target), flag[1]: iterations done.  A thread owns the groups of four
 // consecutive nodes tid + m kPcgThr (m < K) of its CTA's range: d, r and e of a group are one 16-byte word of
 // shared memory each, q stays in registers.  What bounds a pass is the latency of the L2 reads of other
@@ -276,7 +201,7 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
     float2(*part3)[kMostCtas] = sync->part + 1;
     unsigned target = 0;
     FF t1[1], t3[3];
-    grid_total<3>(f3, wsum, part3, wait, target, &s_fail, t3);  // r.z
+    grid_total<3, kPcgThr>(f3, wsum, part3, wait, target, &s_fail, t3);  // r.z
     FF rz = t3[0];
     const float inv0 = inv[0], dia0 = dia[0];
     __syncthreads();
@@ -378,7 +303,7 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
                 v1[0] += dv[c] * Q[m][c];
             }
         }
-        grid_total<1>(v1, wsum, part1, wait, target, &s_fail, t1);
+        grid_total<1, kPcgThr>(v1, wsum, part1, wait, target, &s_fail, t1);
         if (tid == 0) s_alpha = t1[0].hi != 0.f ? ff_ratio(rz, t1[0]) : 0.f;
         __syncthreads();
         if (s_fail) break;
@@ -406,7 +331,7 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
             X4[q] = make_float4(xv[0], xv[1], xv[2], xv[3]);
             R4[q] = make_float4(rn[0], rn[1], rn[2], rn[3]);
         }
-        grid_total<3>(v3, wsum, part3, wait, target, &s_fail, t3);
+        grid_total<3, kPcgThr>(v3, wsum, part3, wait, target, &s_fail, t3);
         it++;
         if (tid == 0) {
             const float over = (t3[2].hi - target_rr.hi) + (t3[2].lo - target_rr.lo);
