@@ -52,7 +52,9 @@ __host__ __device__ inline long long wait_poll_limit(long long arg, long long df
 constexpr long long kMbarWaitPolls = 1ll << 24;
 
 // particles
-int push_blocks_per_sm();  // resident push CTAs per SM (the push grid is this times the SM count)
+// most push CTAs per SM, counted as CTAs of 256 threads (two of the kernel's); a push grid is a number of
+// those times the SM count
+int push_blocks_per_sm();
 void launch_push(const PushArgs& a, cudaStream_t s, int grid);
 // collisions of a.coll for the electrons a.sp as two passes (candidates, their collisions); the
 // push that follows runs without collisions.  cand holds up to the species capacity.

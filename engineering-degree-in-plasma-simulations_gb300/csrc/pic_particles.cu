@@ -16,18 +16,20 @@
 
 namespace pic {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;
 constexpr int kPPT = 4;                     // particles per thread per chunk
 constexpr int kChunk = kThreads * kPPT;     // particles per chunk
-constexpr int kSeg = 256;                   // nodes per staged row segment
+constexpr int kSeg = 108;                   // nodes per staged row segment
 constexpr int kMargin = 2;                  // deposit window starts this many nodes below the gather window
 constexpr int kHalfWin = (kSeg - kMargin - 2) / 2;  // staged base nodes either side of the chunk's anchor
-constexpr int kPushBlocksPerSM = 3;         // resident push CTAs per SM (80 registers, 56 KB shared)
-// shared memory of the push: the next chunk's particles (pos, vel), the E rows (float4) and the
-// fixed-point deposit tile (a low-word and a high-word plane of 32-bit counters), four rows of
-// kSeg nodes each
+constexpr int kPushBlocksPerSM = 8;         // resident push CTAs per SM (64 registers, 27 KB shared)
+constexpr int kCtasPerShape = 2;            // a launch shape counts 256 threads
+// shared memory of the push: the chunk's particles (pos, vel), the E rows (float4), the fixed-point
+// deposit tile (a low-word and a high-word plane of 32-bit counters), four rows of kSeg nodes each,
+// and the list of the second pass
 constexpr size_t kPbufBytes = (size_t)kChunk * 2 * sizeof(float4);
-constexpr size_t kPushSmem = kPbufBytes + 4 * kSeg * sizeof(float4) + 2 * 4 * kSeg * sizeof(unsigned);
+constexpr size_t kPushSmem =
+    kPbufBytes + 4 * kSeg * sizeof(float4) + 2 * 4 * kSeg * sizeof(unsigned) + kChunk * sizeof(unsigned short);
 constexpr long long kWaitLimit = kMbarWaitPolls;  // mbarrier polls of a drain before giving up
 
 // ------------------------------------------------------------------------------------
@@ -39,8 +41,12 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// bytes of the current phase's copies; the phase ends when they have landed and mbar_arrive has been called
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
     unsigned ok;
@@ -128,30 +134,16 @@ __device__ float3 new_vel_electron(const CollDev& c, float E, float3 u, float r_
 // push helpers
 // ------------------------------------------------------------------------------------
 struct Tile {
-    const float4* etile;  // staged E rows (row m at etile + m*kSeg), or nullptr
     unsigned* dtile;      // deposit tile: low words of row m at dtile + m*kSeg, high words 4*kSeg on, or nullptr
     int lo;               // first base node of the staged window
-    int span;             // base nodes lo .. lo + span are staged
+    int bases;            // base nodes lo .. lo + bases - 1 are staged
     int off[4];           // node offsets of the four rows: 0, ni, ni*nj, ni*nj+ni
 };
 
-// E at the eight corners of the cell whose base node is b (Field::gather order)
-__device__ __forceinline__ float3 gather_e(const PushArgs& a, const Tile& t, int b, float3 o) {
-    const float4* e0;
-    int r1, r2, r3;
-    if (t.etile && (unsigned)(b - t.lo) <= (unsigned)t.span) {
-        e0 = t.etile + (b - t.lo);
-        r1 = kSeg;
-        r2 = 2 * kSeg;
-        r3 = 3 * kSeg;
-    } else {
-        e0 = a.ef + b;
-        r1 = t.off[1];
-        r2 = t.off[2];
-        r3 = t.off[3];
-    }
-    float4 e000 = e0[0], e100 = e0[1], e010 = e0[r1], e110 = e0[r1 + 1];
-    float4 e001 = e0[r2], e101 = e0[r2 + 1], e011 = e0[r3], e111 = e0[r3 + 1];
+// E at the eight corners of a cell (Field::gather order); e0: its base node's, r1 .. r3: its rows' offsets
+__device__ __forceinline__ float3 gather_e(const float4* e0, int r1, int r2, int r3, float3 o) {
+    const float4 e000 = e0[0], e100 = e0[1], e010 = e0[r1], e110 = e0[r1 + 1];
+    const float4 e001 = e0[r2], e101 = e0[r2 + 1], e011 = e0[r3], e111 = e0[r3 + 1];
     // trilinear weights as three nested linear interpolations (x, then y, then z)
     auto lx = [&](const float4& p, const float4& q) {
         return make_float3(fmaf(o.x, q.x - p.x, p.x), fmaf(o.x, q.y - p.y, p.y), fmaf(o.x, q.z - p.z, p.z));
@@ -179,11 +171,13 @@ __device__ __forceinline__ int move_particle(const PushArgs& a, int i, int j, in
     o.x = fminf(ox - fx, kBelowOne);
     o.y = fminf(oy - fy, kBelowOne);
     o.z = fminf(oz - fz, kBelowOne);
-    // periodic wrap: one unsigned compare per axis, the modulo only for a particle outside
-    if (g.periodic[0] && (unsigned)i >= (unsigned)g.ci) i = ((i % g.ci) + g.ci) % g.ci;
-    if (g.periodic[1] && (unsigned)j >= (unsigned)g.cj) j = ((j % g.cj) + g.cj) % g.cj;
-    if (g.periodic[2] && (unsigned)k >= (unsigned)g.ck) k = ((k % g.ck) + g.ck) % g.ck;
-    if ((unsigned)i >= (unsigned)g.ci || (unsigned)j >= (unsigned)g.cj || (unsigned)k >= (unsigned)g.ck) return -1;
+    // one branch for the particles that are outside on any axis: the wrap of periodic ones, else they leave
+    if ((unsigned)i >= (unsigned)g.ci || (unsigned)j >= (unsigned)g.cj || (unsigned)k >= (unsigned)g.ck) {
+        if (g.periodic[0]) i = ((i % g.ci) + g.ci) % g.ci;
+        if (g.periodic[1]) j = ((j % g.cj) + g.cj) % g.cj;
+        if (g.periodic[2]) k = ((k % g.ck) + g.ck) % g.ck;
+        if ((unsigned)i >= (unsigned)g.ci || (unsigned)j >= (unsigned)g.cj || (unsigned)k >= (unsigned)g.ck) return -1;
+    }
     if (g.zslab && slab_local_z(g, k) == g.zslab - 1) return -1;  // the cell between two instance slabs
     if (g.n_boxes) {
         float X = ((float)i + o.x) * g.dx[0], Y = ((float)j + o.y) * g.dx[1], Z = ((float)k + o.z) * g.dx[2];
@@ -266,20 +260,18 @@ __device__ __forceinline__ void corner_values32(float s, float3 o, Corners32& c,
 #pragma unroll
     for (int c8 = 0; c8 < 8; c8++) c.q[c8] = add ? c.q[c8] + v[c8] : v[c8];
 }
-// commits a light run: the eight adds are issued before any returned word is examined
-__device__ __forceinline__ void commit_run32(const PushArgs& a, const Tile& t, int b, const Corners32& c) {
-    int loc = b - (t.lo - kMargin);
-    if (t.dtile && loc >= 0 && loc < kSeg - 1) {
-        unsigned old[8];
+// commits a light run to the tile: the eight adds are issued before any returned word is examined, and one
+// branch looks at all carries
+__device__ __forceinline__ void commit_run32(unsigned* dt, const Corners32& c) {
+    unsigned old[8], carry = 0;
 #pragma unroll
-        for (int c8 = 0; c8 < 8; c8++) old[c8] = atomicAdd(&t.dtile[((c8 >> 1) * kSeg) + loc + (c8 & 1)], c.q[c8]);
+    for (int c8 = 0; c8 < 8; c8++) old[c8] = atomicAdd(&dt[((c8 >> 1) * kSeg) + (c8 & 1)], c.q[c8]);
 #pragma unroll
-        for (int c8 = 0; c8 < 8; c8++)
-            if (old[c8] + c.q[c8] < c.q[c8]) atomicAdd(&t.dtile[4 * kSeg + ((c8 >> 1) * kSeg) + loc + (c8 & 1)], 1u);
-    } else {
-#pragma unroll
-        for (int c8 = 0; c8 < 8; c8++)
-            if (c.q[c8]) atomicAdd(&a.sp.acc[b + t.off[c8 >> 1] + (c8 & 1)], (unsigned long long)c.q[c8]);
+    for (int c8 = 0; c8 < 8; c8++) carry |= old[c8] + c.q[c8] < c.q[c8] ? 1u << c8 : 0u;
+    while (carry) {
+        const int c8 = __ffs(carry) - 1;
+        carry &= carry - 1;
+        atomicAdd(&dt[4 * kSeg + (c8 >> 1) * kSeg + (c8 & 1)], 1u);
     }
 }
 
@@ -368,23 +360,37 @@ __device__ __noinline__ Collision collide_candidate(const CollDev& cd, unsigned 
 
 // ------------------------------------------------------------------------------------
 // push + deposit (collisions run before it, k_mcc_candidates / k_mcc_collide)
-//   A CTA takes chunks of 1024 particles (4 consecutive per thread), software-pipelined: the
-//   next chunk's particle arrays are bulk-copied (TMA) into shared memory while the current
-//   chunk is processed.  For each chunk the four node rows around the base node of its middle
-//   particle, [lo + off_m, lo + off_m + L), are bulk-copied into shared memory; the gather reads
-//   them there, and the deposit accumulates into a shared 64-bit fixed-point tile (two 32-bit
-//   word planes) committed to HBM with one atomic per touched node.  Particles outside the window
-//   use HBM directly.
+//   A CTA takes chunks of 512 particles, four consecutive ones a thread.  The particle arrays of a chunk and
+//   the four node rows around the base node of its middle particle, [lo + off_m, lo + off_m + L), are
+//   bulk-copied (TMA) into shared memory; particles are pushed in place and bulk-copied back, so that
+//   neither direction runs through the load-store units with a 64-byte stride; the deposit accumulates into
+//   a shared 64-bit fixed-point tile (two 32-bit word planes) committed to HBM with one atomic per touched
+//   node.  Particles outside the window, and deposits that leave it, go to HBM in a second pass over a list.
+//
+//   What bounds it: shared-memory wavefronts (62 % of the pipe, 90 a warp and turn: eight 16-byte reads of E,
+//   the particles in and out, the deposit's atomics) and issue slots (60 %), with barriers between the phases;
+//   hence many small CTAs: 8 of 128 threads, chunks of 512.  16 M particles on 97 x 113 x 129 nodes,
+//   0.324 -> 0.225 ms (1.02 GB, 0.15 ms at the copy rate); 2 x 100 M, 20 pushes: 39.0 -> 28.1 ms.  Measured
+//   on the way: 4 CTAs of 256 threads 30.1, 7 of 128 29.1, 14 of 64 31.7, 2 of 512 50 ms; E and deposits outside
+//   the window in line with the others (taken by 30 to 60 % of the warps' turns) 5 % slower.
 // ------------------------------------------------------------------------------------
-// bulk copy of one full chunk's particle arrays into the staging buffer
-__device__ __forceinline__ void issue_chunk(const SpeciesDev& sp, int base, float4* ppos, float4* pvel,
-                                            unsigned long long* bar) {
-    const unsigned b16 = kChunk * sizeof(float4);
-    fence_proxy_async();
-    mbar_expect_tx(bar, 2 * b16);
-    bulk_g2s(ppos, sp.pos + base, b16, bar);
-    bulk_g2s(pvel, sp.vel + base, b16, bar);
+// shared -> global bulk copy of the issuing thread's bulk group; addresses and size as above
+__device__ __forceinline__ void bulk_s2g(void* dst, const void* src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
+                 : "memory");
 }
+
+// warp-aggregated record of the particles that left the domain; all lanes call it
+__device__ __forceinline__ void record_dead(const PushArgs& a, bool dead, int p, int lane) {
+    const unsigned dm = __ballot_sync(0xffffffffu, dead);
+    if (!dm) return;
+    int b0 = 0;
+    if (lane == 0) b0 = atomicAdd(&a.sp.counts[2], __popc(dm));
+    b0 = __shfl_sync(0xffffffffu, b0, 0);
+    if (dead) a.sp.dead[b0 + __popc(dm & ((1u << lane) - 1u))] = p;
+}
+constexpr unsigned kDepositOnly = 1u << 15;  // list entry of a particle that has been pushed
+static_assert(kChunk <= (int)kDepositOnly, "a slot and the flag share a 16-bit word");
 
 __global__ void __launch_bounds__(kThreads, kPushBlocksPerSM) k_push(PushArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -392,8 +398,9 @@ __global__ void __launch_bounds__(kThreads, kPushBlocksPerSM) k_push(PushArgs a)
     float4* pvel = ppos + kChunk;
     float4* etile = reinterpret_cast<float4*>(smem + kPbufBytes);
     unsigned* dtile = reinterpret_cast<unsigned*>(etile + 4 * kSeg);
-    __shared__ __align__(8) unsigned long long bar_p, bar_e;
-    __shared__ int s_fail;
+    __shared__ __align__(8) unsigned long long bar;
+    __shared__ int s_lo, s_hi, s_moved, s_later;
+    unsigned short* later = reinterpret_cast<unsigned short*>(dtile + 8 * kSeg);  // slots left for the second pass
 
     const GridDev& g = a.g;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -401,15 +408,6 @@ __global__ void __launch_bounds__(kThreads, kPushBlocksPerSM) k_push(PushArgs a)
     const int nchunks = (n + kChunk - 1) / kChunk;
     const int nij = g.ni * g.nj;
 
-    if (tid == 0) {
-        mbar_init(&bar_p, 1);
-        mbar_init(&bar_e, 1);
-        fence_mbar_init();
-        s_fail = 0;
-    }
-    __syncthreads();
-    unsigned phase_p = 0, phase_e = 0;
-    const long long wait_lim = wait_poll_limit(a.wait_polls, kWaitLimit);
     Tile t;
     t.off[0] = 0;
     t.off[1] = g.ni;
@@ -417,185 +415,215 @@ __global__ void __launch_bounds__(kThreads, kPushBlocksPerSM) k_push(PushArgs a)
     t.off[3] = nij + g.ni;
     // last base node whose eight corners exist: the window must not copy past the node array
     const int max_base = g.nv - 2 - t.off[3];
+    const long long wait_lim = wait_poll_limit(a.wait_polls, kWaitLimit);
 
+    auto full = [&](int ch) { return (ch + 1) * kChunk <= n; };
+    // cell of a chunk's middle particle
+    auto middle = [&](int ch) {
+        return ch < nchunks ? __float_as_int(a.sp.pos[ch * kChunk + (min(kChunk, n - ch * kChunk) >> 1)].w) : -1;
+    };
+    // thread 0: the bulk copies of a full chunk's particles, once the chunk before has been stored
+    auto issue_particles = [&](int ch) {
+        if (!full(ch)) return;
+        const unsigned pb = kChunk * sizeof(float4);
+        fence_proxy_async();
+        mbar_expect_tx(&bar, 2 * pb);
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        bulk_g2s(ppos, a.sp.pos + ch * kChunk, pb, &bar);
+        bulk_g2s(pvel, a.sp.vel + ch * kChunk, pb, &bar);
+    };
+    // thread 0: window of chunk ch, +-kHalfWin base nodes around its middle particle's base node (cell c), and
+    // the bulk copies of its E rows
+    auto issue_window = [&](int c) {
+        int lo = 0, hi = -1;
+        if (a.staged && c >= 0) {
+            const int anchor = cell_base(g, c);
+            lo = max(0, anchor - kHalfWin);
+            hi = min(anchor + kHalfWin, max_base);
+        }
+        s_lo = lo;
+        s_hi = hi;
+        if (hi < lo) return;
+        const unsigned eb = (unsigned)(hi - lo + 2) * (unsigned)sizeof(float4);
+        fence_proxy_async();
+        mbar_expect_tx(&bar, 4 * eb);
+#pragma unroll
+        for (int m = 0; m < 4; m++) bulk_g2s(etile + m * kSeg, a.ef + lo + t.off[m], eb, &bar);
+    };
+
+    unsigned phase = 0;
     int moved = 0;  // particles of this thread that changed cell or left, over all its chunks
     int ch = blockIdx.x;
-    bool pending = false;  // a particle bulk copy into the staging buffer is in flight
-    if (ch < nchunks && (ch + 1) * kChunk <= n && tid == 0) issue_chunk(a.sp, ch * kChunk, ppos, pvel, &bar_p);
-    pending = ch < nchunks && (ch + 1) * kChunk <= n;
-
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+        s_moved = 0;
+        if (ch < nchunks) {
+            issue_particles(ch);
+            issue_window(middle(ch));
+            mbar_arrive(&bar);
+        }
+    }
     for (; ch < nchunks; ch += gridDim.x) {
         const int base = ch * kChunk;
         const int nin = min(kChunk, n - base);
-        // ---- this chunk's particles into registers (staged by TMA, or loaded here for the last,
-        // partial chunk)
-        if (pending) {
-            if (!mbar_wait_bounded(&bar_p, phase_p, wait_lim)) atomicExch(&s_fail, 1);
-            phase_p ^= 1u;
-            pending = false;
-            __syncthreads();
-            if (s_fail) {
-                if (tid == 0) set_error(a.err, kErrBarrierTimeout);
-                mbar_wait_bounded(&bar_p, phase_p ^ 1u);  // the copy in flight, bounded
-                return;
-            }
-        } else {
+        if (a.deposit)
+            for (int x = tid; x < 2 * kSeg; x += kThreads) reinterpret_cast<uint4*>(dtile)[x] = make_uint4(0u, 0u, 0u, 0u);
+        if (tid == 0) s_later = 0;
+        if (!full(ch))
             for (int x = tid; x < nin; x += kThreads) {
                 ppos[x] = a.sp.pos[base + x];
                 pvel[x] = a.sp.vel[base + x];
             }
-            __syncthreads();
-        }
-        // A thread owns particles tid*4 .. tid*4+3.  Read in place, the eight threads of a
-        // quarter-warp would hit the same banks four times over (64-byte stride); reading them in
-        // an order rotated by (lane/2) mod 4 spreads the reads over all 32 banks, and two
-        // conditional register rotations restore the order.
-        float4 P[kPPT], V[kPPT];
-        {
-            const int rot = (lane >> 1) & 3;
-#pragma unroll
-            for (int q = 0; q < kPPT; q++) {
-                const int x = tid * kPPT + ((q + rot) & 3);
-                P[q] = ppos[x];
-                V[q] = pvel[x];
-            }
-            if (rot & 1) {  // U[k] = T[k - 1]
-                const float4 p3 = P[3], v3 = V[3];
-                P[3] = P[2], P[2] = P[1], P[1] = P[0], P[0] = p3;
-                V[3] = V[2], V[2] = V[1], V[1] = V[0], V[0] = v3;
-            }
-            if (rot & 2) {  // P[k] = U[k - 2]
-                float4 t0 = P[0], t1 = P[1];
-                P[0] = P[2], P[1] = P[3], P[2] = t0, P[3] = t1;
-                t0 = V[0], t1 = V[1];
-                V[0] = V[2], V[1] = V[3], V[2] = t0, V[3] = t1;
-            }
-        }
-        // particles past the end of a partial chunk are marked absent
-#pragma unroll
-        for (int q = 0; q < kPPT; q++)
-            if (tid * kPPT + q >= nin) P[q].w = __int_as_float(-1);
-        // ---- window: +-kHalfWin base nodes around the base node of the chunk's middle particle
-        int lo = 0, hi = -1;
-        {
-            const int c = __float_as_int(ppos[nin >> 1].w);
-            if (c >= 0) {
-                const int anchor = cell_base(g, c);
-                lo = max(0, anchor - kHalfWin);
-                hi = min(anchor + kHalfWin, max_base);
-            }
-        }
-        const bool use_tile = a.staged && hi >= lo;
-        __syncthreads();  // every thread has read the staging buffer
-        if (tid == 0) {
-            if (use_tile) {
-                const unsigned bytes = (unsigned)(hi - lo + 2) * (unsigned)sizeof(float4);
-                fence_proxy_async();
-                mbar_expect_tx(&bar_e, 4 * bytes);
-#pragma unroll
-                for (int m = 0; m < 4; m++) bulk_g2s(etile + m * kSeg, a.ef + lo + t.off[m], bytes, &bar_e);
-            }
-            const int nx = ch + gridDim.x;
-            if (nx < nchunks && (nx + 1) * kChunk <= n) issue_chunk(a.sp, nx * kChunk, ppos, pvel, &bar_p);
-        }
-        {
-            const int nx = ch + gridDim.x;
-            pending = nx < nchunks && (nx + 1) * kChunk <= n;
-        }
-        t.lo = lo;
-        t.span = hi - lo;
-        t.etile = nullptr;
-        t.dtile = nullptr;
-        if (use_tile) {
-            if (a.deposit)
-                for (int x = tid; x < 8 * kSeg; x += kThreads) dtile[x] = 0u;
-            if (!mbar_wait_bounded(&bar_e, phase_e, wait_lim)) atomicExch(&s_fail, 1);
-            phase_e ^= 1u;
-            __syncthreads();
-            if (s_fail) {
-                // a copy did not complete in time: record it, wait once more (bounded) for the
-                // copies in flight, and leave without touching the tile
-                if (tid == 0) set_error(a.err, kErrBarrierTimeout);
-                mbar_wait_bounded(&bar_e, phase_e ^ 1u);
-                if (pending) mbar_wait_bounded(&bar_p, phase_p);
-                return;
-            }
-            t.etile = etile;
-            if (a.deposit) t.dtile = dtile;
-        }
-
-        unsigned dead_mask[kPPT];
-        Corners32 run;      // deposit sums of the current run of light particles
-        int run_cell = -1;  // packed cell of the run, -1: none
-#pragma unroll
-        for (int q = 0; q < kPPT; q++) {
-            const int p = base + tid * kPPT + q;
-            dead_mask[q] = 0;
-            int c = __float_as_int(P[q].w);
-            if (c < 0) continue;
-            int i, j, k;
-            cell_ijk(g, c, i, j, k);
-            float3 o = make_float3(P[q].x, P[q].y, P[q].z);
-            float3 v = make_float3(V[q].x, V[q].y, V[q].z);
-            const float w = V[q].w;
-            // leapfrog push (Species.cpp:369-373)
-            float3 E = gather_e(a, t, cell_base(g, c), o);
-            v.x += a.qm_dt * E.x;
-            v.y += a.qm_dt * E.y;
-            v.z += a.qm_dt * E.z;
-            const int newc = move_particle(a, i, j, k, o, v);
-            moved += newc != c;
-            a.sp.pos[p] = make_float4(o.x, o.y, o.z, __int_as_float(newc));
-            a.sp.vel[p] = make_float4(v.x, v.y, v.z, w);
-            if (newc >= 0) {
-                if (a.deposit) {
-                    const float s = w * a.dep_scale;
-                    if (s < kLightMax) {
-                        if (newc != run_cell && run_cell >= 0)
-                            commit_run32(a, t, cell_base(g, run_cell), run);
-                        corner_values32(s, o, run, newc == run_cell);
-                        run_cell = newc;
-                    } else {
-                        Corners hc;
-                        corner_values(w, o, a.dep_scale, hc, false);
-                        commit_corners(a, t, cell_base(g, newc), hc);
-                    }
-                }
-            } else {
-                dead_mask[q] = 1;
-            }
-        }
-        if (run_cell >= 0)
-            commit_run32(a, t, cell_base(g, run_cell), run);
-        // warp-aggregated record of the particles that left the domain
-#pragma unroll
-        for (int q = 0; q < kPPT; q++) {
-            unsigned dm = __ballot_sync(0xffffffffu, dead_mask[q] != 0);
-            if (dm) {
-                int b0 = 0;
-                if (lane == __ffs(dm) - 1) b0 = atomicAdd(&a.sp.counts[2], __popc(dm));
-                b0 = __shfl_sync(0xffffffffu, b0, __ffs(dm) - 1);
-                if (dead_mask[q]) a.sp.dead[b0 + __popc(dm & ((1u << lane) - 1u))] = base + tid * kPPT + q;
-            }
-        }
         __syncthreads();
-        if (use_tile && a.deposit) {
+        t.lo = s_lo;
+        t.bases = s_hi - t.lo + 1;
+        const bool use_tile = t.bases > 0;
+        const int fail = !mbar_wait_bounded(&bar, phase, wait_lim);
+        phase ^= 1u;
+        if (__syncthreads_or(fail)) {
+            // a copy did not complete in time: record it, wait once more (bounded) for the copies in flight,
+            // and leave without touching the chunk
+            if (tid == 0) {
+                set_error(a.err, kErrBarrierTimeout);
+                mbar_wait_bounded(&bar, phase ^ 1u);
+                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            return;
+        }
+        t.dtile = use_tile && a.deposit ? dtile : nullptr;
+        const int next_c = tid == 0 ? middle(ch + gridDim.x) : -1;  // read ahead of its use
+
+        // First pass: particles whose cell lies in the window and stays in its deposit tile, the light ones.
+        // The others (and their deposits) are listed and go in the second pass, so that a warp does not
+        // run the HBM paths for a few of its lanes in most of its turns.
+        // A thread owns particles tid*4 .. tid*4+3.  Taken in the same order, the eight threads of a
+        // quarter-warp would hit the same banks four times over (64-byte stride); an order rotated by
+        // (lane/2) mod 4 spreads them over all 32 banks.  Results go back to the same slots.
+        Corners32 run;     // deposit sums of the current run of light particles
+        int run_loc = -1;  // its slot in the deposit tile, -1: none
+#pragma unroll 2
+        for (int q = 0; q < kPPT; q++) {
+            const int x = tid * kPPT + ((q + (lane >> 1)) & 3);
+            const float4 P = ppos[x];
+            const int c = x < nin ? __float_as_int(P.w) : -1;
+            bool dead = false, put_off = false;
+            unsigned entry = x;
+            if (c >= 0) {
+                const int at = cell_base(g, c) - t.lo;
+                if ((unsigned)at < (unsigned)t.bases) {
+                    const float4 V = pvel[x];
+                    int i, j, k;
+                    cell_ijk(g, c, i, j, k);
+                    float3 o = make_float3(P.x, P.y, P.z);
+                    float3 v = make_float3(V.x, V.y, V.z);
+                    const float w = V.w;
+                    // leapfrog push (Species.cpp:369-373)
+                    const float3 E = gather_e(etile + at, kSeg, 2 * kSeg, 3 * kSeg, o);
+                    v.x += a.qm_dt * E.x;
+                    v.y += a.qm_dt * E.y;
+                    v.z += a.qm_dt * E.z;
+                    const int newc = move_particle(a, i, j, k, o, v);
+                    moved += newc != c;
+                    ppos[x] = make_float4(o.x, o.y, o.z, __int_as_float(newc));
+                    pvel[x] = make_float4(v.x, v.y, v.z, w);
+                    dead = newc < 0;
+                    if (a.deposit && !dead) {
+                        const int loc = cell_base(g, newc) - (t.lo - kMargin);
+                        const float s = w * a.dep_scale;
+                        put_off = (unsigned)loc >= (unsigned)(kSeg - 1) || !(s < kLightMax);
+                        entry |= kDepositOnly;
+                        if (!put_off) {
+                            if (loc != run_loc && run_loc >= 0) commit_run32(dtile + run_loc, run);
+                            corner_values32(s, o, run, loc == run_loc);
+                            run_loc = loc;
+                        }
+                    }
+                } else {
+                    put_off = true;
+                }
+            }
+            const unsigned pm = __ballot_sync(0xffffffffu, put_off);
+            if (pm) {
+                int b0 = 0;
+                if (lane == 0) b0 = atomicAdd(&s_later, __popc(pm));
+                b0 = __shfl_sync(0xffffffffu, b0, 0);
+                if (put_off) later[b0 + __popc(pm & ((1u << lane) - 1u))] = (unsigned short)entry;
+            }
+            record_dead(a, dead, base + x, lane);
+        }
+        if (run_loc >= 0) commit_run32(dtile + run_loc, run);
+        __syncthreads();
+        // Second pass: gathers and deposits in HBM
+        for (int e0 = tid & ~31; e0 < s_later; e0 += kThreads) {
+            bool dead = false;
+            int x = 0;
+            if (e0 + lane < s_later) {
+                const unsigned entry = later[e0 + lane];
+                x = entry & (kDepositOnly - 1);
+                const float4 P = ppos[x], V = pvel[x];
+                int newc = __float_as_int(P.w);
+                float3 o = make_float3(P.x, P.y, P.z);
+                if (!(entry & kDepositOnly)) {
+                    int i, j, k;
+                    cell_ijk(g, newc, i, j, k);
+                    const float3 E = gather_e(a.ef + cell_base(g, newc), t.off[1], t.off[2], t.off[3], o);
+                    const float3 v = make_float3(V.x + a.qm_dt * E.x, V.y + a.qm_dt * E.y, V.z + a.qm_dt * E.z);
+                    const int c = newc;
+                    newc = move_particle(a, i, j, k, o, v);
+                    moved += newc != c;
+                    ppos[x] = make_float4(o.x, o.y, o.z, __int_as_float(newc));
+                    pvel[x] = make_float4(v.x, v.y, v.z, V.w);
+                    dead = newc < 0;
+                }
+                if (a.deposit && !dead) {
+                    Corners hc;
+                    corner_values(V.w, o, a.dep_scale, hc, false);
+                    commit_corners(a, t, cell_base(g, newc), hc);
+                }
+            }
+            record_dead(a, dead, base + x, lane);
+        }
+        fence_proxy_async();  // the results, before the bulk stores read them
+        __syncthreads();
+        if (full(ch)) {
+            if (tid == 0) {
+                bulk_s2g(a.sp.pos + base, ppos, kChunk * sizeof(float4));
+                bulk_s2g(a.sp.vel + base, pvel, kChunk * sizeof(float4));
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+        } else {
+            for (int x = tid; x < nin; x += kThreads) {
+                a.sp.pos[base + x] = ppos[x];
+                a.sp.vel[base + x] = pvel[x];
+            }
+        }
+        if (tid == 0 && ch + gridDim.x < nchunks) {
+            issue_window(next_c);
+            issue_particles(ch + gridDim.x);
+            mbar_arrive(&bar);
+        }
+        if (t.dtile) {
             // commit the tile: slot o of row m is node lo - kMargin + off_m + o (only slots that
             // received a deposit are nonzero, and those are nodes of the grid)
-            const int wlo = lo - kMargin;
-            for (int x = tid; x < 4 * kSeg; x += kThreads) {
-                unsigned long long v = (unsigned long long)dtile[x] + ((unsigned long long)dtile[4 * kSeg + x] << 32);
-                if (v) atomicAdd(&a.sp.acc[wlo + t.off[x / kSeg] + (x % kSeg)], v);
+            for (int x = tid; x < kSeg; x += kThreads) {
+                unsigned long long* acc = a.sp.acc + (t.lo - kMargin + x);
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    const unsigned long long v =
+                        (unsigned long long)dtile[m * kSeg + x] | ((unsigned long long)dtile[(4 + m) * kSeg + x] << 32);
+                    if (v) atomicAdd(acc + (((m & 1) ? g.ni : 0) + ((m & 2) ? nij : 0)), v);
+                }
             }
         }
         __syncthreads();
     }
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     // cell-order bookkeeping for the sort policy: one global atomic per CTA (a per-warp atomic on
     // one address serialises hundreds of thousands of updates per launch)
-    __shared__ int s_moved;
-    if (tid == 0) s_moved = 0;
-    __syncthreads();
     const int wm = __reduce_add_sync(0xffffffffu, moved);
+    __syncthreads();
     if (lane == 0 && wm) atomicAdd(&s_moved, wm);
     __syncthreads();
     if (tid == 0 && s_moved) atomicAdd(&a.sp.counts[5], s_moved);
@@ -651,10 +679,9 @@ __global__ void __launch_bounds__(128) k_mcc_collide(PushArgs a, const int* cand
     const int nc = *ncand;
     unsigned st_cand = 0, st_coll = 0, st_ion = 0, st_lost = 0;
     Tile t;  // no staged rows: gathers and deposits go to HBM
-    t.etile = nullptr;
     t.dtile = nullptr;
     t.lo = 0;
-    t.span = -1;
+    t.bases = 0;
     t.off[0] = 0;
     t.off[1] = g.ni;
     t.off[2] = g.ni * g.nj;
@@ -685,7 +712,7 @@ __global__ void __launch_bounds__(128) k_mcc_collide(PushArgs a, const int* cand
                              make_float4(col.nv.x, col.nv.y, col.nv.z, w), child_id(id, cd.step, 2), a.err))
             st_lost++;
         float3 po = col.po, pv = col.pv;
-        const float3 Ep = gather_e(a, t, cell_base(g, c), po);
+        const float3 Ep = gather_e(a.ef + cell_base(g, c), t.off[1], t.off[2], t.off[3], po);
         pv.x += a.qm_dt * Ep.x;
         pv.y += a.qm_dt * Ep.y;
         pv.z += a.qm_dt * Ep.z;
@@ -722,14 +749,15 @@ int push_blocks_per_sm() {
     if (!nb) {
         cudaFuncSetAttribute(k_push, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPushSmem);
         cudaFuncSetAttribute(k_push, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_push, kThreads, kPushSmem) != cudaSuccess || nb < 1)
-            nb = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_push, kThreads, kPushSmem) != cudaSuccess || nb < 2)
+            nb = 2;
+        nb /= kCtasPerShape;
     }
     return nb;
 }
 void launch_push(const PushArgs& a, cudaStream_t s, int grid) {
     push_blocks_per_sm();
-    k_push<<<grid, kThreads, kPushSmem, s>>>(a);
+    k_push<<<kCtasPerShape * grid, kThreads, kPushSmem, s>>>(a);
 }
 
 // ------------------------------------------------------------------------------------
@@ -935,18 +963,9 @@ __device__ __forceinline__ void from_abs_one(const GridDev& g, const SpeciesDev&
     }
     if (cell >= 0 && rewind && ef) {
         // vel -= q/m E dt/2 (Species.cpp:431)
-        PushArgs dummy;
-        dummy.ef = ef;
-        Tile t;
-        t.etile = nullptr;
-        t.dtile = nullptr;
-        t.lo = 0;
-        t.span = -1;
-        t.off[0] = 0;
-        t.off[1] = g.ni;
-        t.off[2] = g.ni * g.nj;
-        t.off[3] = g.ni * g.nj + g.ni;
-        float3 E = gather_e(dummy, t, cell_base_node(g, ijk[0], ijk[1], ijk[2]), make_float3(o[0], o[1], o[2]));
+        const int nij = g.ni * g.nj;
+        const float3 E = gather_e(ef + cell_base_node(g, ijk[0], ijk[1], ijk[2]), g.ni, nij, nij + g.ni,
+                                  make_float3(o[0], o[1], o[2]));
         v.x -= qm_half_dt * E.x;
         v.y -= qm_half_dt * E.y;
         v.z -= qm_half_dt * E.z;
@@ -1612,17 +1631,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge(MergeArgs a) {
             linear_ijk(a.g, c, i, j, k);
             int bnode = cell_base_node(a.g, i, j, k);
             const int cpk = pack_cell(i, j, k);
-            Tile t;
-            t.etile = nullptr;
-            t.dtile = nullptr;
-            t.lo = 0;
-            t.span = -1;
-            t.off[0] = 0;
-            t.off[1] = a.g.ni;
-            t.off[2] = a.g.ni * a.g.nj;
-            t.off[3] = a.g.ni * a.g.nj + a.g.ni;
-            PushArgs pa;
-            pa.ef = a.ef;
+            const int nij = a.g.ni * a.g.nj;
             for (int side = 0; side < 2; side++) {
                 int l = side == 0 ? la : lb;
                 float4 ps = a.sp.pos[s0 + l];
@@ -1634,7 +1643,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge(MergeArgs a) {
                     atomicAdd(&a.stats[2], 1ull);
                     continue;
                 }
-                float3 Ev = gather_e(pa, t, bnode, o);
+                const float3 Ev = gather_e(a.ef + bnode, a.g.ni, nij, nij + a.g.ni, o);
                 v.x -= a.qm_half_dt * Ev.x;
                 v.y -= a.qm_half_dt * Ev.y;
                 v.z -= a.qm_half_dt * Ev.z;

@@ -311,7 +311,7 @@ int pic_autotune(pic_world* w, int* push_ctas_per_sm, int* node_grid);
 int pic_launch_shapes(pic_world* w, int* push_ctas_per_sm, int* node_grid, int* cg_grid);
 /* Sets the launch shapes, e.g. the ones pic_launch_shapes reported after pic_autotune on an earlier
  * world of the same size (no reference counterpart).  push_ctas_per_sm: 1 to the push's occupancy
- * limit; node_grid, cg_grid: CTA counts (a launch takes at most one CTA per 1024 nodes); 0 keeps
+ * limit, in CTAs of 256 threads (two of the kernel's); node_grid, cg_grid: CTA counts (a launch takes at most one CTA per 1024 nodes); 0 keeps
  * the built-in default for that shape.  PIC_ERR_ARG for a negative value or too many push CTAs. */
 int pic_set_launch_shapes(pic_world* w, int push_ctas_per_sm, int node_grid, int cg_grid);
 /* one iteration of the time loop: advanceTime, [merge], collisions + push + deposit,
