@@ -782,6 +782,220 @@ __global__ void __launch_bounds__(kUp0X * kUp0Y / R, kUp0CtasPerSM)
         grid_sum<2>(vv, gpart, gstride, ticket, out);
     }
 }
+// The same level as a march in z, for grids with enough planes to keep every CTA on one column of 64 x 16
+// nodes for a while.  A CTA takes an equal share of all columns' planes; planes of r, q and FREE bits arrive
+// through a ring of four stages (cp.async, two planes ahead), and a thread keeps the three plane sums of its
+// 4 x 2 outputs and the x-y interpolation of two coarse planes in registers: every staged word is read once,
+// 1.5 shared loads an output and plane (6 with the tile kernel's single columns), no plane of a tile's z
+// halo is recomputed, and the offsets of a thread's copies are formed once a column.
+// Bound by issue (0.66 of the slots, 16 warps an SM, 85 instructions a node of which 36 are the taps; the tiles
+// of 32 x 8 x 8: 126) at twice its time at the copy rate: 256 x 256 x 512 nodes 196 -> 143 us, 256^3 102 -> 82.
+constexpr int kMaX = 64, kMaY = 16, kMaThr = kMaX / 4 * kMaY / 2, kMaStages = 4, kMaCtasPerSM = 4;
+constexpr int kMaP = kMaX + 8, kMaO = 4;  // pitch of a staged row and the place of its body (16-byte aligned)
+constexpr int kMaRows = kMaY + 2, kMaCP = kMaX / 2 + 8, kMaCRows = kMaY / 2 + 2;  // coarse row: from x0 / 2 - 4
+constexpr int kMaStage = kMaP * kMaRows + kMaX * kMaY + 2 * kMaY;  // floats: r, q, FREE words
+constexpr int kMaSmem = 4 * (kMaStages * kMaStage + 2 * kMaCP * kMaCRows);
+static_assert(kMaCP / 4 * kMaCRows <= kMaThr, "a thread copies one group of a coarse plane");
+// four words from row + x (mapped by the view's rule) to shared memory; whole: all inside and aligned
+__device__ __forceinline__ void ma_copy4(float* dst, const LView& v, const float* row, int x, bool whole) {
+    if (whole) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc_smem_u32(dst)), "l"(row + x) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int ux = row ? lv_map(x + i, v.n[0], v.per[0]) : -1;
+            cp_async_f32(dst + i, ux >= 0 ? row + ux : v.a, ux >= 0);
+        }
+    }
+}
+__global__ void __launch_bounds__(kMaThr, kMaCtasPerSM)
+    k_lp_up0_march(GridDev g, LView rin, LView cin, float* __restrict__ z, const float* __restrict__ S0,
+                   const float* __restrict__ q, double* gpart, int gstride, unsigned* ticket, double* out,
+                   const int* flag, int cx_n, int pairs, long units) {
+    if (flag && flag[0]) return;
+    extern __shared__ __align__(16) float ma_dyn[];
+    float* coarse = ma_dyn + kMaStages * kMaStage;  // two planes
+    const int tid = threadIdx.x, lx = tid & 15, p = tid >> 4;
+    float w[27];
+#pragma unroll
+    for (int m = 0; m < 27; m++) w[m] = __ldg(&S0[m]);
+    float f_zr = 0.f, f_zq = 0.f;
+    long u = units * blockIdx.x / gridDim.x;
+    const long u_end = units * (blockIdx.x + 1) / gridDim.x;
+    while (u < u_end) {
+        // planes zs .. ze - 1 of column col (zs is even)
+        const int col = (int)(u / pairs), zs = 2 * (int)(u - (long)col * pairs);
+        const int ze = min(g.nk, zs + 2 * (int)min((long)pairs, u_end - u));
+        u += (ze - zs + 1) / 2;
+        const int x0 = (col % cx_n) * kMaX, y0 = (col / cx_n) * kMaY, xc = x0 + 4 * lx;
+        // offsets of this thread's copies within a plane (-1: outside, zero): rows p, p + 8 and (p < 2) p + 16 of
+        // r, its halo word, rows p, p + 8 of q, its FREE word, its four coarse words
+        const bool whole = xc + 3 < rin.n[0];
+        int oy[3], oh = -1, ob = -1, oc = -1;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int uy = lv_map(y0 - 1 + p + 8 * j, rin.n[1], rin.per[1]);
+            oy[j] = uy < 0 ? -1 : uy * rin.sy;
+        }
+        if (tid < 2 * kMaRows) {
+            const int ux = lv_map(tid & 1 ? x0 + kMaX : x0 - 1, rin.n[0], rin.per[0]);
+            const int uy = lv_map(y0 - 1 + (tid >> 1), rin.n[1], rin.per[1]);
+            oh = (ux | uy) < 0 ? -1 : ux + uy * rin.sy;
+        }
+        if (tid < 2 * kMaY && y0 + (tid >> 1) < g.nj && (x0 >> 5) + (tid & 1) < g.free_wpr)
+            ob = (y0 + (tid >> 1)) * g.free_wpr + (x0 >> 5) + (tid & 1);
+        const int rowc = tid / (kMaCP / 4), xcc = x0 / 2 - 4 + 4 * (tid % (kMaCP / 4));
+        bool wholec = false;
+        if (cin.a && rowc < kMaCRows) {
+            const int uy = lv_map(y0 / 2 - 1 + rowc, cin.n[1], cin.per[1]);
+            oc = uy < 0 ? -1 : uy * cin.sy;
+            wholec = ((cin.sy | cin.sz) & 3) == 0 && xcc >= 0 && xcc + 3 < cin.n[0];
+        }
+        // the copies of input plane zi as one group: r unless it lies before the first tap, q and FREE bits of an
+        // output plane, the coarse plane zi / 2 with even planes
+        auto issue = [&](int zi) {
+            float* st = ma_dyn + (zi & 3) * kMaStage;
+            if (zi >= zs - 1 && zi <= ze) {
+                const int uz = lv_map(zi, rin.n[2], rin.per[2]);
+                const float* src = rin.a + (uz < 0 ? 0 : (size_t)uz * rin.sz);
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    if (j == 2 && p >= 2) break;
+                    const bool row = (uz | oy[j]) >= 0;
+                    ma_copy4(st + (p + 8 * j) * kMaP + kMaO + 4 * lx, rin, row ? src + oy[j] : nullptr, xc, whole && row);
+                }
+                if (tid < 2 * kMaRows) {
+                    const bool ok = (uz | oh) >= 0;
+                    cp_async_f32(st + (tid >> 1) * kMaP + (tid & 1 ? kMaO + kMaX : kMaO - 1), ok ? src + oh : rin.a, ok);
+                }
+            }
+            if (zi >= zs && zi < ze) {
+                float* sq = st + kMaP * kMaRows;
+                if (q && xc < g.ni) {
+                    const float* src = q + ((size_t)zi * g.nj + y0 + p) * g.ni;
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+                        if (y0 + p + 8 * j < g.nj) ma_copy4(sq + (p + 8 * j) * kMaX + 4 * lx, rin, src + 8 * j * g.ni, xc, true);
+                }
+                if (ob >= 0)
+                    cp_async_f32(sq + kMaX * kMaY + tid,
+                                 reinterpret_cast<const float*>(g.free_bits + (size_t)zi * g.nj * g.free_wpr + ob), true);
+            }
+            if (cin.a && !(zi & 1) && zi <= ze && rowc < kMaCRows) {
+                const int uz = lv_map(zi >> 1, cin.n[2], cin.per[2]);
+                const bool row = (uz | oc) >= 0;
+                ma_copy4(coarse + ((zi >> 1) & 1) * kMaCP * kMaCRows + 4 * tid, cin,
+                         row ? cin.a + (size_t)uz * cin.sz + oc : nullptr, xcc, wholec && row);
+            }
+            cp_async_commit();
+        };
+        // plane sums of outputs zi - 1, zi; x-y interpolations of coarse planes k - 1, k, k = zi / 2
+        float A[2][4], B[2][4], po[2][4], pn[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) A[h][i] = B[h][i] = po[h][i] = pn[h][i] = 0.f;
+        auto step = [&](int zi, auto even) {
+            cp_async_wait<1>();
+            __syncthreads();  // plane zi of every thread has landed, and plane zi - 2 has been read
+            issue(zi + 2);
+            if (decltype(even)::value && cin.a) {
+                const float* C = coarse + ((zi >> 1) & 1) * kMaCP * kMaCRows + p * kMaCP + 4 + 2 * lx;
+                float xi[3][4];
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    const float2 c = *reinterpret_cast<const float2*>(C + r * kMaCP);
+                    const float cm = C[r * kMaCP - 1], cp = C[r * kMaCP + 2];
+                    xi[r][0] = 0.75f * c.x + 0.25f * cm;
+                    xi[r][1] = 0.75f * c.x + 0.25f * c.y;
+                    xi[r][2] = 0.75f * c.y + 0.25f * c.x;
+                    xi[r][3] = 0.75f * c.y + 0.25f * cp;
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        po[h][i] = pn[h][i];
+                        pn[h][i] = 0.75f * xi[1][i] + 0.25f * xi[2 * h][i];
+                    }
+            }
+            if (zi < zs - 1) return;
+            const float* st = ma_dyn + (zi & 3) * kMaStage;
+            float C[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) C[h][i] = 0.f;
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float* T = st + (2 * p + r) * kMaP + kMaO + 4 * lx;
+                const float4 b = *reinterpret_cast<const float4*>(T);
+                const float v[6] = {T[-1], b.x, b.y, b.z, b.w, T[4]};
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int dy = r - h;
+                    if (dy < 0 || dy > 2) continue;
+#pragma unroll
+                    for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            A[h][i] = fmaf(w[18 + 3 * dy + dx], v[i + dx], A[h][i]);
+                            B[h][i] = fmaf(w[9 + 3 * dy + dx], v[i + dx], B[h][i]);
+                            C[h][i] = fmaf(w[3 * dy + dx], v[i + dx], C[h][i]);
+                        }
+                }
+            }
+            if (zi > zs) {  // output plane zi - 1 is complete
+                const float* so = ma_dyn + ((zi - 1) & 3) * kMaStage;
+                const float* sq = so + kMaP * kMaRows;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int row = 2 * p + h, y = y0 + row;
+                    if (xc >= g.ni || y >= g.nj) continue;
+                    const unsigned fr = __float_as_uint(sq[kMaX * kMaY + 2 * row + (lx >> 3)]) >> ((4 * lx) & 31);
+                    const float4 rc = *reinterpret_cast<const float4*>(so + (row + 1) * kMaP + kMaO + 4 * lx);
+                    const float rv[4] = {rc.x, rc.y, rc.z, rc.w};
+                    float o[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        float v = A[h][i];
+                        // output 2k - 1 at step 2k lies towards the later coarse plane, 2k at 2k + 1 the earlier
+                        if (cin.a) v += decltype(even)::value ? 0.75f * po[h][i] + 0.25f * pn[h][i]
+                                                              : 0.75f * pn[h][i] + 0.25f * po[h][i];
+                        o[i] = (fr >> i) & 1u ? v : 0.f;
+                        f_zr += o[i] * rv[i];
+                    }
+                    if (q) {
+                        const float4 qc = *reinterpret_cast<const float4*>(sq + row * kMaX + 4 * lx);
+                        f_zq += o[0] * qc.x + o[1] * qc.y + o[2] * qc.z + o[3] * qc.w;
+                    }
+                    *reinterpret_cast<float4*>(z + ((size_t)(zi - 1) * g.nj + y) * g.ni + xc) =
+                        make_float4(o[0], o[1], o[2], o[3]);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    A[h][i] = B[h][i];
+                    B[h][i] = C[h][i];
+                }
+        };
+        __syncthreads();  // the column before has been read
+        issue(zs - 2);
+        issue(zs - 1);
+        for (int zi = zs - 2; zi <= ze; zi += 2) {
+            step(zi, std::true_type{});
+            if (zi + 1 <= ze) step(zi + 1, std::false_type{});
+        }
+        cp_async_wait<0>();
+    }
+    if (out) {
+        const float vv[2] = {f_zr, f_zq};
+        grid_sum<2>(vv, gpart, gstride, ticket, out);
+    }
+}
+
 // A network level's operator e = op(z) + P e_coarse on 3-D tiles of 32 x 8 x 8 voxels: the z tile with
 // its two-voxel halo (36 x 12 x 12) is staged in shared memory with all loads in flight, and a
 // thread rolls the five 5 x 5 plane sums of each tile plane into its column's eight outputs.
@@ -1066,6 +1280,9 @@ __global__ void __launch_bounds__(256) k_lp_restrict_tiled(LView f, LView c, con
     }
 }
 
+// planes of a column that a CTA of the march has at least (it reads four more than it writes): whole solves of
+// 12 iterations take 2.26 ms with it and 2.30 without at 8 planes, 2.49 and 2.52 at 10, 4.69 and 4.95 at 27
+constexpr int kMaLeast = 8;
 // z = B r on the finest level: the tiled kernel when its CTAs fit the reduction's partial slots
 static void launch_up0(const GridDev& g, LView r0, LView cin, float* z, const uint16_t* kind, const float* S0,
                        const float* q, double* gpart, int gstride, unsigned* ticket, double* out, const int* flag,
@@ -1073,7 +1290,14 @@ static void launch_up0(const GridDev& g, LView r0, LView cin, float* z, const ui
     const int bx_n = (g.ni + kUp0X - 1) / kUp0X, by_n = (g.nj + kUp0Y - 1) / kUp0Y;
     const long tiles = (long)bx_n * by_n * ((g.nk + kUp0Z - 1) / kUp0Z);
     const long ctas = std::min(tiles, (long)std::max(1, sms) * kUp0CtasPerSM);
-    if (!out || ctas <= gstride) {
+    const long cols = (long)((g.ni + kMaX - 1) / kMaX) * ((g.nj + kMaY - 1) / kMaY);
+    const int march = std::max(1, sms) * kMaCtasPerSM;
+    if ((g.ni & 3) == 0 && ((r0.sy | r0.sz) & 3) == 0 && cols * g.nk >= kMaLeast * (long)march && (!out || march <= gstride)) {
+        cudaFuncSetAttribute(k_lp_up0_march, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaSmem);
+        const int pairs = (g.nk + 1) / 2;
+        k_lp_up0_march<<<march, kMaThr, kMaSmem, s>>>(g, r0, cin, z, S0, q, gpart, gstride, ticket, out, flag,
+                                                     (g.ni + kMaX - 1) / kMaX, pairs, cols * pairs);
+    } else if (!out || ctas <= gstride) {
         static int dyn_set = -1;  // the device whose attributes are set (one device per process here)
         int dev = 0;
         cudaGetDevice(&dev);
