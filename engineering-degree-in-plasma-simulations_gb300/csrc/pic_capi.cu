@@ -258,9 +258,9 @@ void collect_timers(pic_world* w) {
 }
 
 int check_device_error(pic_world* w) {
-    unsigned h = 0;
-    CU(cudaMemcpyAsync(&h, w->err, sizeof(unsigned), cudaMemcpyDeviceToHost, w->stream));
+    CU(cudaMemcpyAsync(w->h_flag + 3, w->err, sizeof(unsigned), cudaMemcpyDeviceToHost, w->stream));
     CU(cudaStreamSynchronize(w->stream));
+    const unsigned h = (unsigned)w->h_flag[3];
     if (h) {
         CU(cudaMemsetAsync(w->err, 0, sizeof(unsigned), w->stream));
         if (h & kErrCapacity) return fail(PIC_ERR_CAPACITY, "a species ran out of capacity (device flags 0x%x)", h);
@@ -924,19 +924,17 @@ extern "C" int pic_world_get_field(pic_world* w, int which, double* out) {
 extern "C" int pic_world_potential_energy(pic_world* w, double* pe) {
     if (!w || !pe) return fail(PIC_ERR_ARG, "null argument");
     CU(cudaSetDevice(w->device));
-    const int grid = 512;
+    const int grid = 8 * w->sms;
+    double* total = w->part + grid;
     {
         Scope sc(w, "diagnostics", 1);
-        launch_field_energy(w->g, w->ef, w->part, w->stream, grid);
+        launch_field_energy(w->g, w->ef, w->part, w->ticket, total, w->stream, grid);
     }
-    std::vector<double> h(grid);
-    CU(cudaMemcpyAsync(h.data(), w->part, sizeof(double) * grid, cudaMemcpyDeviceToHost, w->stream));
-    CU(cudaStreamSynchronize(w->stream));
-    double t = 0;
-    for (int b = 0; b < grid; b++) t += h[b];
+    CU(cudaMemcpyAsync(w->h_scal, total, sizeof(double), cudaMemcpyDeviceToHost, w->stream));
+    const int rc = check_device_error(w);  // synchronises
     const GridDev& g = w->g;
-    *pe = 0.5 * kEps0 * g.dxd[0] * g.dxd[1] * g.dxd[2] * t;
-    return check_device_error(w);
+    *pe = 0.5 * kEps0 * g.dxd[0] * g.dxd[1] * g.dxd[2] * w->h_scal[0];
+    return rc;
 }
 extern "C" int pic_world_set_field(pic_world* w, int which, const double* in) {
     if (!w || !in) return fail(PIC_ERR_ARG, "null argument");
@@ -1345,12 +1343,12 @@ int push_species(pic_world* w, int sp, double dt, int deposit, bool with_mcc, bo
     {
         const bool neu = objects && s.charge != 0 && s.obj_neu != sp;
         const bool spu = objects && s.charge != 0 && s.obj_sputtering && s.obj_spu != s.obj_neu && s.obj_spu != sp;
-        Scope sc(w, "compact", (a.coll.enabled ? 5 : 4) + neu + spu);
-        launch_commit_appends(s.dev, w->err, w->stream);
-        if (a.coll.enabled) launch_commit_appends(w->sp[w->mcc_i].dev, w->err, w->stream);
-        if (neu) launch_commit_appends(w->sp[s.obj_neu].dev, w->err, w->stream);
-        if (spu) launch_commit_appends(w->sp[s.obj_spu].dev, w->err, w->stream);
-        launch_compact(s.dev, w->stream, w->sms * 4);
+        Scope sc(w, "compact", 1);
+        CommitList other;
+        if (a.coll.enabled) other.sp[other.n++] = w->sp[w->mcc_i].dev;
+        if (neu) other.sp[other.n++] = w->sp[s.obj_neu].dev;
+        if (spu) other.sp[other.n++] = w->sp[s.obj_spu].dev;
+        launch_compact(s.dev, other, w->err, wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls), w->stream);
     }
     return PIC_OK;
 }
@@ -1558,24 +1556,22 @@ extern "C" int pic_species_sums(pic_world* w, int sp, double* out) {
     if (!valid_sp(w, sp) || !out) return fail(PIC_ERR_ARG, "bad arguments");
     CU(cudaSetDevice(w->device));
     // enough CTAs to keep the particle stream in flight (5 partials per CTA fit the partial buffer)
-    const int grid = std::min(8 * w->sms, kParts * 8 / 5);
+    const int grid = std::min(8 * w->sms, kParts * 8 / 5 - 1);
+    double* total = w->part + 5 * (size_t)grid;
     {
         Scope sc(w, "sums", 1);
-        launch_sums(w->sp[sp].dev, w->part, w->stream, grid);
+        launch_sums(w->sp[sp].dev, w->part, w->ticket, total, w->stream, grid);
     }
-    std::vector<double> h(grid * 5);
-    CU(cudaMemcpyAsync(h.data(), w->part, sizeof(double) * grid * 5, cudaMemcpyDeviceToHost, w->stream));
-    CU(cudaStreamSynchronize(w->stream));
-    double t[5] = {0, 0, 0, 0, 0};
-    for (int b = 0; b < grid; b++)
-        for (int c = 0; c < 5; c++) t[c] += h[b * 5 + c];
+    CU(cudaMemcpyAsync(w->h_scal, total, sizeof(double) * 5, cudaMemcpyDeviceToHost, w->stream));
+    const int rc = check_device_error(w);  // synchronises
+    const double* t = w->h_scal;
     double m = w->sp[sp].mass;
     out[0] = t[0];
     out[1] = t[1] * m;
     out[2] = t[2] * m;
     out[3] = t[3] * m;
     out[4] = t[4] * m * 0.5;
-    return check_device_error(w);
+    return rc;
 }
 
 // =====================================================================================
@@ -2596,9 +2592,8 @@ extern "C" int pic_species_merge(pic_world* w, int sp, int min_count) {
                      (unsigned)w->ts, w->err, w->merge_stats, w->stream, w->sms * 8);
     }
     {
-        Scope sc(w, "compact", 4);
-        launch_commit_appends(s.dev, w->err, w->stream);
-        launch_compact(s.dev, w->stream, w->sms * 4);
+        Scope sc(w, "compact", 1);
+        launch_compact(s.dev, CommitList{}, w->err, wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls), w->stream);
     }
     CU(cudaGetLastError());
     return PIC_OK;

@@ -228,40 +228,67 @@ void launch_efield(const GridDev& g, const float2* phi, float4* ef, cudaStream_t
 // field energy sum |E|^2 V_node / V_cell (World::getPE, World.cpp:108-119): node volumes halve
 // on every non-periodic face (slab faces for stacked instances); the duplicate last plane of a
 // periodic axis is skipped.  Per-thread sums in float-float, FP64 from the warp sums on; the
-// host adds the block partials and scales by eps0/2 * V_cell.
+// last CTA adds the block partials, the host scales by eps0/2 * V_cell.
 // ------------------------------------------------------------------------------------
-__global__ void k_field_energy(GridDev g, const float4* __restrict__ ef, double* part) {
+__global__ void __launch_bounds__(256) k_field_energy(GridDev g, const float4* __restrict__ ef, double* part,
+                                                      unsigned* ticket, double* out) {
     FF a{0.f, 0.f};
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.nv; n += gridDim.x * blockDim.x) {
-        int ijk[3];
-        node_ijk(g, n, ijk[0], ijk[1], ijk[2]);
-        const int nn[3] = {g.ni, g.nj, g.zslab ? g.zslab : g.nk};
-        ijk[2] = slab_local_z(g, ijk[2]);
-        float f = 1.f;
-        bool alias = false;
-        for (int d = 0; d < 3; d++) {
-            const bool face = ijk[d] == 0 || ijk[d] == nn[d] - 1;
-            if (g.periodic[d]) alias |= ijk[d] == nn[d] - 1;
-            else if (face) f *= 0.5f;
+    const int nn[3] = {g.ni, g.nj, g.zslab ? g.zslab : g.nk};
+    const int step = gridDim.x * blockDim.x;
+    for (int n0 = blockIdx.x * blockDim.x + threadIdx.x; n0 < g.nv; n0 += 4 * step) {
+        float4 e[4];  // four reads in flight: one at a time leaves 0.4 of the copy rate
+#pragma unroll
+        for (int u = 0; u < 4; u++) e[u] = __ldg(&ef[min(n0 + u * step, g.nv - 1)]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int n = n0 + u * step;
+            if (n >= g.nv) continue;
+            int ijk[3];
+            node_ijk(g, n, ijk[0], ijk[1], ijk[2]);
+            ijk[2] = slab_local_z(g, ijk[2]);
+            float f = 1.f;
+            bool alias = false;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const bool face = ijk[d] == 0 || ijk[d] == nn[d] - 1;
+                if (g.periodic[d]) alias |= ijk[d] == nn[d] - 1;
+                else if (face) f *= 0.5f;
+            }
+            if (alias) continue;
+            const FF e2 = ff_add(ff_add(two_prod(e[u].x, e[u].x), two_prod(e[u].y, e[u].y)), two_prod(e[u].z, e[u].z));
+            a = ff_add(a, FF{e2.hi * f, e2.lo * f});  // f is a power of two: exact
         }
-        if (alias) continue;
-        const float4 e = __ldg(&ef[n]);
-        FF e2 = ff_add(ff_add(two_prod(e.x, e.x), two_prod(e.y, e.y)), two_prod(e.z, e.z));
-        a = ff_add(a, FF{e2.hi * f, e2.lo * f});  // f is a power of two: exact
     }
-    __shared__ double s[32];
+    __shared__ double s[8];
+    __shared__ unsigned s_last;
     double x = (double)a.hi + (double)a.lo;
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
     if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = x;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s[w];
+        for (int w = 0; w < 8; w++) t += s[w];
         part[blockIdx.x] = t;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x < 32) {  // lanes add runs of consecutive CTAs, then in lane order
+        const int per = ((int)gridDim.x + 31) / 32;
+        double t = 0;
+        for (int b = threadIdx.x * per; b < min((int)gridDim.x, ((int)threadIdx.x + 1) * per); b++) t += __ldcg(&part[b]);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) {
+            *out = t;
+            *ticket = 0u;
+        }
     }
 }
-void launch_field_energy(const GridDev& g, const float4* ef, double* part, cudaStream_t s, int grid) {
-    k_field_energy<<<grid, 256, 0, s>>>(g, ef, part);
+void launch_field_energy(const GridDev& g, const float4* ef, double* part, unsigned* ticket, double* out, cudaStream_t s,
+                         int grid) {
+    k_field_energy<<<std::max(1, std::min(grid, (g.nv + 1023) / 1024)), 256, 0, s>>>(g, ef, part, ticket, out);
 }
 
 // ------------------------------------------------------------------------------------
@@ -323,9 +350,9 @@ __device__ __forceinline__ void row_neighbours(const GridDev& g, int j, int k, i
     kp = g.periodic[2] ? wrap_p(k, g.nk, 1) : min(k + 1, g.nk - 1);
 }
 
-// Four consecutive nodes of one row per thread and iteration.  When rows are a multiple of four
-// nodes and the group does not touch the row ends, the group and its y / z neighbour rows are read
-// with 16-byte loads and the two x neighbours with scalar loads; other groups go node by node.
+// Four consecutive nodes of one row per thread and iteration when rows are a multiple of four nodes: the
+// group and its y / z neighbour rows are read with 16-byte loads and the two x neighbours with scalar loads.
+// Other grids go node by node, a node a thread (four in turn a thread: 14 us for 21^3 nodes, latency).
 // Capped at 80 registers (three CTAs per SM; a few bytes spill): measured faster than two CTAs at
 // 116 registers or four at 64.
 __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __restrict__ phi_in,
@@ -348,9 +375,9 @@ __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __
     const int nij = g.ni * g.nj;
     const float ie_f = kIeHi;
     float acc_r = 0.f, acc_b = 0.f, acc_s = 0.f;  // per-thread sums in FP32, block and grid sums in FP64
-    const int ngroups = (g.nv + 3) >> 2;
+    const int ngroups = rows4 ? g.nv >> 2 : g.nv;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ngroups; q += gridDim.x * blockDim.x) {
-        const int n0 = q << 2;
+        const int n0 = rows4 ? q << 2 : q;
         int i0, j, k;
         node_ijk(g, n0, i0, j, k);
         if (rows4) {
@@ -427,17 +454,16 @@ __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __
             continue;
         }
         // node by node
-        for (int n = n0; n < min(n0 + 4, g.nv); n++) {
+        {
+            const int n = n0;
             const uint16_t kd = kind[n];
             if ((kd & 3) != kFree) {
                 if (ae) phi_out[n] = phi_in[n];
                 r[n] = 0.f;
                 continue;
             }
-            int i, jj, kk;
-            node_ijk(g, n, i, jj, kk);
             Stencil st;
-            stencil(g, i, jj, kk, st);
+            stencil(g, i0, j, k, st);
             float2 pn[6];
             float en[6];
 #pragma unroll
@@ -465,7 +491,9 @@ __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __
 void launch_residual(const GridDev& g, SolveWork& w, int apply_e, cudaStream_t s, float* rho_prev, float* bfix_out) {
     const float2* in = w.phi;
     float2* out = apply_e ? w.phi_alt : w.phi;
-    k_residual<<<stream_blocks(g), 256, 0, s>>>(g, in, out, w.e, w.rho,
+    const int blocks = (g.ni & 3) && g.node_grid <= 0 ? std::max(stream_blocks(g), std::min(kParts, (g.nv + 255) / 256))
+                                                     : stream_blocks(g);
+    k_residual<<<blocks, 256, 0, s>>>(g, in, out, w.e, w.rho,
                                                           reinterpret_cast<const uint16_t*>(w.kind), w.r, w.gpart,
                                                           w.gstride, w.ticket, w.scal + kS_R2, apply_e, rho_prev,
                                                           bfix_out);

@@ -60,7 +60,13 @@ void launch_push(const PushArgs& a, cudaStream_t s, int grid);
 // push that follows runs without collisions.  cand holds up to the species capacity.
 void launch_mcc(const PushArgs& a, int* cand, int* ncand, cudaStream_t s, int sms);
 void launch_commit_appends(SpeciesDev sp, unsigned* err, cudaStream_t s);
-void launch_compact(SpeciesDev sp, cudaStream_t s, int grid);
+struct CommitList {  // species whose appends are committed beside a compaction
+    int n = 0;
+    SpeciesDev sp[3];
+};
+// commits the appends of sp (and of the others) and removes its dead; polls: of the wait between the two
+// halves of the move
+void launch_compact(SpeciesDev sp, const CommitList& other, unsigned* err, long long polls, cudaStream_t s);
 void launch_sort(const GridDev& g, SpeciesDev sp, float4* pos_alt, float4* vel_alt, unsigned long long* id_alt,
                  int* cell_count, int* cell_start, int* scan_aux, cudaStream_t s, int grid);
 void launch_from_abs(const GridDev& g, SpeciesDev sp, const double* pos, const double* vel, const double* w,
@@ -137,7 +143,8 @@ struct DsmcArgs {
     unsigned call, tag;           // counter words: the call number and the interaction's tag
 };
 void launch_dsmc(const DsmcArgs& a, cudaStream_t s);
-void launch_sums(SpeciesDev sp, double* out, cudaStream_t s, int grid);
+// part: 5 grid doubles, ticket: a counter that is zero at rest, out: 5 doubles
+void launch_sums(SpeciesDev sp, double* part, unsigned* ticket, double* out, cudaStream_t s, int grid);
 void launch_sample_moments(const GridDev& g, SpeciesDev sp, float4* mom, cudaStream_t s, int grid);
 // mean velocity (3 per node) and temperature of nodes first .. first + m - 1 from the sampled moments
 // (null outputs are skipped)
@@ -165,7 +172,8 @@ struct FinalizeArgs {
 void launch_finalize_rho(const FinalizeArgs& a, cudaStream_t s, int grid);
 void launch_efield(const GridDev& g, const float2* phi, float4* ef, cudaStream_t s, int grid);
 // per-block partials of sum |E|^2 f over the distinct nodes, f the node's volume in cells
-void launch_field_energy(const GridDev& g, const float4* ef, double* part, cudaStream_t s, int grid);
+void launch_field_energy(const GridDev& g, const float4* ef, double* part, unsigned* ticket, double* out, cudaStream_t s,
+                         int grid);
 void launch_kinds(const GridDev& g, uint8_t* kind, cudaStream_t s);
 
 struct SolveWork {

@@ -115,19 +115,30 @@ __device__ __forceinline__ void grid_sum(const float (&v)[N], double* part, int 
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-#pragma unroll
-    for (int c = 0; c < N; c++) {
+    // several warps a value, four partials of a lane in flight, one barrier: FP64 runs at two operations a clock
+    // and SM, so the tail costs its additions, one per 32 partials and five a warp
+    const int per = max(1, nw / N);  // warps of a value
+    for (int job = wp; job < per * N; job += nw) {
+        const double* row = part + (size_t)(job % N) * stride;
         double x = 0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) x += __ldcg(&part[c * stride + b]);
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        __syncthreads();
-        if (lane == 0) s[c][wp] = x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0;
-            for (int w = 0; w < nw; w++) t += s[c][w];
-            out[c] = t;
+        for (int b0 = lane + 32 * (job / N); b0 < (int)gridDim.x; b0 += 4 * 32 * per) {
+            double t[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                t[u] = b0 + 32 * per * u < (int)gridDim.x ? __ldcg(&row[b0 + 32 * per * u]) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (b0 - lane + 32 * per * u < (int)gridDim.x) x += t[u];
         }
+        if (32 * (job / N) < (int)gridDim.x)
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) s[job % N][job / N] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double x = s[threadIdx.x][0];
+        for (int w = 1; w < per && 32 * w < (int)gridDim.x; w++) x += s[threadIdx.x][w];
+        out[threadIdx.x] = x;
     }
     if (threadIdx.x == 0) *ticket = 0u;
 }
