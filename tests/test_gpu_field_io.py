@@ -23,3 +23,19 @@ def test_field_round_trip_is_exact(pic, nn):
     W.ef = e
     assert np.array_equal(W.ef, e.astype(np.float32).astype(np.float64))
     W.close()
+
+
+@pytest.mark.parametrize("nn", [(128, 128, 128), (131, 127, 129), (200, 201, 203)])
+def test_large_reads_fill_every_value(pic, nn):
+    """Arrays whose pages are first written by several threads: shares of whole pages, an odd last one, and an
+    output that the caller has already used and that does not start on a page."""
+    W = pic.World(*nn, (0.0, 0.0, 0.0), (1.0, 1.0, 1.0))
+    v = np.random.default_rng(0).normal(size=W.nv)
+    W.phi = v
+    got = W.phi
+    assert np.max(np.abs(got - v)) <= 1e-13 * np.max(np.abs(v))  # float-float storage
+    used = np.full(W.nv + 3, 7.0)
+    out = used[1:-2]
+    assert W._L.pic_world_get_field(W._h, 0, out.ctypes.data) == pic.PIC_OK
+    assert np.array_equal(out, got) and used[0] == 7.0 and np.all(used[-2:] == 7.0)
+    W.close()
