@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kLvThr, 1) k_lp_mid(const __grid_constant__ Lp
     lp_load_levels(sm, a.lev, a.lev.m, a.lev.ld, kLvThr);
     __syncthreads();
     unsigned target = 0;
-    const bool ok = lp_coarse_levels(sm.lev, sm, a.wait, target, &s_fail);
+    const bool ok = lp_coarse_levels<true>(sm.lev, sm, a.wait, target, &s_fail);
     if (threadIdx.x == 0) {
         if (!ok) {
             set_error(a.wait.err, kErrBarrierTimeout);
@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(kLvThr, 1) k_lp_dense(const __grid_constant__ 
     float* base = den_dyn + sizeof(LevelSmem) / 4;
     const int ld = a.lev.m, nlev = a.lev.nlev, tid = threadIdx.x, n = a.lev.z[ld].nvox;
     lp_load_levels(sm, a.lev, ld, nlev, kLvThr);
+    lp_levels_ready();
     for (int col = blockIdx.x; col < n; col += gridDim.x) {
         __syncthreads();
         // z of levels ld .. nlev - 1 one after the other, then two e's that alternate

@@ -96,15 +96,29 @@ struct LevelSmem {
     float tile[kLvTile];
     int mx[64], myz[320];  // offsets of a staged tile's points and rows (-1: outside)
 };
+// The stencils of the face classes that occur (a periodic axis has no faces: 3 of 27 classes with two of
+// them), as asynchronous copies: lp_levels_ready waits for the calling thread's
 __device__ __forceinline__ void lp_load_levels(LevelSmem& sm, const LpCoarseLevels& lev, int first, int nlev, int nt) {
-    const float* const* fold = lev.fold;
     if (threadIdx.x == 0) sm.lev = lev;
+    const int lane = threadIdx.x & 31;
     for (int l = first; l < nlev && l <= kLpNetLevels; l++)
-        for (int x = threadIdx.x; x < 27 * 128; x += nt) {
-            const int cls = x >> 7, d = x & 127;
-            sm.k5[l - 1][cls][d] = d < 125 ? fold[l][kLpFold + 125 * cls + d] : 0.f;
+        for (int cls = threadIdx.x >> 5; cls < 27; cls += nt >> 5) {
+            const int* per = lev.z[l].per;
+            if ((per[0] && cls % 3) || (per[1] && cls / 3 % 3) || (per[2] && cls / 9)) continue;
+            const float* src = lev.fold[l] + kLpFold + 125 * cls;
+#pragma unroll
+            for (int d = lane; d < 128; d += 32) {
+                float* dst = &sm.k5[l - 1][cls][d];
+                if (d < 125)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                                 "l"(src + d)
+                                 : "memory");
+                else
+                    *dst = 0.f;
+            }
         }
 }
+__device__ __forceinline__ void lp_levels_ready() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 static_assert(kLvTile >= kLpDenseMost, "the dense level's values lie in the staged tile's place");
 // a value of a level: shared memory, or global memory that other CTAs write (L2)
 template <bool SH>
@@ -317,7 +331,9 @@ __device__ __forceinline__ void lp_dense_level(const LpCoarseLevels& a, float* z
     }
 }
 // z of levels m .. and e of levels .. m from f0's values (published before the call; e of level m is
-// published by the caller's next barrier).  False when a grid barrier ran out.
+// published by the caller's next barrier).  False when a grid barrier ran out.  LOADING: lp_load_levels may
+// still be on its way.
+template <bool LOADING>
 __device__ __forceinline__ bool lp_coarse_levels(const LpCoarseLevels& a, LevelSmem& sm, const GridWait& wait,
                                                  unsigned& target, int* s_fail) {
     const int cta = blockIdx.x, nctas = gridDim.x;
@@ -325,6 +341,7 @@ __device__ __forceinline__ bool lp_coarse_levels(const LpCoarseLevels& a, LevelS
     bool ok = true;
     for (int l = a.m; l <= last && ok; l++) {
         lp_restrict_level<false>(l == a.m ? a.f0 : a.z[l - 1], a.z[l], cta, nctas);
+        if (l == last && LOADING) lp_levels_ready();  // published to the CTA by the barrier
         ok = grid_barrier(wait, target, s_fail);
     }
     for (int l = last; l >= a.m && ok; l--) {

@@ -113,7 +113,12 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
         s_fail = s_stop = 0;
         s_alpha = s_beta = 0.f;
     }
-    lp_load_levels(sm, a.lev, 1, a.lev.ld, kThr);
+    if (tid == 0) sm.lev = a.lev;  // once a solve: lp_load_levels measured 1 % slower here
+    for (int l = 1; l < a.lev.ld && l <= kLpNetLevels; l++)
+        for (int x = tid; x < 27 * 128; x += kThr) {
+            const int cls = x >> 7, dd = x & 127;
+            sm.k5[l - 1][cls][dd] = dd < 125 ? a.lev.fold[l][kLpFold + 125 * cls + dd] : 0.f;
+        }
     // zero what is only written on unknowns, and the flags of the CTA's tiles
     for (int n = blockIdx.x * kThr + tid; n < g.nv; n += gridDim.x * kThr) a.e[n] = a.z[n] = a.q[n] = a.d[0][n] = a.d[1][n] = 0.f;
     auto node = [&](const TileAt& t, int k) { return ((t.z0 + tz + k) * g.nj + t.y0 + ty) * g.ni + t.x0 + tx; };
@@ -229,7 +234,7 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
             lp_dense_level(sm.lev, sm.tile);
         } else {
             if (a.lev.m < a.lev.nlev)
-                ok = lp_coarse_levels(sm.lev, sm, a.wait, target, &s_fail) && grid_barrier(a.wait, target, &s_fail);
+                ok = lp_coarse_levels<false>(sm.lev, sm, a.wait, target, &s_fail) && grid_barrier(a.wait, target, &s_fail);
             if (!ok) break;
             lp_net_level<false, false>(a.z1, a.e2, a.e1, sm.k5[0], sm, blockIdx.x, gridDim.x);
         }
