@@ -206,6 +206,7 @@ struct pic_world {
     std::vector<cudaEvent_t> event_pool;
     long launches = 0;
     int grid_nodes = 1024;
+    int grid_stream = 1216;  // CTAs of the node kernels without block partials: one wave of 8 an SM
     int grid_push_mcc = 304, grid_push = 456, grid_parts = 1216;
     long long wait_polls_arg = 0;  // PushArgs::wait_polls of this world's pushes (0: the default)
 };
@@ -658,6 +659,7 @@ extern "C" int pic_world_create(pic_world** out, int ni, int nj, int nk, const d
     cudaMemsetAsync(w->ticket, 0, sizeof(unsigned) * 4, w->stream);
     w->gstride = std::max(kParts, 2 * node_blocks(nv));
     w->grid_nodes = (int)std::min<long long>(kParts, std::max<long long>(1, (nv + 255) / 256));
+    w->grid_stream = (int)std::min<long long>(8 * w->sms, std::max<long long>(1, (nv + 255) / 256));
     w->grid_parts = w->sms * 8;
     w->grid_push = w->sms * push_blocks_per_sm();
     w->grid_push_mcc = w->sms * 2;
@@ -1505,7 +1507,7 @@ extern "C" int pic_charge_density(pic_world* w) {
     a.rho = w->rho;
     {
         Scope sc(w, "rho", 1);
-        launch_finalize_rho(a, w->stream, w->grid_nodes);
+        launch_finalize_rho(a, w->stream, w->grid_stream);
     }
     // the accumulators are cleared when a species deposits again, so a species that was not
     // pushed this step keeps the density of its last push (main.cpp:222-234 subcycling)
@@ -1532,7 +1534,7 @@ extern "C" int pic_species_update_averages(pic_world* w, int sp) {
     float b = 1.f / s.avg_samples, a = (float)(s.avg_samples - 1) / s.avg_samples;
     {
         Scope sc(w, "averages", 1);
-        launch_den_avg(s.den_avg, s.den, w->g.nv, a, b, w->stream, w->grid_nodes);
+        launch_den_avg(s.den_avg, s.den, w->g.nv, a, b, w->stream, w->grid_stream);
     }
     CU(cudaGetLastError());
     return PIC_OK;
@@ -2267,7 +2269,7 @@ extern "C" int pic_solver_compute_ef(pic_world* w) {
     CU(cudaSetDevice(w->device));
     {
         Scope sc(w, "efield", 1);
-        launch_efield(w->g, w->phi, w->ef, w->stream, w->grid_nodes);
+        launch_efield(w->g, w->phi, w->ef, w->stream, w->grid_stream);
     }
     CU(cudaGetLastError());
     return PIC_OK;
@@ -2724,7 +2726,7 @@ extern "C" int pic_autotune(pic_world* w, int* push_ctas_per_sm, int* node_grid)
         const int most = std::min<long>((w->g.nv / 4 + 255) / 256, (long)w->gstride);
         int best = 0;
         float best_ms = 0.f;
-        for (int m : {2, 4, 8, 16}) {
+        for (int m : {2, 3, 4, 5, 8, 16}) {
             const int cand = std::min(w->sms * m, most);
             if (cand < 1 || cand == best) continue;
             w->g.node_grid = cand;
@@ -2746,7 +2748,7 @@ extern "C" int pic_autotune(pic_world* w, int* push_ctas_per_sm, int* node_grid)
         const int most = std::min<long>((w->g.nv / 4 + 255) / 256, (long)w->gstride);
         int best = 0;
         float best_ms = 0.f;
-        for (int m : {2, 4, 8, 16}) {
+        for (int m : {2, 3, 4, 5, 8, 16}) {
             const int cand = std::min(w->sms * m, most);
             if (cand < 1 || cand == best) continue;
             w->g.cg_grid = cand;

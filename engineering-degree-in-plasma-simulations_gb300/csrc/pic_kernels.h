@@ -215,16 +215,26 @@ constexpr int kParts = 1024;
 constexpr int kNodeThreads = 256;
 constexpr int kNodeTile = 4 * kNodeThreads;
 inline int node_blocks(int nv) { return (nv + kNodeTile - 1) / kNodeTile; }
-// streaming node kernels (four consecutive nodes per thread and 16-byte loads, grid-stride): a
-// few CTAs per SM keep every SM busy, and the grid sum adds few partials
-inline int stream_blocks(int nv, int cap = 1216) {
+// Streaming node kernels (four consecutive nodes per thread and 16-byte loads, grid-stride): one wave of the
+// CTAs that fit the SMs, since a CTA has the same share of the nodes whichever wave it runs in.  With 1216
+// CTAs of a kernel that fits three an SM, 2.7 waves, the last wave leaves a third of the SMs idle: 12 learned
+// iterations of 256 x 256 x 512 nodes 7.90 ms, one wave 7.67 (304 CTAs 8.23, 532 8.46); of 32 x 32 x 2048
+// 1.53 -> 1.43; 300 Jacobi-PCG iterations of 144^3, five an SM, 12.5 -> 9.6 ms (456 CTAs 10.2, 912 13.0).
+constexpr int kSms = 152;
+constexpr int kResPerSM = 3;  // residual and learned-CG kernels (80 registers; the others' sums stay short)
+constexpr int kPcgPerSM = 5;  // Jacobi-PCG kernels (48 registers)
+inline int stream_blocks(int nv, int cap) {
     const int want = (nv / 4 + 255) / 256;
     return want < 1 ? 1 : (want < cap ? want : cap);
 }
-inline int stream_blocks(const GridDev& g) { return stream_blocks(g.nv, g.node_grid > 0 ? g.node_grid : 1216); }
-// the CG stencil kernels wait on five neighbour rows per group of four nodes: they want more warps
-// in flight than the streaming kernels, so their CTA count is tuned on its own
-inline int cg_blocks(const GridDev& g) { return g.cg_grid > 0 ? stream_blocks(g.nv, g.cg_grid) : stream_blocks(g); }
+inline int stream_blocks(const GridDev& g, int per_sm) {
+    return stream_blocks(g.nv, g.node_grid > 0 ? g.node_grid : per_sm * kSms);
+}
+// the CG stencil kernels wait on five neighbour rows per group of four nodes, so their CTA count can be tuned
+// on its own
+inline int cg_blocks(const GridDev& g, int per_sm) {
+    return g.cg_grid > 0 ? stream_blocks(g.nv, g.cg_grid) : stream_blocks(g, per_sm);
+}
 // device scalar slots of the solvers
 enum : int {
     kS_RZ = 0,      // [0..1] r.z of iterations it (double-buffered by parity)

@@ -1575,7 +1575,7 @@ __device__ __forceinline__ void cg_pair(const GridDev& g, int i0, int j0, int k,
     cg_row4(c3, nb, xend, wrapx, v[2], Nb, xe[2], xe[3], kb, d_out, q, acc);
 }
 
-__global__ void __launch_bounds__(256) k_lpcg_k1(GridDev g, const float* __restrict__ z,
+__global__ void __launch_bounds__(256, kResPerSM) k_lpcg_k1(GridDev g, const float* __restrict__ z,
                                                           const float* __restrict__ d_in, float* __restrict__ d_out,
                                                           float* __restrict__ q, const uint16_t* __restrict__ kind,
                                                           double* gpart, int gstride, unsigned* ticket,
@@ -1705,9 +1705,9 @@ void launch_lpcg_init(const GridDev& g, SolveWork& w, const LpState& L, cudaStre
 void launch_lpcg_iter(const GridDev& g, SolveWork& w, const LpState& L, float* d_in, float* d_out, int it,
                       double target_rr, cudaStream_t s, int sms) {
     const uint16_t* kd = reinterpret_cast<const uint16_t*>(w.kind);
-    k_lpcg_k1<<<cg_blocks(g), 256, 0, s>>>(g, w.z, d_in, d_out, w.q, kd, w.gpart, w.gstride, w.ticket, w.scal, w.flag,
+    k_lpcg_k1<<<cg_blocks(g, kResPerSM), 256, 0, s>>>(g, w.z, d_in, d_out, w.q, kd, w.gpart, w.gstride, w.ticket, w.scal, w.flag,
                                            it, target_rr);
-    k_lpcg_k2<<<stream_blocks(g), 256, 0, s>>>(g, d_out, w.q, w.e, w.r, kd, w.gpart, w.gstride, w.ticket, w.scal,
+    k_lpcg_k2<<<stream_blocks(g, kResPerSM), 256, 0, s>>>(g, d_out, w.q, w.e, w.r, kd, w.gpart, w.gstride, w.ticket, w.scal,
                                                   w.flag, it);
     launch_lp_apply(g, L, w, w.r, w.z, w.q, true, w.flag, s, sms);
 }
@@ -1715,7 +1715,7 @@ void launch_lpcg_iter(const GridDev& g, SolveWork& w, const LpState& L, float* d
 // arrays): what the launch-shape tuner times
 void launch_lpcg_k1_probe(const GridDev& g, SolveWork& w, float* d_in, float* d_out, cudaStream_t s) {
     const uint16_t* kd = reinterpret_cast<const uint16_t*>(w.kind);
-    k_lpcg_k1<<<cg_blocks(g), 256, 0, s>>>(g, w.z, d_in, d_out, w.q, kd, w.gpart, w.gstride, w.ticket, w.scal, w.flag,
+    k_lpcg_k1<<<cg_blocks(g, kResPerSM), 256, 0, s>>>(g, w.z, d_in, d_out, w.q, kd, w.gpart, w.gstride, w.ticket, w.scal, w.flag,
                                            0, 0.0);
 }
 
