@@ -946,7 +946,7 @@ extern "C" int pic_world_get_field(pic_world* w, int which, double* out) {
 extern "C" int pic_world_potential_energy(pic_world* w, double* pe) {
     if (!w || !pe) return fail(PIC_ERR_ARG, "null argument");
     CU(cudaSetDevice(w->device));
-    const int grid = 8 * w->sms;
+    const int grid = 6 * w->sms;  // one resident wave
     double* total = w->part + grid;
     {
         Scope sc(w, "diagnostics", 1);
@@ -1579,8 +1579,8 @@ extern "C" int pic_species_sort(pic_world* w, int sp, int32_t* cell_counts) {
 extern "C" int pic_species_sums(pic_world* w, int sp, double* out) {
     if (!valid_sp(w, sp) || !out) return fail(PIC_ERR_ARG, "bad arguments");
     CU(cudaSetDevice(w->device));
-    // enough CTAs to keep the particle stream in flight (5 partials per CTA fit the partial buffer)
-    const int grid = std::min(8 * w->sms, kParts * 8 / 5 - 1);
+    // one resident wave of CTAs (5 partials per CTA fit the partial buffer)
+    const int grid = std::min(6 * w->sms, kParts * 8 / 5 - 1);
     double* total = w->part + 5 * (size_t)grid;
     {
         Scope sc(w, "sums", 1);

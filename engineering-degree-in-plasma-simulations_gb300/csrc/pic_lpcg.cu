@@ -34,7 +34,7 @@ constexpr int kWarps = kThr / 32, kRowsPer = (kRows + kWarps - 1) / kWarps;
 constexpr int kCX = kTX / 2 + 2, kCY = kTY / 2 + 2, kCZ = kTZ / 2 + 2, kCTile = kCX * kCY * kCZ;
 constexpr int kMostRounds = 16;                            // tiles a CTA owns
 // The tiles of a CTA are serial, while the launches fill the SMs better the more tiles there are: a loop of
-// 1.0 M nodes runs 26.8 ms here and 33.2 as launches, one of 2.1 M nodes 21.5 and 21.6; the line lies between.
+// 1.0 M nodes spends 15.6 ms in solves here and 18.7 as launches, one of 2.1 M nodes 12.6 and 11.5; the line lies between.
 constexpr int kLpcgMostNodes = 3 << 19;
 struct LpcgArgs {
     GridDev g;

@@ -1472,8 +1472,9 @@ __device__ __forceinline__ void sums_step(double* x, int o, bool upper) {
 // kSumsRun particles a thread at least before another CTA takes part: FP64 runs at two operations a clock
 // and SM, so that the conversion and reduction of every thread's totals bound the sums of few particles
 // (2 M: 30 us with 1216 CTAs, 9 of 36 us of a call in the copy of the CTAs' partials to the host).  A warp
-// reduces five values in 9 FP64 additions, the last CTA adds the partials in CTA order.
-constexpr int kSumsRun = 32;
+// reduces five values in 9 FP64 additions, the last CTA adds the partials in CTA order.  A call on 2 M particles: 36 ->
+// 25 us (26 with runs of 32, 28 of 8, 33 of 64); on 100 M, six CTAs an SM in one wave, 253 us (eight, 1.3 waves: 310).
+constexpr int kSumsRun = 16;
 __global__ void __launch_bounds__(256) k_sums(SpeciesDev sp, double* part, unsigned* ticket, double* out) {
     const int n = sp.counts[0];
     const int nb = min((int)gridDim.x, max(1, (n + 256 * kSumsRun - 1) / (256 * kSumsRun)));
