@@ -368,8 +368,8 @@ __device__ __noinline__ Collision collide_candidate(const CollDev& cd, unsigned 
 //   a shared 64-bit fixed-point tile (two 32-bit word planes) committed to HBM with one atomic per touched
 //   node.  Particles outside the window, and deposits that leave it, go to HBM in a second pass over a list.
 //
-//   What bounds it: shared-memory wavefronts (62 % of the pipe, 90 a warp and turn: eight 16-byte reads of E,
-//   the particles in and out, the deposit's atomics) and issue slots (60 %), with barriers between the phases;
+//   What bounds it: shared-memory wavefronts (68 % of the pipe, 87 a warp and turn: eight 16-byte reads of E,
+//   the particles in and out, the deposit's atomics) and issue slots (64 %), with barriers between the phases;
 //   hence many small CTAs: 8 of 128 threads, chunks of 512.  16 M particles on 97 x 113 x 129 nodes,
 //   0.324 -> 0.225 ms (1.02 GB, 0.15 ms at the copy rate); 2 x 100 M, 20 pushes: 39.0 -> 28.1 ms.  Measured
 //   on the way: 4 CTAs of 256 threads 30.1, 7 of 128 29.1, 14 of 64 31.7, 2 of 512 50 ms; E and deposits outside
