@@ -423,13 +423,15 @@ __global__ void __launch_bounds__(kThreads, kPushBlocksPerSM) k_push(PushArgs a)
     auto middle = [&](int ch) {
         return ch < nchunks ? __float_as_int(a.sp.pos[ch * kChunk + (min(kChunk, n - ch * kChunk) >> 1)].w) : -1;
     };
-    // thread 0: the bulk copies of a full chunk's particles, once the chunk before has been stored
+    // thread 0: the bulk copies of a full chunk's particles.  The stores of the chunk before must have read
+    // their shared memory first, also where the next chunk is the partial one, which the threads write themselves
+    // after the barrier that ends the turn.
     auto issue_particles = [&](int ch) {
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         if (!full(ch)) return;
         const unsigned pb = kChunk * sizeof(float4);
         fence_proxy_async();
         mbar_expect_tx(&bar, 2 * pb);
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         bulk_g2s(ppos, a.sp.pos + ch * kChunk, pb, &bar);
         bulk_g2s(pvel, a.sp.vel + ch * kChunk, pb, &bar);
     };
