@@ -170,9 +170,12 @@ __device__ __forceinline__ unsigned wrap_flags(const GridDev& g, int i, int j) {
 // colours and relaxed with omega = 1): nodes on one seam by colour, then those on two, then on three,
 // so that no two neighbours are updated at once and the result does not depend on timing.
 // Every CTA lists its nodes by pass once; a pass is one shared-memory update per listed node, and ends
-// when the neighbours' values of the pass have arrived.  The barriers alternate between passes: a
-// neighbour can be one pass ahead (it has all of this CTA's values of the pass, so their reads of the
-// halo are done), never two.
+// when the neighbours' values of the pass have arrived.  The barriers alternate between passes, so no CTA may
+// be two passes ahead of a neighbour.  Values bound the drift: a CTA that has all of a neighbour's values of
+// pass p knows that the neighbour has left pass p - 1 and done its reads of the halo for p.  A CTA
+// without unknowns of a pass in its boundary plane (a wall or a plate there, or a pass that only relaxes a
+// seam elsewhere) has no values to send; it sends the neighbour one word that nobody reads instead, as
+// it begins the pass.
 // ------------------------------------------------------------------------------------
 // A list entry is the node's slot (20 bits), mirror mask (6) and wrap flags (4), and its r.  The
 // off-diagonal sum needs no mask: e stays zero on MIRROR and FIXED nodes.
@@ -183,15 +186,17 @@ __global__ void __launch_bounds__(1024, 1) k_sor_cluster(GridDev g, float* __res
     const int nij = g.ni * g.nj, nt = blockDim.x;
     uint2* L = reinterpret_cast<uint2*>(sm);                 // planes * nij, by pass
     float* E = sm + 2 * (size_t)planes * nij;                // (planes + 2) * nij
-    __shared__ int cnt[8], start[9], halo[8];
-    __shared__ float dia_tab[64];
+    // per pass, for the sides towards lower and higher planes: unknowns in the neighbour's and in this CTA's
+    // boundary plane
+    __shared__ int cnt[8], start[9], halo[2][8], edge[2][8];
+    __shared__ float dia_tab[64], unread;
     __shared__ __align__(8) unsigned long long bar[2];
     const Slab s = make_slab(g, planes, E);
     const int tid = threadIdx.x, own = s.np * nij, n0 = s.k0 * nij;
     const float c3[3] = {g.inv_dx[0] * g.inv_dx[0], g.inv_dx[1] * g.inv_dx[1], g.inv_dx[2] * g.inv_dx[2]};
     for (int x = tid; x < (s.np + 2) * nij; x += nt) E[x] = 0.f;
     if (tid < 64) dia_tab[tid] = mask_diag(c3, (unsigned)tid);
-    if (tid < 8) cnt[tid] = halo[tid] = 0;
+    if (tid < 8) cnt[tid] = halo[0][tid] = halo[1][tid] = edge[0][tid] = edge[1][tid] = 0;
     if (tid < 2) bar_init(&bar[tid]);
     const bool sx = g.periodic[0] && ((g.ni - 1) & 1), sy = g.periodic[1] && ((g.nj - 1) & 1),
                sz = g.periodic[2] && ((g.nk - 1) & 1);
@@ -209,12 +214,15 @@ __global__ void __launch_bounds__(1024, 1) k_sor_cluster(GridDev g, float* __res
     unsigned wf;
     for (int x = tid; x < own; x += nt) {
         const int p = info(n0 + x, kind[n0 + x], wf);
-        if (p >= 0) atomicAdd(&cnt[p], 1);
+        if (p < 0) continue;
+        atomicAdd(&cnt[p], 1);
+        if (x < nij) atomicAdd(&edge[0][p], 1);
+        if (x >= own - nij) atomicAdd(&edge[1][p], 1);
     }
     for (int x = tid; x < 2 * nij; x += nt) {  // what the neighbours send in each pass
         const int n = halo_node(s, x);
         const int p = n >= 0 ? info(n, kind[n], wf) : -1;
-        if (p >= 0) atomicAdd(&halo[p], 1);
+        if (p >= 0) atomicAdd(&halo[x >= nij][p], 1);
     }
     __syncthreads();
     if (tid == 0) {
@@ -243,9 +251,14 @@ __global__ void __launch_bounds__(1024, 1) k_sor_cluster(GridDev g, float* __res
     bool ok = true;
     for (int it = 0; it < sweeps && ok; it++)
         for (int p = 0; p < npass; p++, q ^= 1) {
-            if (tid == 0) bar_expect(&bar[q], 4u * (unsigned)halo[p]);
             const unsigned lo_bar = s.has_lo ? map_rank(&bar[q], s.lo_rank) : 0u,
                            hi_bar = s.has_hi ? map_rank(&bar[q], s.hi_rank) : 0u;
+            if (tid == 0) {
+                const int words = (s.has_lo ? max(1, halo[0][p]) : 0) + (s.has_hi ? max(1, halo[1][p]) : 0);
+                bar_expect(&bar[q], 4u * (unsigned)words);
+                if (s.has_lo && !edge[0][p]) st_async(map_rank(&unread, s.lo_rank), 0.f, lo_bar);
+                if (s.has_hi && !edge[1][p]) st_async(map_rank(&unread, s.hi_rank), 0.f, hi_bar);
+            }
             const float om = p < 2 ? omega : 1.0f;
             for (int y = start[p] + tid; y < start[p + 1]; y += nt) {
                 const uint2 u = L[y];
