@@ -260,6 +260,7 @@ void collect_timers(pic_world* w) {
     w->pending.clear();
 }
 
+long long wait_polls(const pic_world* w) { return wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls); }
 int check_device_error(pic_world* w) {
     CU(cudaMemcpyAsync(w->h_flag + 3, w->err, sizeof(unsigned), cudaMemcpyDeviceToHost, w->stream));
     CU(cudaStreamSynchronize(w->stream));
@@ -578,7 +579,7 @@ SolveWork solve_work(pic_world* w) {
     s.gstride = w->gstride;
     s.ticket = w->ticket;
     s.err = w->err;
-    s.wait_polls = wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls);
+    s.wait_polls = wait_polls(w);
     return s;
 }
 
@@ -1062,7 +1063,7 @@ extern "C" int pic_species_add_particles(pic_world* w, int sp, const double* pos
                 Scope sc(w, "load", 5);
                 launch_from_abs(w->g, s.dev, dp + 3 * a, dv + 3 * a, dw + a, di ? di + a : nullptr,
                                 id0 + (unsigned long long)a, (int)m, rewind, (float)(s.charge / s.mass * 0.5 * w->dt),
-                                w->ef, w->stream);
+                                w->ef, w->err, wait_polls(w), w->stream);
             }
             if (!ids) s.next_id += n;
             CU(cudaStreamSynchronize(w->stream));
@@ -1088,7 +1089,7 @@ extern "C" int pic_species_add_particles(pic_world* w, int sp, const double* pos
         if (ids) CU(cudaMemcpyAsync(di, ids + a, sizeof(unsigned long long) * m, cudaMemcpyHostToDevice, w->stream));
         Scope sc(w, "load", 5);
         launch_from_abs(w->g, s.dev, dp, dv, dw, ids ? di : nullptr, id0 + (unsigned long long)a, (int)m, rewind,
-                        (float)(s.charge / s.mass * 0.5 * w->dt), w->ef, w->stream);
+                        (float)(s.charge / s.mass * 0.5 * w->dt), w->ef, w->err, wait_polls(w), w->stream);
     }
     if (!ids) s.next_id += n;
     CU(cudaStreamSynchronize(w->stream));
@@ -1149,7 +1150,7 @@ extern "C" int pic_species_add_particles_batch(pic_world* w, int count, const in
             // two CTAs per SM keep the host link busy and leave the SMs to the previous species' sort
             launch_from_abs(w->g, s.dev, dp + 3 * a, dv + 3 * a, dw + a, di ? di + a : nullptr,
                             id0 + (unsigned long long)a, (int)m, rewind, (float)(s.charge / s.mass * 0.5 * w->dt),
-                            w->ef, w->upload_stream, 2 * w->sms);
+                            w->ef, w->err, wait_polls(w), w->upload_stream, 2 * w->sms);
         }
         if (!idk) s.next_id += n[k];
         CU(cudaEventRecord(ev[k], w->upload_stream));
@@ -1370,7 +1371,7 @@ int push_species(pic_world* w, int sp, double dt, int deposit, bool with_mcc, bo
         if (a.coll.enabled) other.sp[other.n++] = w->sp[w->mcc_i].dev;
         if (neu) other.sp[other.n++] = w->sp[s.obj_neu].dev;
         if (spu) other.sp[other.n++] = w->sp[s.obj_spu].dev;
-        launch_compact(s.dev, other, w->err, wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls), w->stream);
+        launch_compact(s.dev, other, w->err, wait_polls(w), w->stream);
     }
     return PIC_OK;
 }
@@ -2363,7 +2364,7 @@ extern "C" int pic_source_sample(pic_world* w, int source_id) {
         Scope sc(w, "source", 6);
         launch_source(sa, dp, dv, dw, w->stream);
         launch_from_abs(w->g, s.dev, dp, dv, dw, nullptr, s.next_id + (unsigned long long)a, (int)m, 1,
-                        (float)(s.charge / s.mass * 0.5 * w->dt), w->ef, w->stream);
+                        (float)(s.charge / s.mass * 0.5 * w->dt), w->ef, w->err, wait_polls(w), w->stream);
     }
     s.next_id += n;
     CU(cudaGetLastError());
@@ -2617,7 +2618,7 @@ extern "C" int pic_species_merge(pic_world* w, int sp, int min_count) {
     }
     {
         Scope sc(w, "compact", 1);
-        launch_compact(s.dev, CommitList{}, w->err, wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls), w->stream);
+        launch_compact(s.dev, CommitList{}, w->err, wait_polls(w), w->stream);
     }
     CU(cudaGetLastError());
     return PIC_OK;

@@ -784,8 +784,12 @@ void launch_commit_appends(SpeciesDev sp, unsigned* err, cudaStream_t s) { k_com
 // become holes, live particles above it fill them after a grid barrier, the last CTA to leave sets the
 // counts.  Four launches of 2 to 4 us before (commit, holes, moves, counts), most of it their latency: 10 to
 // 16 us a push, now 3 us without a dead particle and 6 with.  other: species that only commit.
+// A wait at the barrier that runs out is reported, and the last CTA, which knows that all holes are listed, makes
+// the moves that are left: the species stays whole.  For that a particle that has moved is marked removed in
+// its old place.
 __global__ void __launch_bounds__(256) k_compact(SpeciesDev sp, CommitList other, unsigned* err, long long polls) {
-    __shared__ int s_fail;
+    __shared__ int s_fail, s_last;  // s_last: 1 the last CTA, 2 with moves left to make
+    constexpr int kFailed = 1 << 16;  // added to the exits by a CTA whose wait ran out
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
     if (tid < other.n) commit_appends(other.sp[tid], err);
     const int n0 = sp.counts[0], pend = sp.counts[1], nd = sp.counts[2];
@@ -799,23 +803,34 @@ __global__ void __launch_bounds__(256) k_compact(SpeciesDev sp, CommitList other
         const int idx = sp.dead[d];
         if (idx < nnew) sp.holes[atomicAdd(&sp.counts[3], 1)] = idx;
     }
+    auto fill = [&](int idx) {
+        const float4 p = __ldcg(&sp.pos[idx]);
+        if (__float_as_int(p.w) < 0) return;
+        const int h = __ldcg(&sp.holes[atomicAdd(&sp.counts[4], 1)]);
+        sp.pos[h] = p;
+        sp.vel[h] = sp.vel[idx];
+        sp.id[h] = sp.id[idx];
+        sp.pos[idx].w = __int_as_float(-1);
+    };
     unsigned target = 0;
     const GridWait wait{reinterpret_cast<unsigned*>(sp.counts + 6), polls, err, nullptr};
-    if (grid_barrier(wait, target, &s_fail)) {
-        for (int t = tid; t < nd; t += nthr) {
-            const int idx = nnew + t;
-            const float4 p = sp.pos[idx];
-            if (__float_as_int(p.w) < 0) continue;
-            const int h = __ldcg(&sp.holes[atomicAdd(&sp.counts[4], 1)]);
-            sp.pos[h] = p;
-            sp.vel[h] = sp.vel[idx];
-            sp.id[h] = sp.id[idx];
-        }
-    } else if (threadIdx.x == 0) {
-        set_error(err, kErrBarrierTimeout);
+    const bool ok = grid_barrier(wait, target, &s_fail);
+    if (ok)
+        for (int t = tid; t < nd; t += nthr) fill(nnew + t);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (!ok) set_error(err, kErrBarrierTimeout);
+        __threadfence();
+        const int left = atomicAdd(&sp.counts[7], ok ? 1 : 1 + kFailed);
+        s_last = (left & (kFailed - 1)) != (int)gridDim.x - 1 ? 0 : (ok && left < kFailed ? 1 : 2);
     }
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&sp.counts[7], 1) == (int)gridDim.x - 1) {
+    if (s_last == 2) {
+        __threadfence();
+        for (int t = threadIdx.x; t < nd; t += blockDim.x) fill(nnew + t);
+        __syncthreads();
+    }
+    if (s_last && threadIdx.x == 0) {
         sp.counts[0] = nnew;
         for (int c = 1; c < 8; c++)
             if (c != 5) sp.counts[c] = 0;
@@ -1028,13 +1043,13 @@ __global__ void k_from_abs_count(SpeciesDev sp, int n, unsigned* err) {
 }
 void launch_from_abs(const GridDev& g, SpeciesDev sp, const double* pos, const double* vel, const double* w,
                      const unsigned long long* id, unsigned long long id0, int n, int rewind, float qm_half_dt,
-                     const float4* ef, cudaStream_t s, int max_grid) {
+                     const float4* ef, unsigned* err, long long polls, cudaStream_t s, int max_grid) {
     int grid = (n + 255) / 256;
     if (grid > max_grid) grid = max_grid;
     if (grid < 1) grid = 1;
     k_from_abs<<<grid, 256, 0, s>>>(g, sp, pos, vel, w, id, id0, n, rewind, qm_half_dt, ef);
     k_from_abs_count<<<1, 1, 0, s>>>(sp, n, nullptr);
-    launch_compact(sp, CommitList{}, nullptr, kMbarWaitPolls, s);
+    launch_compact(sp, CommitList{}, err, polls, s);
 }
 
 // export of particles first, first + stride, ... (n of them) to absolute FP64 positions
