@@ -1364,13 +1364,13 @@ int push_species(pic_world* w, int sp, double dt, int deposit, bool with_mcc, bo
         launch_object_hits(o, w->stream, w->sms);
     }
     {
-        const bool neu = objects && s.charge != 0 && s.obj_neu != sp;
-        const bool spu = objects && s.charge != 0 && s.obj_sputtering && s.obj_spu != s.obj_neu && s.obj_spu != sp;
         Scope sc(w, "compact", 1);
         CommitList other;
-        if (a.coll.enabled) other.sp[other.n++] = w->sp[w->mcc_i].dev;
-        if (neu) other.sp[other.n++] = w->sp[s.obj_neu].dev;
-        if (spu) other.sp[other.n++] = w->sp[s.obj_spu].dev;
+        if (a.coll.enabled) other.add(w->sp[w->mcc_i].dev, s.dev);
+        if (objects && s.charge != 0) {
+            other.add(w->sp[s.obj_neu].dev, s.dev);
+            if (s.obj_sputtering) other.add(w->sp[s.obj_spu].dev, s.dev);
+        }
         launch_compact(s.dev, other, w->err, wait_polls(w), w->stream);
     }
     return PIC_OK;

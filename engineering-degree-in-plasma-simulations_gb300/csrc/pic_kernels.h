@@ -60,9 +60,17 @@ void launch_push(const PushArgs& a, cudaStream_t s, int grid);
 // push that follows runs without collisions.  cand holds up to the species capacity.
 void launch_mcc(const PushArgs& a, int* cand, int* ncand, cudaStream_t s, int sms);
 void launch_commit_appends(SpeciesDev sp, unsigned* err, cudaStream_t s);
-struct CommitList {  // species whose appends are committed beside a compaction
+// Species whose appends are committed beside a compaction, each once: a thread commits one entry, and two threads
+// on the same counts would race.
+struct CommitList {
     int n = 0;
     SpeciesDev sp[3];
+    // unless it is the compacted species (which commits too) or in the list
+    void add(const SpeciesDev& s, const SpeciesDev& compacted) {
+        bool known = s.counts == compacted.counts;
+        for (int k = 0; k < n; k++) known |= s.counts == sp[k].counts;
+        if (!known) sp[n++] = s;
+    }
 };
 // commits the appends of sp (and of the others) and removes its dead; polls: of the wait between the two
 // halves of the move
