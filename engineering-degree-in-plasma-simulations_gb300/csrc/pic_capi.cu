@@ -26,6 +26,7 @@ constexpr double kFp32Unit = 0x1p-24;  // unit roundoff of FP32 round-to-nearest
 constexpr long kUploadChunk = 1l << 22;  // particles per upload staging round (256 MB)
 constexpr int kClusterMost = 16;         // CTAs of the one-cluster inner solvers
 constexpr long kFieldChunk = 1l << 22;   // doubles per round of a node field's staging (32 MB)
+constexpr long kSmallStage = 1l << 13;   // and without device memory for it (64 KB, allocated with the world)
 constexpr long kSortMovedFraction = 50;   // re-sort a species when 2 % of it left cell order
 
 namespace {
@@ -155,7 +156,8 @@ struct pic_world {
     double time = 0.0;
     double* upload_buf = nullptr;  // particle upload staging (upload_cap particles, at most kUploadChunk)
     long upload_cap = 0;
-    std::mutex stage_mutex;  // held from the first to the last enqueued use of upload_buf in a call
+    double* small_stage = nullptr;  // kSmallStage doubles: staging of node fields where upload_buf cannot grow
+    std::mutex stage_mutex;  // held from the first to the last enqueued use of upload_buf and small_stage in a call
     // bound on the 2-norm of the rounding error of the FP32 residual r (valid with rhs_valid)
     double r_err = 0.0;
     // solver
@@ -641,6 +643,7 @@ extern "C" int pic_world_create(pic_world** out, int ni, int nj, int nk, const d
          alloc((void**)&w->scal, sizeof(double) * 16) && alloc((void**)&w->flag, sizeof(int) * 4) &&
          alloc((void**)&w->gpart, sizeof(double) * 8 * (size_t)std::max(kParts, 2 * node_blocks(nv))) &&
          alloc((void**)&w->ticket, sizeof(unsigned) * 4) &&
+         alloc((void**)&w->small_stage, sizeof(double) * kSmallStage) &&
          alloc((void**)&w->cell_count, sizeof(int) * (g.nc + 1)) &&
          alloc((void**)&w->cell_start, sizeof(int) * (g.nc + 1)) &&
          alloc((void**)&w->scan_aux, sizeof(int) * (g.nc / 2048 + 2)) && alloc((void**)&w->err, sizeof(unsigned)) &&
@@ -707,7 +710,7 @@ extern "C" int pic_world_destroy(pic_world* w) {
     }
     void* ptrs[] = {w->ef,   w->phi,  w->phi_alt, w->rho,        w->kind,       w->r,        w->e,
                     w->d,    w->d2,   w->q,       w->z,          w->part,       w->scal,     w->flag,
-                    w->gpart, w->ticket,
+                    w->gpart, w->ticket, w->small_stage,
                     w->cell_count,    w->cell_start,             w->scan_aux,   w->err,      w->tE,
                     w->tS,   w->stats,  w->merge_list, w->merge_stats};
     for (void* p : ptrs)
@@ -811,28 +814,39 @@ int ensure_upload(pic_world* w, long n) {
     }
     return PIC_OK;
 }
-// the same buffer as FP64 staging of node fields, per_node doubles a node: *nodes of it fit (at most
-// kFieldChunk doubles are used)
-int ensure_field_stage(pic_world* w, int per_node, int* nodes) {
+// FP64 staging of node fields, per_node doubles a node: *nodes of it fit *buf.  The particle staging grows to
+// kFieldChunk doubles at most for it; where the device has no memory left, fields go through what there is
+struct FieldStage {
+    double* buf;
+    int nodes;
+};
+FieldStage field_stage(pic_world* w, int per_node) {
     const long vals = std::min<long>(kFieldChunk, (long)w->g.nv * per_node);
-    int rc = ensure_upload(w, (vals + 7) / 8);
-    if (rc) return rc;
-    *nodes = (int)(std::min<long>(kFieldChunk, w->upload_cap * 8) / per_node);
-    return PIC_OK;
+    if (vals > kSmallStage && w->upload_cap * 8 < vals) {
+        double* b = nullptr;
+        const long cap = (vals + 7) / 8;
+        if (cudaMalloc(&b, (size_t)cap * 8 * sizeof(double)) == cudaSuccess) {
+            if (w->upload_buf) cudaFree(w->upload_buf);
+            w->upload_buf = b;
+            w->upload_cap = cap;
+        } else {
+            cudaGetLastError();
+        }
+    }
+    if (vals <= kSmallStage || w->upload_cap * 8 < kSmallStage) return {w->small_stage, (int)(kSmallStage / per_node)};
+    return {w->upload_buf, (int)(std::min<long>(kFieldChunk, w->upload_cap * 8) / per_node)};
 }
 // a node field of per_node doubles a node to the caller's array, from(first node, nodes, staging)
 // filling the staging buffer on the world's stream
 template <class F>
 int field_out(pic_world* w, int per_node, double* out, F from) {
     std::lock_guard<std::mutex> lock(w->stage_mutex);
-    int cap = 0;
-    int rc = ensure_field_stage(w, per_node, &cap);
-    if (rc) return rc;
+    const FieldStage st = field_stage(w, per_node);
     touch_pages(out, sizeof(double) * per_node * (size_t)w->g.nv);
-    for (int a = 0; a < w->g.nv; a += cap) {
-        const int m = std::min(cap, w->g.nv - a);
-        from(a, m, w->upload_buf);
-        CU(cudaMemcpyAsync(out + (size_t)per_node * a, w->upload_buf, sizeof(double) * per_node * m,
+    for (int a = 0; a < w->g.nv; a += st.nodes) {
+        const int m = std::min(st.nodes, w->g.nv - a);
+        from(a, m, st.buf);
+        CU(cudaMemcpyAsync(out + (size_t)per_node * a, st.buf, sizeof(double) * per_node * m,
                            cudaMemcpyDeviceToHost, w->stream));
     }
     CU(cudaStreamSynchronize(w->stream));
@@ -842,14 +856,12 @@ int field_out(pic_world* w, int per_node, double* out, F from) {
 template <class F>
 int field_in(pic_world* w, int per_node, const double* in, F to) {
     std::lock_guard<std::mutex> lock(w->stage_mutex);
-    int cap = 0;
-    int rc = ensure_field_stage(w, per_node, &cap);
-    if (rc) return rc;
-    for (int a = 0; a < w->g.nv; a += cap) {
-        const int m = std::min(cap, w->g.nv - a);
-        CU(cudaMemcpyAsync(w->upload_buf, in + (size_t)per_node * a, sizeof(double) * per_node * m,
-                           cudaMemcpyHostToDevice, w->stream));
-        to(a, m, w->upload_buf);
+    const FieldStage st = field_stage(w, per_node);
+    for (int a = 0; a < w->g.nv; a += st.nodes) {
+        const int m = std::min(st.nodes, w->g.nv - a);
+        CU(cudaMemcpyAsync(st.buf, in + (size_t)per_node * a, sizeof(double) * per_node * m, cudaMemcpyHostToDevice,
+                           w->stream));
+        to(a, m, st.buf);
     }
     CU(cudaStreamSynchronize(w->stream));
     CU(cudaGetLastError());
@@ -1436,10 +1448,9 @@ extern "C" int pic_species_gas_properties(pic_world* w, int sp, double* vel, dou
         return PIC_OK;
     }
     std::lock_guard<std::mutex> lock(w->stage_mutex);
-    int cap = 0;
-    int rc = ensure_field_stage(w, 4, &cap);
-    if (rc) return rc;
-    double *dv = w->upload_buf, *dt = dv + 3 * (size_t)cap;
+    const FieldStage st = field_stage(w, 4);
+    const int cap = st.nodes;
+    double *dv = st.buf, *dt = dv + 3 * (size_t)cap;
     if (vel) touch_pages(vel, sizeof(double) * 3 * (size_t)nv);
     if (T) touch_pages(T, sizeof(double) * (size_t)nv);
     for (int a = 0; a < nv; a += cap) {
