@@ -486,14 +486,8 @@ void free_lp(pic_world* w) {
     w->lp = nullptr;
 }
 
-// the learned preconditioner of the world's current grid and periodic axes (created on first use,
-// weights at their multilevel-diagonal start)
-int ensure_lp(pic_world* w) {
+int build_lp(pic_world* w) {
     const GridDev& g = w->g;
-    if (w->lp && w->lp->per[0] == w->periodic[0] && w->lp->per[1] == w->periodic[1] &&
-        w->lp->per[2] == w->periodic[2])
-        return PIC_OK;
-    free_lp(w);
     int n0[3] = {g.ni - w->periodic[0], g.nj - w->periodic[1], g.nk - w->periodic[2]};
     if (std::min(n0[0], std::min(n0[1], n0[2])) < 2)
         return fail(PIC_ERR_ARG, "the learned preconditioner needs at least 2 distinct nodes per axis");
@@ -532,8 +526,13 @@ int ensure_lp(pic_world* w) {
         const int* d = L->dims[L->dense_level];
         const size_t n = (size_t)d[0] * d[1] * d[2];
         L->dense_pitch = (int)(n + 3) / 4 * 4;
-        CU(cudaMalloc(&L->dense, sizeof(float) * n * L->dense_pitch));
-        CU(cudaMemsetAsync(L->dense, 0, sizeof(float) * n * L->dense_pitch, w->stream));  // the rows' padding
+        if (cudaMalloc(&L->dense, sizeof(float) * n * L->dense_pitch) == cudaSuccess) {
+            CU(cudaMemsetAsync(L->dense, 0, sizeof(float) * n * L->dense_pitch, w->stream));  // the rows' padding
+        } else {  // no memory for it (16 MB at most): every level is applied by itself
+            cudaGetLastError();
+            L->dense = nullptr;
+            L->dense_level = L->nlev;
+        }
     }
     std::vector<float> hw(L->lay.total);
     lp_init_weights(L->lay, L->diag, L->nlev, hw.data());
@@ -542,6 +541,18 @@ int ensure_lp(pic_world* w) {
     CU(cudaStreamSynchronize(w->stream));
     CU(cudaGetLastError());
     return PIC_OK;
+}
+
+// the learned preconditioner of the world's current grid and periodic axes (created on first use,
+// weights at their multilevel-diagonal start)
+int ensure_lp(pic_world* w) {
+    if (w->lp && w->lp->per[0] == w->periodic[0] && w->lp->per[1] == w->periodic[1] &&
+        w->lp->per[2] == w->periodic[2])
+        return PIC_OK;
+    free_lp(w);
+    const int rc = build_lp(w);
+    if (rc) free_lp(w);  // nothing half made is left for the next call
+    return rc;
 }
 
 int ensure_lp_train(pic_world* w) {
