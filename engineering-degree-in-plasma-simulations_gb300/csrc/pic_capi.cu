@@ -106,8 +106,11 @@ struct pic_world {
     unsigned* ticket = nullptr;  // last-block counter of those reductions
     double* scal = nullptr;
     int* flag = nullptr;
-    double* h_scal = nullptr;  // pinned
-    int* h_flag = nullptr;     // pinned
+    double* h_scal = nullptr;  // pinned: the solver's scalars
+    int* h_flag = nullptr;     // pinned: [0..2] the solver's flags, [3] the device error word
+    double* h_diag = nullptr;  // pinned: results of the diagnostics, which other host threads may ask for during a solve
+    std::mutex diag_mutex;     // held from a diagnostic's launch until its result has been read from h_diag
+    std::mutex err_mutex;      // held while h_flag[3] is in use
     // cells
     int* cell_count = nullptr;
     int* cell_start = nullptr;
@@ -262,6 +265,7 @@ void collect_timers(pic_world* w) {
 
 long long wait_polls(const pic_world* w) { return wait_poll_limit(w->wait_polls_arg, kMbarWaitPolls); }
 int check_device_error(pic_world* w) {
+    std::lock_guard<std::mutex> lock(w->err_mutex);
     CU(cudaMemcpyAsync(w->h_flag + 3, w->err, sizeof(unsigned), cudaMemcpyDeviceToHost, w->stream));
     CU(cudaStreamSynchronize(w->stream));
     const unsigned h = (unsigned)w->h_flag[3];
@@ -659,7 +663,8 @@ extern "C" int pic_world_create(pic_world** out, int ni, int nj, int nk, const d
          alloc((void**)&w->cell_start, sizeof(int) * (g.nc + 1)) &&
          alloc((void**)&w->scan_aux, sizeof(int) * (g.nc / 2048 + 2)) && alloc((void**)&w->err, sizeof(unsigned)) &&
          cudaMallocHost((void**)&w->h_scal, sizeof(double) * 16) == cudaSuccess &&
-         cudaMallocHost((void**)&w->h_flag, sizeof(int) * 4) == cudaSuccess;
+         cudaMallocHost((void**)&w->h_flag, sizeof(int) * 4) == cudaSuccess &&
+         cudaMallocHost((void**)&w->h_diag, sizeof(double) * 5) == cudaSuccess;
     if (!ok) {
         pic_world_destroy(w);
         return fail(PIC_ERR_CUDA, "device allocation failed for a %d x %d x %d grid", ni, nj, nk);
@@ -727,6 +732,7 @@ extern "C" int pic_world_destroy(pic_world* w) {
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (w->h_scal) cudaFreeHost(w->h_scal);
+    if (w->h_diag) cudaFreeHost(w->h_diag);
     if (w->upload_buf) cudaFree(w->upload_buf);
     if (w->h_flag) cudaFreeHost(w->h_flag);
     for (auto& p : w->pending) {
@@ -938,16 +944,17 @@ extern "C" int pic_world_get_field(pic_world* w, int which, double* out) {
 extern "C" int pic_world_potential_energy(pic_world* w, double* pe) {
     if (!w || !pe) return fail(PIC_ERR_ARG, "null argument");
     CU(cudaSetDevice(w->device));
+    std::lock_guard<std::mutex> lock(w->diag_mutex);
     const int grid = 6 * w->sms;  // one resident wave
     double* total = w->part + grid;
     {
         Scope sc(w, "diagnostics", 1);
         launch_field_energy(w->g, w->ef, w->part, w->ticket, total, w->stream, grid);
     }
-    CU(cudaMemcpyAsync(w->h_scal, total, sizeof(double), cudaMemcpyDeviceToHost, w->stream));
+    CU(cudaMemcpyAsync(w->h_diag, total, sizeof(double), cudaMemcpyDeviceToHost, w->stream));
     const int rc = check_device_error(w);  // synchronises
     const GridDev& g = w->g;
-    *pe = 0.5 * kEps0 * g.dxd[0] * g.dxd[1] * g.dxd[2] * w->h_scal[0];
+    *pe = 0.5 * kEps0 * g.dxd[0] * g.dxd[1] * g.dxd[2] * w->h_diag[0];
     return rc;
 }
 extern "C" int pic_world_set_field(pic_world* w, int which, const double* in) {
@@ -1570,6 +1577,7 @@ extern "C" int pic_species_sort(pic_world* w, int sp, int32_t* cell_counts) {
 extern "C" int pic_species_sums(pic_world* w, int sp, double* out) {
     if (!valid_sp(w, sp) || !out) return fail(PIC_ERR_ARG, "bad arguments");
     CU(cudaSetDevice(w->device));
+    std::lock_guard<std::mutex> lock(w->diag_mutex);
     // one resident wave of CTAs (5 partials per CTA fit the partial buffer)
     const int grid = std::min(6 * w->sms, kParts * 8 / 5 - 1);
     double* total = w->part + 5 * (size_t)grid;
@@ -1577,9 +1585,9 @@ extern "C" int pic_species_sums(pic_world* w, int sp, double* out) {
         Scope sc(w, "sums", 1);
         launch_sums(w->sp[sp].dev, w->part, w->ticket, total, w->stream, grid);
     }
-    CU(cudaMemcpyAsync(w->h_scal, total, sizeof(double) * 5, cudaMemcpyDeviceToHost, w->stream));
+    CU(cudaMemcpyAsync(w->h_diag, total, sizeof(double) * 5, cudaMemcpyDeviceToHost, w->stream));
     const int rc = check_device_error(w);  // synchronises
-    const double* t = w->h_scal;
+    const double* t = w->h_diag;
     double m = w->sp[sp].mass;
     out[0] = t[0];
     out[1] = t[1] * m;
