@@ -1713,7 +1713,7 @@ constexpr double kInnerTarget = 0.64;
 
 // a bounded wait of an inner solver ran out (flag[2], read into h_flag[2]): the solve ends with an error
 int inner_wait_failed(pic_world* w) {
-    w->rhs_valid = false;
+    w->rhs_valid = w->dphi_valid = false;
     CU(cudaMemsetAsync(w->flag, 0, sizeof(int) * 4, w->stream));
     CU(cudaMemsetAsync(w->ticket, 0, sizeof(unsigned) * 4, w->stream));  // counters of a barrier left half-way
     int rc = check_device_error(w);
@@ -1944,7 +1944,10 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
         }
         rc = residual_norms(w, sw, 1, r2, b2, s2);
         if (rc) return rc;
-        if (waited && w->h_flag[2]) return inner_wait_failed(w);
+        if (waited && w->h_flag[2]) {
+            std::swap(w->phi, w->phi_alt);  // the potential without the unfinished correction
+            return inner_wait_failed(w);
+        }
         bn = stop_scale(w, b2, s2);
         rel = std::sqrt(r2) / bn;
         if (!(rel == rel)) break;  // NaN: diverged
