@@ -1720,16 +1720,17 @@ int inner_wait_failed(pic_world* w) {
     return rc ? rc : fail(PIC_ERR_DEVICE, "a bounded wait of the Poisson solver expired");
 }
 
-// FP32 flexible CG with the learned preconditioner on L e = r (w->r), e from zero, until
+// FP32 flexible CG with the learned preconditioner on L e = r (w->r, r.r = r2), e from zero, until
 // r.r <= target or cap iterations; *done = iterations, *conv = reached the target.  Iterations go
 // out in batches between which the host reads the stop flag (the iterations of a batch after the
 // stop return at once, about 30 us each at 256^3): first_batch, then 2, 4, 4, ...
-int learned_inner(pic_world* w, SolveWork& sw, double target, int cap, int first_batch, int* done, bool* conv) {
+int learned_inner(pic_world* w, SolveWork& sw, double r2, double target, int cap, int first_batch, int* done, bool* conv) {
     if (plan_lpcg_grid(w->g, *w->lp, w->sms)) {
         // the whole solve in one launch; the residual's partner is the unused one of the two potentials
         {
             Scope sc(w, "poisson", 1);
-            launch_lpcg_grid(w->g, sw, *w->lp, w->d2, reinterpret_cast<float*>(sw.phi_alt), target, cap, w->stream, w->sms);
+            launch_lpcg_grid(w->g, sw, *w->lp, w->d2, reinterpret_cast<float*>(sw.phi_alt), r2, target, cap, w->stream,
+                             w->sms);
         }
         CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
         CU(cudaStreamSynchronize(w->stream));
@@ -1780,7 +1781,7 @@ int learned_validation_iters(pic_world* w, const float* r, int cap, int* iters) 
     CU(cudaStreamSynchronize(w->stream));
     SolveWork sw = solve_work(w);
     bool conv = false;
-    int rc = learned_inner(w, sw, 1e-12 * w->h_scal[0], cap, 4, iters, &conv);
+    int rc = learned_inner(w, sw, w->h_scal[0], 1e-12 * w->h_scal[0], cap, 4, iters, &conv);
     if (!conv) *iters = cap;
     return rc;
 }
@@ -1884,7 +1885,7 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
             // first N converged, so the first batch runs N + 1 iterations (a cold solve, which needs
             // several times more, neither uses nor sets the count)
             const int first_batch = warm && first_learned && w->lp_hint > 0 ? w->lp_hint + 1 : 4;
-            rc = learned_inner(w, sw, target, std::min(kLearnedInnerCap, w->max_it - iters), first_batch, &done, &conv);
+            rc = learned_inner(w, sw, r2, target, std::min(kLearnedInnerCap, w->max_it - iters), first_batch, &done, &conv);
             if (rc) return rc;
             if (warm && first_learned && conv) w->lp_hint = done;
             first_learned = false;
@@ -1906,9 +1907,9 @@ int solve_impl(pic_world* w, int* iters_out, double* rel_out) {
                 Scope sc(w, "poisson", 1);
                 const int most = std::min(cap, w->max_it - iters);
                 if (w->pcg_planes > 0)
-                    launch_pcg_cluster(w->g, sw, target, most, w->pcg_planes, w->stream);
+                    launch_pcg_cluster(w->g, sw, r2, target, most, w->pcg_planes, w->stream);
                 else
-                    launch_pcg_grid(w->g, sw, target, most, w->pcg_chunk, w->stream);
+                    launch_pcg_grid(w->g, sw, r2, target, most, w->pcg_chunk, w->stream);
                 CU(cudaMemcpyAsync(w->h_flag, w->flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, w->stream));
                 CU(cudaStreamSynchronize(w->stream));
                 if (w->h_flag[2]) return inner_wait_failed(w);

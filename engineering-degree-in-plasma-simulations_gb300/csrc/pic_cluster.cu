@@ -17,6 +17,7 @@
 // The arithmetic of a node is that of k_rbsor and k_pcg_* (pic_fields.cu), in the same order.
 #include <algorithm>
 #include "pic_ff.cuh"
+#include "pic_grid_sync.cuh"
 #include "pic_stencil.cuh"
 
 namespace pic {
@@ -39,7 +40,12 @@ __device__ __forceinline__ unsigned map_rank(const void* p, unsigned rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
-// remote store that counts its bytes on an mbarrier of the receiving CTA
+// remote stores that count their bytes on an mbarrier of the receiving CTA
+__device__ __forceinline__ void st_async2(unsigned a, float x, float y, unsigned bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(a), "f"(x),
+                 "f"(y), "r"(bar)
+                 : "memory");
+}
 __device__ __forceinline__ void st_async(unsigned a, float v, unsigned bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(a), "f"(v), "r"(bar)
                  : "memory");
@@ -293,28 +299,26 @@ __global__ void __launch_bounds__(1024, 1) k_sor_cluster(GridDev g, float* __res
 // ------------------------------------------------------------------------------------
 // the whole inner CG solve of L e = r from e = 0 (the iteration of k_pcg_k1 / k_pcg_k2)
 // ------------------------------------------------------------------------------------
-// Sums of N per-thread values over the cluster, in every lane of warp 0 of every CTA: FP32 within a
-// warp, float-float (48 bits) over the warps of the cluster in a fixed order.  Every warp sends its
+// Sums of N per-thread values over the cluster, times scale, in every lane of warp 0 of every CTA, float-float
+// (48 bits) in a fixed order (scale and what rounds as in grid_total).  Every warp sends its
 // partials straight to all CTAs (red, counted on bar), so a sum is one message deep and costs no block
 // barrier.  FP64 is kept out of this chain: its adds and above all its divides run on a pipe so narrow
 // here that they were a third of an iteration.  False when the partials did not arrive in time.
 template <int N, int NW>
-__device__ __forceinline__ bool cluster_sum(const float (&v)[N], float (*red)[kMaxCtas * NW], int ctas,
+__device__ __forceinline__ bool cluster_sum(const FF (&v)[N], const float (&scale)[N], float2 (*red)[kMaxCtas * NW], int ctas,
                                             unsigned long long* bar, unsigned parity, long long polls, FF (&out)[N]) {
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) bar_expect(bar, 4u * N * NW * (unsigned)ctas);
-    float x[N];
+    if (threadIdx.x == 0) bar_expect(bar, 8u * N * NW * (unsigned)ctas);
+    const FF x = warp_halved(v);
+    FF p[N];
 #pragma unroll
-    for (int c = 0; c < N; c++) x[c] = v[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < N; c++) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
+    for (int c = 0; c < N; c++)
+        p[c] = FF{__shfl_sync(0xffffffffu, x.hi, warp_home<N>(c)) * scale[c], __shfl_sync(0xffffffffu, x.lo, warp_home<N>(c)) * scale[c]};
     if (lane < ctas) {
         const unsigned rb = map_rank(bar, (unsigned)lane);
 #pragma unroll
         for (int c = 0; c < N; c++)
-            st_async(map_rank(&red[c][cluster_rank() * NW + wp], (unsigned)lane), x[c], rb);
+            st_async2(map_rank(&red[c][cluster_rank() * NW + wp], (unsigned)lane), p[c].hi, p[c].lo, rb);
     }
     if (wp != 0) return true;
     const bool ok = bar_wait(bar, parity, polls);
@@ -323,24 +327,9 @@ __device__ __forceinline__ bool cluster_sum(const float (&v)[N], float (*red)[kM
     for (int c = 0; c < N; c++) out[c] = FF{0.f, 0.f};
     for (int y = lane; y < ctas * NW; y += 32)
 #pragma unroll
-        for (int c = 0; c < N; c++) {
-            const FF t = two_sum(out[c].hi, red[c][y]);
-            out[c] = FF{t.hi, out[c].lo + t.lo};
-        }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < N; c++) {
-            const FF t{__shfl_xor_sync(0xffffffffu, out[c].hi, o), __shfl_xor_sync(0xffffffffu, out[c].lo, o)};
-            out[c] = ff_add(out[c], t);
-        }
+        for (int c = 0; c < N; c++) out[c] = ff_gather(out[c], FF{red[c][y].x, red[c][y].y});
+    warp_total(out);
     return ok;
-}
-// a / b rounded to FP32: one FP32 quotient and its correction by the exact remainder
-__device__ __forceinline__ float ff_quotient(FF a, FF b) {
-    const float q = a.hi / b.hi;
-    const float rem = fmaf(-q, b.hi, a.hi) + (a.lo - q * b.lo);
-    return q + rem / b.hi;
 }
 
 // flag[0]: converged (r.r <= target), flag[1]: iterations done.  A thread keeps K nodes (x = tid + m NT of
@@ -350,12 +339,13 @@ __device__ __forceinline__ float ff_quotient(FF a, FF b) {
 // value was read.
 template <int NT, int K>
 __global__ void __launch_bounds__(NT, 1) k_pcg_cluster(GridDev g, float* __restrict__ e, const float* __restrict__ r,
-                                                       const uint16_t* __restrict__ kind, FF target, int cap, int planes,
-                                                       int* flag, ClusterWait wait) {
+                                                       const uint16_t* __restrict__ kind, SumScales sc, FF target, int cap,
+                                                       int planes, int* flag, ClusterWait wait) {
     constexpr int NW = NT / 32;
+    const float sc1[1] = {sc.rz}, sc3[3] = {sc.rz, sc.rz, sc.rr};
     extern __shared__ __align__(16) float sm[];
     float* D = sm;  // direction, (planes + 2) * nij
-    __shared__ float red1[1][kMaxCtas * NW], red3[3][kMaxCtas * NW];
+    __shared__ float2 red1[1][kMaxCtas * NW], red3[3][kMaxCtas * NW];
     __shared__ __align__(8) unsigned long long bar_d, bar_1, bar_3;
     __shared__ float inv_tab[64], dia_tab[64];
     __shared__ float s_alpha, s_beta;
@@ -378,7 +368,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_cluster(GridDev g, float* __restr
     }
     for (int x = tid; x < (s.np + 2) * nij; x += NT) D[x] = 0.f;
     __syncthreads();
-    float R[K], X[K], Q[K], f[3] = {0.f, 0.f, 0.f};
+    static_assert(K <= kFp32Nodes, "a thread's FP32 sums");
+    float R[K], X[K], Q[K], f = 0.f;
     unsigned M[K];  // 0: no unknown; bit 0 set, mirror mask (6 bits), wrap flags (4 bits)
 #pragma unroll
     for (int m = 0; m < K; m++) {
@@ -392,7 +383,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_cluster(GridDev g, float* __restr
         node_ijk(g, n0 + x, i, j, k);
         M[m] = 1u | ((kd >> 2) & 63u) << 1 | wrap_flags(g, i, j) << 7;
         R[m] = r[n0 + x];
-        f[0] += R[m] * (R[m] * inv_tab[(kd >> 2) & 63u]);
+        f += R[m] * (R[m] * inv_tab[(kd >> 2) & 63u]);
     }
     for (int x = tid; x < 2 * nij; x += NT) {
         const int n = halo_node(s, x);
@@ -401,7 +392,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_cluster(GridDev g, float* __restr
     cluster_sync();  // every CTA's halo planes are zero and its barriers are there
     FF t1[1], t3[3], rz;
     unsigned ph3 = 0, ph = 0;
-    bool ok = cluster_sum<3, NW>(f, red3, ctas, &bar_3, ph3, wait.polls, t3);  // r.z
+    const FF v0[3] = {FF{f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}};
+    bool ok = cluster_sum<3, NW>(v0, sc3, red3, ctas, &bar_3, ph3, wait.polls, t3);  // r.z
     ph3 ^= 1u;
     rz = t3[0];
     if (tid == 0 && !ok) s_stop = 2;
@@ -424,7 +416,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_cluster(GridDev g, float* __restr
             break;
         }
         // q = L d, d.q
-        float v1[1] = {0.f};
+        float f1 = 0.f;
 #pragma unroll
         for (int m = 0; m < K; m++) {
             if (!M[m]) continue;
@@ -438,18 +430,19 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_cluster(GridDev g, float* __restr
             for (int d = 0; d < 6; d++) off += c3[d >> 1] * dp[o[d]];  // zero on MIRROR and FIXED nodes
             const float dn = dp[0];
             Q[m] = dia_tab[(M[m] >> 1) & 63u] * dn - off;
-            v1[0] += dn * Q[m];
+            f1 += dn * Q[m];
         }
-        ok = cluster_sum<1, NW>(v1, red1, ctas, &bar_1, ph, wait.polls, t1);
+        const FF v1[1] = {FF{f1, 0.f}};
+        ok = cluster_sum<1, NW>(v1, sc1, red1, ctas, &bar_1, ph, wait.polls, t1);
         if (tid == 0) {
-            s_alpha = t1[0].hi != 0.f ? ff_quotient(rz, t1[0]) : 0.f;
+            s_alpha = t1[0].hi != 0.f ? ff_ratio(rz, t1[0]) : 0.f;
             if (!ok) s_stop = 2;
         }
         __syncthreads();
         if (s_stop) break;
         // e += alpha d, r -= alpha q, z = r / D
         const float alpha = s_alpha;
-        float v3[3] = {0.f, 0.f, 0.f};
+        float f3[3] = {0.f, 0.f, 0.f};
 #pragma unroll
         for (int m = 0; m < K; m++) {
             if (!M[m]) continue;
@@ -458,18 +451,19 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_cluster(GridDev g, float* __restr
             const float ro = R[m];
             const float rn = ro - alpha * Q[m];
             const float zn = rn * inv;
-            v3[0] += rn * zn;
-            v3[1] += rn * (ro * inv);
-            v3[2] += rn * rn;
+            f3[0] += rn * zn;
+            f3[1] += rn * (ro * inv);
+            f3[2] += rn * rn;
             R[m] = rn;
         }
-        ok = cluster_sum<3, NW>(v3, red3, ctas, &bar_3, ph3, wait.polls, t3);
+        const FF v3[3] = {FF{f3[0], 0.f}, FF{f3[1], 0.f}, FF{f3[2], 0.f}};
+        ok = cluster_sum<3, NW>(v3, sc3, red3, ctas, &bar_3, ph3, wait.polls, t3);
         it++;
         if (tid == 0) {
             const float over = (t3[2].hi - target.hi) + (t3[2].lo - target.lo);
             if (!ok) s_stop = 2;
             else if (!(over > 0.f)) s_stop = over <= 0.f ? 1 : 3;  // converged, or not a number
-            s_beta = ff_quotient(ff_add(t3[0], ff_neg(t3[1])), rz);
+            s_beta = ff_ratio(ff_add(t3[0], ff_neg(t3[1])), rz);
         }
         rz = t3[0];
         ph ^= 1u;
@@ -530,7 +524,7 @@ bool fits(K kernel, int ctas, int threads, size_t smem) {
     cudaGetLastError();  // a cluster of this size does not fit this GPU
     return false;
 }
-using PcgKernel = void (*)(GridDev, float*, const float*, const uint16_t*, FF, int, int, int*, ClusterWait);
+using PcgKernel = void (*)(GridDev, float*, const float*, const uint16_t*, SumScales, FF, int, int, int*, ClusterWait);
 // the smallest form whose registers hold a CTA's nodes
 PcgKernel pcg_kernel(long own, int* threads) {
     *threads = own <= 2048 ? 256 : 512;
@@ -578,15 +572,16 @@ void launch_sor_cluster(const GridDev& g, SolveWork& w, float omega, int sweeps,
     cudaLaunchKernelEx(&cfg, k_sor_cluster, g, w.e, (const float*)w.r, reinterpret_cast<const uint16_t*>(w.kind), omega,
                        sweeps, planes, ClusterWait{w.wait_polls, w.err, w.flag + 2});
 }
-void launch_pcg_cluster(const GridDev& g, SolveWork& w, double target_rr, int cap, int planes, cudaStream_t s) {
+void launch_pcg_cluster(const GridDev& g, SolveWork& w, double r2, double target_rr, int cap, int planes, cudaStream_t s) {
     const long nij = (long)g.ni * g.nj;
     int threads;
     PcgKernel k = pcg_kernel(nij * planes, &threads);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     fill_config((stack_planes(g) + planes - 1) / planes, threads, pcg_smem(nij, planes), s, cfg, at);
-    cudaLaunchKernelEx(&cfg, k, g, w.e, (const float*)w.r, reinterpret_cast<const uint16_t*>(w.kind),
-                       ff_from_double(target_rr), cap, planes, w.flag, ClusterWait{w.wait_polls, w.err, w.flag + 2});
+    const SumScales sc = sum_scales(g, r2);
+    cudaLaunchKernelEx(&cfg, k, g, w.e, (const float*)w.r, reinterpret_cast<const uint16_t*>(w.kind), sc,
+                       ff_from_double(target_rr * sc.rr), cap, planes, w.flag, ClusterWait{w.wait_polls, w.err, w.flag + 2});
 }
 
 }  // namespace pic

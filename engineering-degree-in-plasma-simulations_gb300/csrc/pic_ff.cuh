@@ -42,6 +42,21 @@ __device__ __forceinline__ FF ff_add_f(FF a, float b) {
     FF s = two_sum(a.hi, b);
     return two_sum(s.hi, s.lo + a.lo);
 }
+// a + t and a + b for running sums: the high parts by TwoSum, the low parts collected (normalised once at the end)
+__device__ __forceinline__ FF ff_acc(FF a, float t) {
+    const FF s = two_sum(a.hi, t);
+    return FF{s.hi, a.lo + s.lo};
+}
+__device__ __forceinline__ FF ff_gather(FF a, FF b) {
+    const FF s = two_sum(a.hi, b.hi);
+    return FF{s.hi, a.lo + (b.lo + s.lo)};
+}
+// a / b rounded to FP32: one FP32 quotient and its correction by the exact remainder
+__device__ __forceinline__ float ff_ratio(FF a, FF b) {
+    const float q = a.hi / b.hi;
+    const float rem = fmaf(-q, b.hi, a.hi) + (a.lo - q * b.lo);
+    return q + rem / b.hi;
+}
 __device__ __forceinline__ FF ff_neg(FF a) { return FF{-a.hi, -a.lo}; }
 // a - b for stored values, unnormalised (the high parts exactly, the low parts in FP32)
 __device__ __forceinline__ FF ff_diff(float2 a, float2 b) {

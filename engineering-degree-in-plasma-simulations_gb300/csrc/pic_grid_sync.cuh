@@ -39,44 +39,74 @@ struct GridSync {
     unsigned pad[31];
     float2 part[4][kMostCtas];  // float-float partials: d.q, then the three sums after the update
 };
-// a + t, the high parts by TwoSum, the low parts collected (normalised once at the end of a sum)
-__device__ __forceinline__ FF ff_gather(FF a, FF t) {
-    const FF s = two_sum(a.hi, t.hi);
-    return FF{s.hi, a.lo + (t.lo + s.lo)};
-}
 constexpr int kAtOnce = 5;  // partials a lane reads at once: 152 CTAs in one go
-// Sums of N per-thread values over the grid, in every lane of warp 0 of every CTA: FP32 within a warp,
-// float-float over the warps and the CTAs, in a fixed order; passes one grid barrier (false: it failed).
-// part: the N slots of this sum, not read by anyone since the last barrier but one.
-template <int N, int NT>
-__device__ __forceinline__ bool grid_total(const float (&v)[N], float (*wsum)[NT / 32], float2 (*part)[kMostCtas],
-                                           const GridWait& w, unsigned& target, int* s_fail, FF (&out)[N]) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    float x[N];
-#pragma unroll
-    for (int c = 0; c < N; c++) x[c] = v[c];
+// sums over a warp in every lane
+template <int N>
+__device__ __forceinline__ void warp_total(FF (&x)[N]) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int c = 0; c < N; c++) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
-    if (lane == 0)
+        for (int c = 0; c < N; c++)
+            x[c] = ff_gather(x[c], FF{__shfl_xor_sync(0xffffffffu, x[c].hi, o), __shfl_xor_sync(0xffffffffu, x[c].lo, o)});
 #pragma unroll
-        for (int c = 0; c < N; c++) wsum[c][wp] = x[c];
-    auto tree = [&]() {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int c = 0; c < N; c++)
-                out[c] = ff_gather(out[c], FF{__shfl_xor_sync(0xffffffffu, out[c].hi, o),
-                                              __shfl_xor_sync(0xffffffffu, out[c].lo, o)});
-#pragma unroll
-        for (int c = 0; c < N; c++) out[c] = two_sum(out[c].hi, out[c].lo);
+    for (int c = 0; c < N; c++) x[c] = two_sum(x[c].hi, x[c].lo);
+}
+// One warp's sum of each of N values: value c ends in lane warp_home<N>(c).  The shuffles bound the sums of all warps
+// of a CTA, so a lane hands over the half of the values that it does not keep first: 12 shuffles of 32 bits for
+// three values instead of 30.
+template <int N>
+__device__ __forceinline__ constexpr int warp_home(int c) {
+    return N == 2 ? 16 * c : 8 * c;
+}
+template <int N>
+__device__ __forceinline__ FF warp_halved(const FF (&x)[N]) {
+    static_assert(N >= 1 && N <= 3, "the steps below");
+    const int lane = threadIdx.x & 31;
+    auto from = [](FF v, int o) {
+        return FF{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
     };
+    const bool up = lane & 16, up8 = lane & 8;
+    FF a = x[0];
+    if (N == 1) {
+        a = ff_gather(a, from(a, 16));
+        a = ff_gather(a, from(a, 8));
+    } else if (N == 2) {
+        a = ff_gather(up ? x[N - 1] : x[0], from(up ? x[0] : x[N - 1], 16));
+        a = ff_gather(a, from(a, 8));
+    } else {  // value 2 goes up, then value 1
+        a = ff_gather(up ? x[N - 1] : x[0], from(up ? x[0] : x[N - 1], 16));
+        const FF b = ff_gather(x[N / 2], from(x[N / 2], 16));
+        a = ff_gather(up8 ? b : a, from(up8 ? a : b, 8));
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a = ff_gather(a, from(a, o));
+    return two_sum(a.hi, a.lo);
+}
+// Sums of N per-thread values over the grid, times scale, in every lane of warp 0 of every CTA, in a fixed order;
+// passes one grid barrier (false: it failed).  part: the N slots of this sum, not read by anyone since the last
+// barrier but one.  Float-float from the threads' values on (48 bits), since FP64 runs at two operations a clock
+// and SM; only the sums of kFp32Nodes nodes at most that a thread adds first round at FP32.  Against FP64 a sum of
+// |r|^2 is off by 2.6e-9 at 40 000 nodes and 7.3e-10 at 2.1 million (5.5e-9 and 8.5e-10 with FP32 over a thread and
+// a warp and FP64 above, as in the launch-per-pass kernels).  scale is a power of two that brings the sum near 1: a
+// warp's sum lies in FP32's range, the grid's need not.
+constexpr int kFp32Nodes = 16;
+template <int N, int NT>
+__device__ __forceinline__ bool grid_total(const FF (&v)[N], const float (&scale)[N], float2 (*wsum)[NT / 32],
+                                           float2 (*part)[kMostCtas], const GridWait& w, unsigned& target, int* s_fail,
+                                           FF (&out)[N]) {
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const FF x = warp_halved(v);
+#pragma unroll
+    for (int c = 0; c < N; c++)
+        if (lane == warp_home<N>(c)) wsum[c][wp] = make_float2(x.hi * scale[c], x.lo * scale[c]);
     __syncthreads();
     if (wp == 0) {
 #pragma unroll
-        for (int c = 0; c < N; c++) out[c] = FF{lane < NT / 32 ? wsum[c][lane] : 0.f, 0.f};
-        tree();
+        for (int c = 0; c < N; c++) {
+            const float2 t = lane < NT / 32 ? wsum[c][lane] : make_float2(0.f, 0.f);
+            out[c] = FF{t.x, t.y};
+        }
+        warp_total(out);
         if (lane == 0)
 #pragma unroll
             for (int c = 0; c < N; c++) __stcg(&part[c][blockIdx.x], make_float2(out[c].hi, out[c].lo));
@@ -97,15 +127,8 @@ __device__ __forceinline__ bool grid_total(const float (&v)[N], float (*wsum)[NT
 #pragma unroll
                 for (int c = 0; c < N; c++) out[c] = ff_gather(out[c], FF{t[u][c].x, t[u][c].y});
         }
-        tree();
+        warp_total(out);
     }
     return ok;
 }
-__device__ __forceinline__ float ff_ratio(FF a, FF b) {  // a / b rounded to FP32
-    const float q = a.hi / b.hi;
-    const float rem = fmaf(-q, b.hi, a.hi) + (a.lo - q * b.lo);
-    return q + rem / b.hi;
-}
-
-
 }  // namespace pic

@@ -1,5 +1,6 @@
 // Host-side launch wrappers shared between the kernel translation units and the C ABI.
 #pragma once
+#include <cmath>
 #include "pic_common.cuh"
 
 namespace pic {
@@ -203,19 +204,33 @@ struct SolveWork {
     int gstride;
     unsigned* ticket; // last-block counter of the node-kernel reductions
 };
+// Powers of two that bring r.r and r.z, d.q, z.q of an inner solve near 1 (z and e are r over the operator's
+// diagonal): the persistent kernels keep these sums in pairs of FP32, whose range a sum of many nodes can leave
+// where no node's share does.  The exponents are clamped to FP32's, which leaves the sums in range.
+struct SumScales {
+    float rr, rz;
+};
+inline SumScales sum_scales(const GridDev& g, double r2) {
+    if (!(r2 > 0.0) || !std::isfinite(r2)) return {1.f, 1.f};
+    double diag = 0.0;
+    for (int d = 0; d < 3; d++) diag += 2.0 / (g.dxd[d] * g.dxd[d]);
+    const int k = std::ilogb(r2), kd = std::ilogb(diag);
+    auto pow2 = [](int e) { return std::ldexp(1.f, e < -126 ? -126 : (e > 126 ? 126 : e)); };
+    return {pow2(-k), pow2(kd - k)};
+}
 // Inner solvers on one thread-block cluster (pic_cluster.cu): planes per CTA, 0 when the grid does not
 // fit a cluster of at most `most` CTAs
 int plan_sor_cluster(const GridDev& g, int most);
 int plan_pcg_cluster(const GridDev& g, int most);
 // sweeps from e = 0 (with the seam passes); the whole inner CG solve from e = 0, at most cap iterations
-// (flag[0] converged, flag[1] iterations)
+// (flag[0] converged, flag[1] iterations); r2: r.r
 void launch_sor_cluster(const GridDev& g, SolveWork& w, float omega, int sweeps, int planes, cudaStream_t s);
-void launch_pcg_cluster(const GridDev& g, SolveWork& w, double target_rr, int cap, int planes, cudaStream_t s);
+void launch_pcg_cluster(const GridDev& g, SolveWork& w, double r2, double target_rr, int cap, int planes, cudaStream_t s);
 // The same over the whole GPU (pic_persist.cu): nodes per CTA, 0 when the grid does not fit its SMs' shared memory
 int plan_sor_grid(const GridDev& g, int sms);
 int plan_pcg_grid(const GridDev& g, int sms);
 void launch_sor_grid(const GridDev& g, SolveWork& w, float omega, int sweeps, int chunk, cudaStream_t s);
-void launch_pcg_grid(const GridDev& g, SolveWork& w, double target_rr, int cap, int chunk, cudaStream_t s);
+void launch_pcg_grid(const GridDev& g, SolveWork& w, double r2, double target_rr, int cap, int chunk, cudaStream_t s);
 constexpr int kParts = 1024;
 // Node kernels take a tile of kNodeTile consecutive nodes per block, kNodeTile / blockDim.x per
 // thread, strided by blockDim.x so that every load is coalesced and a thread's loads are

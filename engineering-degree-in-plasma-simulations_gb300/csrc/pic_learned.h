@@ -113,10 +113,10 @@ void launch_lpcg_init(const GridDev& g, SolveWork& w, const LpState& L, cudaStre
 void launch_lpcg_iter(const GridDev& g, SolveWork& w, const LpState& L, float* d_in, float* d_out, int it,
                       double target_rr, cudaStream_t s, int sms);
 // the whole inner solve in one launch (pic_lpcg.cu): whether the grid takes it; e from zero, at most cap
-// iterations (w.flag[0] converged, [1] iterations, [2] a wait ran out); d2, r2: node arrays, scratch
+// iterations (w.flag[0] converged, [1] iterations, [2] a wait ran out); d2, r_alt: node arrays, scratch; r2: r.r
 bool plan_lpcg_grid(const GridDev& g, const LpState& L, int sms);
-void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d2, float* r2, double target_rr, int cap,
-                      cudaStream_t s, int sms);
+void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d2, float* r_alt, double r2, double target_rr,
+                      int cap, cudaStream_t s, int sms);
 void launch_lpcg_k1_probe(const GridDev& g, SolveWork& w, float* d_in, float* d_out, cudaStream_t s);
 
 }  // namespace pic

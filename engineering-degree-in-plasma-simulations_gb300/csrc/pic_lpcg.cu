@@ -43,6 +43,7 @@ struct LpcgArgs {
     float *r[2], *d[2], *z, *q, *e;
     const uint16_t* kind;
     const float* S0;
+    SumScales sc;
     FF target;
     int cap, tx_n, ty_n, ntiles, rounds;
     int* flag;
@@ -86,7 +87,10 @@ __device__ __forceinline__ void stage_write(float* T, const Staged& s) {
     }
 }
 
-// flag[0]: converged (r.r <= target), flag[1]: iterations done
+// flag[0]: converged (r.r <= target), flag[1]: iterations done.  LONG: some CTA owns more than kRun tiles, so that
+// a thread's FP32 sums are cut into runs
+constexpr int kRun = kFp32Nodes / 4;  // tiles
+template <bool LONG>
 __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ LpcgArgs a) {
     extern __shared__ __align__(16) float dyn[];
     LevelSmem& sm = *reinterpret_cast<LevelSmem*>(dyn);
@@ -96,10 +100,12 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
     int* tabR = tabS + a.rounds * kRows;                     // restriction rule
     int4* org = reinterpret_cast<int4*>(tabR + a.rounds * kRows);  // origins of the CTA's tiles
     unsigned char* F = reinterpret_cast<unsigned char*>(org + a.rounds);  // node flags: FREE 128, mirrors
-    __shared__ float S[27], dia[64], wsum[2][kThr / 32], s_alpha, s_beta;
+    __shared__ float S[27], dia[64], s_alpha, s_beta;
+    __shared__ float2 wsum[2][kThr / 32], runs[2][LONG ? kThr : 1];
     __shared__ int s_fail, s_stop;
     static_assert(kCTile <= kLvTile, "the tile of e_1 shares the level tile's place");
     const GridDev& g = a.g;
+    const float sc_rr[1] = {a.sc.rr}, sc_dq[1] = {a.sc.rz}, sc_z[2] = {a.sc.rz, a.sc.rz};
     const int tid = threadIdx.x, tx = tid & 31, ty = (tid >> 5) & 7, tz = (tid >> 8) * 4;
     const float c3[3] = {g.inv_dx[0] * g.inv_dx[0], g.inv_dx[1] * g.inv_dx[1], g.inv_dx[2] * g.inv_dx[2]};
     if (tid < 27) S[tid] = a.S0[tid];
@@ -160,13 +166,26 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
     FF dq[1] = {FF{0.f, 0.f}}, rr[1], zz[2], rz{0.f, 0.f};
     int it = 0, rc = 0, dc = 0;  // r[rc], d[dc]: the residual and the last direction
 
+    // The FP32 sum f of a thread's columns of four nodes joins its pair runs[c] every kFp32Nodes nodes; whole_run is the
+    // pair at the end.  In shared memory: pairs in registers cost 3 us an iteration of a million nodes in spills.
+    auto run = [&](int round, int c, float& f) {
+        if (!LONG || (round + 1) % kRun || round + 1 >= mine) return;
+        const float2 p = round + 1 == kRun ? make_float2(0.f, 0.f) : runs[c][tid];
+        const FF s = ff_acc(FF{p.x, p.y}, f);
+        runs[c][tid] = make_float2(s.hi, s.lo);
+        f = 0.f;
+    };
+    auto whole_run = [&](int c, float f) {
+        const float2 p = LONG && mine > kRun ? runs[c][tid] : make_float2(0.f, 0.f);
+        return ff_acc(FF{p.x, p.y}, f);
+    };
     // r -= alpha q (into r[rc ^ 1]), e += alpha d, r.r, z_1 = R r; the first time only z_1 of r[0]
     auto update = [&](bool first) {
         const float alpha = s_alpha;
         const float* r = a.r[rc];
         const float* d = a.d[dc];
         float* rn = a.r[rc ^ 1];
-        float acc[1] = {0.f};
+        float f = 0.f;
         Staged s;
         float ev[4], dv[4];
         auto read = [&](int round) {
@@ -199,10 +218,11 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
                 for (int k = 0; k < 4; k++) {
                     if (!inside(t, k)) continue;
                     const float v = Tb[((tz + k + 1) * kHY + ty + 1) * kP + tx + 1];
-                    acc[0] += v * v;
+                    f += v * v;
                     rn[node(t, k)] = v;
                     a.e[node(t, k)] = en[k];
                 }
+                run(round, 0, f);
             }
             // 16 x 4 x 4 coarse voxels, two threads each (two of the four fine planes)
             const int v = tid >> 1, i = v & 15, j = (v >> 4) & 3, k = v >> 6, h = tid & 1;
@@ -223,7 +243,8 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
             const int cx = (t.x0 >> 1) + i, cy = (t.y0 >> 1) + j, cz = (t.z0 >> 1) + k;
             if (h == 0 && cx < a.z1.n[0] && cy < a.z1.n[1] && cz < a.z1.n[2]) a.z1.a[lv_off(a.z1, cx, cy, cz)] = sum;
         }
-        return grid_total<1, kThr>(acc, wsum, a.sync->part + 1, a.wait, target, &s_fail, rr);
+        const FF acc[1] = {whole_run(0, f)};
+        return grid_total<1, kThr>(acc, sc_rr, wsum, a.sync->part + 1, a.wait, target, &s_fail, rr);
     };
 
     bool ok = grid_barrier(a.wait, target, &s_fail);  // the zeros are there
@@ -241,7 +262,7 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
         if (!(ok = grid_barrier(a.wait, target, &s_fail))) break;
         {
             const float* r = a.r[rc];
-            float acc[2] = {0.f, 0.f}, w[27];
+            float w[27], f[2] = {0.f, 0.f};
 #pragma unroll
             for (int m = 0; m < 27; m++) w[m] = S[m];
             Staged s;
@@ -304,14 +325,17 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
                         const int lz = 1 + (k >> 1), sz = (k & 1) ? 1 : -1;
                         const float v = Pr + a2 + (0.75f * px[lz] + 0.25f * px[lz + sz]);
                         a.z[node(t, k)] = v;
-                        acc[0] += v * Tb[((tz + k + 1) * kHY + ty + 1) * kP + tx + 1];
-                        acc[1] += v * q0[k];
+                        f[0] += v * Tb[((tz + k + 1) * kHY + ty + 1) * kP + tx + 1];
+                        f[1] += v * q0[k];
                     }
                     Pr = Qr + a1;
                     Qr = a0;
                 }
+                run(round, 0, f[0]);
+                run(round, 1, f[1]);
             }
-            ok = grid_total<2, kThr>(acc, wsum, a.sync->part + 2, a.wait, target, &s_fail, zz);  // z.r, z.q
+            const FF acc[2] = {whole_run(0, f[0]), whole_run(1, f[1])};
+            ok = grid_total<2, kThr>(acc, sc_z, wsum, a.sync->part + 2, a.wait, target, &s_fail, zz);  // z.r, z.q
         }
         if (tid == 0) s_beta = it > 0 && dq[0].hi != 0.f ? -ff_ratio(zz[1], dq[0]) : 0.f;
         rz = zz[0];
@@ -322,7 +346,7 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
             const float beta = s_beta;
             const float* d = a.d[dc];
             float* dn = a.d[dc ^ 1];
-            float acc[1] = {0.f};
+            float f = 0.f;
             Staged s;
             auto read = [&](int round) {
                 const int x0 = at(round).x0;
@@ -352,12 +376,14 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
                     off += c3[2] * c[k];
                     off += c3[2] * c[k + 2];
                     const float qn = dia[fl & 63u] * c[k + 1] - off;
-                    acc[0] += c[k + 1] * qn;
+                    f += c[k + 1] * qn;
                     dn[node(t, k)] = c[k + 1];
                     a.q[node(t, k)] = qn;
                 }
+                run(round, 0, f);
             }
-            ok = grid_total<1, kThr>(acc, wsum, a.sync->part, a.wait, target, &s_fail, dq);
+            const FF acc[1] = {whole_run(0, f)};
+            ok = grid_total<1, kThr>(acc, sc_dq, wsum, a.sync->part, a.wait, target, &s_fail, dq);
         }
         if (tid == 0) s_alpha = dq[0].hi != 0.f ? ff_ratio(rz, dq[0]) : 0.f;
         __syncthreads();
@@ -387,6 +413,8 @@ __global__ void __launch_bounds__(kThr, 1) k_lpcg_grid(const __grid_constant__ L
 size_t lpcg_bytes(int rounds) {
     return sizeof(LevelSmem) + sizeof(float) * 2 * kRows * kP + (size_t)rounds * (2 * sizeof(int) * kRows + sizeof(int4) + kTile);
 }
+using LpcgKernel = void (*)(LpcgArgs);
+LpcgKernel lpcg_kernel(int rounds) { return rounds > kRun ? (LpcgKernel)k_lpcg_grid<true> : (LpcgKernel)k_lpcg_grid<false>; }
 int tiles_of(const LpState& L, int* tx, int* ty) {
     *tx = (L.dims[0][0] + kTX - 1) / kTX;
     *ty = (L.dims[0][1] + kTY - 1) / kTY;
@@ -399,16 +427,17 @@ bool plan_lpcg_grid(const GridDev& g, const LpState& L, int sms) {
     const int nt = tiles_of(L, &tx, &ty), rounds = (nt + sms - 1) / std::max(1, sms);
     if (L.nlev < 2 || g.nv > kLpcgMostNodes || sms < 1 || sms > kMostCtas || rounds > kMostRounds) return false;
     int n = 0;
-    const bool ok = cudaFuncSetAttribute(k_lpcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const auto kernel = lpcg_kernel(rounds);
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)lpcg_bytes(kMostRounds)) == cudaSuccess &&
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_lpcg_grid, kThr, lpcg_bytes(rounds)) == cudaSuccess &&
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThr, lpcg_bytes(rounds)) == cudaSuccess &&
                     n > 0;
     if (!ok) cudaGetLastError();
     return ok;
 }
 
-void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d2, float* r2, double target_rr, int cap,
-                      cudaStream_t s, int sms) {
+void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d2, float* r_alt, double r2, double target_rr,
+                      int cap, cudaStream_t s, int sms) {
     LpcgArgs a;
     a.g = g;
     a.f = lp_node_view(g, L, nullptr);
@@ -419,7 +448,7 @@ void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d
     lp_coarse_setup(L, L.dense_level == 1 ? 1 : 2, a.z1, a.lev);
     a.lev.fold[1] = L.fold;
     a.r[0] = w.r;
-    a.r[1] = r2;
+    a.r[1] = r_alt;
     a.d[0] = w.d;
     a.d[1] = d2;
     a.z = w.z;
@@ -427,7 +456,8 @@ void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d
     a.e = w.e;
     a.kind = reinterpret_cast<const uint16_t*>(w.kind);
     a.S0 = L.W + L.lay.s0;
-    a.target = ff_from_double(target_rr);
+    a.sc = sum_scales(g, r2);
+    a.target = ff_from_double(target_rr * a.sc.rr);
     a.cap = cap;
     a.ntiles = tiles_of(L, &a.tx_n, &a.ty_n);
     a.rounds = (a.ntiles + sms - 1) / sms;
@@ -436,7 +466,7 @@ void launch_lpcg_grid(const GridDev& g, SolveWork& w, const LpState& L, float* d
     a.wait = GridWait{&a.sync->arrived, w.wait_polls, w.err, w.flag + 2};
     cudaMemsetAsync(a.sync, 0, sizeof(unsigned), s);
     void* args[] = {&a};
-    cudaLaunchCooperativeKernel((const void*)k_lpcg_grid, dim3((unsigned)sms), dim3(kThr), args,
+    cudaLaunchCooperativeKernel((const void*)lpcg_kernel(a.rounds), dim3((unsigned)sms), dim3(kThr), args,
                                 lpcg_bytes(a.rounds), s);
 }
 }  // namespace pic

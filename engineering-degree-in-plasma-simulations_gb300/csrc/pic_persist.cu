@@ -157,16 +157,20 @@ __global__ void __launch_bounds__(kThr, 1) k_sor_grid(GridDev g, float* __restri
 constexpr unsigned long long kPlain4 = 0x0001000100010001ull, kWrap4 = 0x1F801F801F801F80ull;
 template <int K>
 __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __restrict__ e, const float* __restrict__ r,
-                                                      float* dg, const uint16_t* __restrict__ kind, FF target_rr,
-                                                      int cap, int chunk, int* flag, GridSync* sync,
+                                                      float* dg, const uint16_t* __restrict__ kind, SumScales sc,
+                                                      FF target_rr, int cap, int chunk, int* flag, GridSync* sync,
                                                       GridWait wait) {
+    const float sc1[1] = {sc.rz}, sc3[3] = {sc.rz, sc.rz, sc.rr};
+    constexpr int kRun = kFp32Nodes / 4;  // groups that a thread adds in FP32
+    static_assert(K <= 2 * kRun, "two such sums at most");
     extern __shared__ __align__(16) float sm[];
     float4* D4 = reinterpret_cast<float4*>(sm);
     float4* R4 = D4 + chunk / 4;
     float4* X4 = R4 + chunk / 4;
     unsigned long long* M4 = reinterpret_cast<unsigned long long*>(X4 + chunk / 4);  // four 16-bit flag words
     float* D = sm;
-    __shared__ float dia[64], inv[64], wsum[3][kPcgThr / 32], s_alpha, s_beta;
+    __shared__ float dia[64], inv[64], s_alpha, s_beta;
+    __shared__ float2 wsum[3][kPcgThr / 32];
     __shared__ int s_fail, s_stop;  // s_stop: 1 converged, 3 not a number
     const int tid = threadIdx.x, n0 = blockIdx.x * chunk, len = min(chunk, g.nv - n0);
     const int ng = chunk / 4, nij = g.ni * g.nj;
@@ -180,19 +184,20 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
     }
     __syncthreads();
     float* G = dg + n0;
-    float f3[3] = {0.f, 0.f, 0.f};
+    FF f3[3] = {FF{0.f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}};
     for (int q = tid; q < ng; q += kPcgThr) {
-        float rv[4];
+        float rv[4], f = 0.f;
         unsigned long long mm = 0;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             const int x = 4 * q + c;
-            const unsigned f = x < len ? node_flags(g, n0 + x, kind[n0 + x]) : 0u;
-            rv[c] = f ? r[n0 + x] : 0.f;
+            const unsigned fl = x < len ? node_flags(g, n0 + x, kind[n0 + x]) : 0u;
+            rv[c] = fl ? r[n0 + x] : 0.f;
             if (x < len) G[x] = 0.f;
-            mm |= (unsigned long long)f << (16 * c);
-            f3[0] += rv[c] * (rv[c] * inv[(f >> 1) & 63u]);
+            mm |= (unsigned long long)fl << (16 * c);
+            f += rv[c] * (rv[c] * inv[(fl >> 1) & 63u]);
         }
+        f3[0] = ff_acc(f3[0], f);
         D4[q] = X4[q] = make_float4(0.f, 0.f, 0.f, 0.f);
         R4[q] = make_float4(rv[0], rv[1], rv[2], rv[3]);
         M4[q] = mm;
@@ -201,7 +206,7 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
     float2(*part3)[kMostCtas] = sync->part + 1;
     unsigned target = 0;
     FF t1[1], t3[3];
-    grid_total<3, kPcgThr>(f3, wsum, part3, wait, target, &s_fail, t3);  // r.z
+    grid_total<3, kPcgThr>(f3, sc3, wsum, part3, wait, target, &s_fail, t3);  // r.z
     FF rz = t3[0];
     const float inv0 = inv[0], dia0 = dia[0];
     __syncthreads();
@@ -238,12 +243,17 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
         }
         if (!grid_barrier(wait, target, &s_fail)) break;
         // q = L d, d.q
-        float v1[1] = {0.f};
+        FF v1[1] = {FF{0.f, 0.f}};
+        float f1 = 0.f;
 #pragma unroll
         for (int m = 0; m < K; m++) {
             const int q = tid + m * kPcgThr;
             Q[m][0] = Q[m][1] = Q[m][2] = Q[m][3] = 0.f;
             if (q >= ng) break;
+            if (m == kRun) {
+                v1[0].hi = f1;
+                f1 = 0.f;
+            }
             const unsigned long long mm = M4[q];
             if (!mm) continue;
             const int l = 4 * q;
@@ -300,20 +310,28 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
                 for (int d = 0; d < 6; d++) off += c3[d >> 1] * nb[c][d];
                 const float di = mm == kPlain4 ? dia0 : dia[(f >> 1) & 63u];
                 Q[m][c] = f ? di * dv[c] - off : 0.f;
-                v1[0] += dv[c] * Q[m][c];
+                f1 += dv[c] * Q[m][c];
             }
         }
-        grid_total<1, kPcgThr>(v1, wsum, part1, wait, target, &s_fail, t1);
+        v1[0] = ff_acc(v1[0], f1);
+        grid_total<1, kPcgThr>(v1, sc1, wsum, part1, wait, target, &s_fail, t1);
         if (tid == 0) s_alpha = t1[0].hi != 0.f ? ff_ratio(rz, t1[0]) : 0.f;
         __syncthreads();
         if (s_fail) break;
         // e += alpha d, r -= alpha q, z = r / diagonal
         const float alpha = s_alpha;
-        float v3[3] = {0.f, 0.f, 0.f};
+        FF v3[3] = {FF{0.f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}};
+        float f[3] = {0.f, 0.f, 0.f};
 #pragma unroll
         for (int m = 0; m < K; m++) {
             const int q = tid + m * kPcgThr;
             if (q >= ng) break;
+            if (m == kRun)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    v3[c].hi = f[c];
+                    f[c] = 0.f;
+                }
             const unsigned long long mm = M4[q];
             if (!mm) continue;
             const float4 d4 = D4[q], x4 = X4[q], r4 = R4[q];
@@ -324,14 +342,16 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
                 const float iv = mm == kPlain4 ? inv0 : inv[(unsigned)(mm >> (16 * c + 1)) & 63u];
                 xv[c] += alpha * dv[c];
                 rn[c] = rv[c] - alpha * Q[m][c];
-                v3[0] += rn[c] * (rn[c] * iv);
-                v3[1] += rn[c] * (rv[c] * iv);
-                v3[2] += rn[c] * rn[c];
+                f[0] += rn[c] * (rn[c] * iv);
+                f[1] += rn[c] * (rv[c] * iv);
+                f[2] += rn[c] * rn[c];
             }
             X4[q] = make_float4(xv[0], xv[1], xv[2], xv[3]);
             R4[q] = make_float4(rn[0], rn[1], rn[2], rn[3]);
         }
-        grid_total<3, kPcgThr>(v3, wsum, part3, wait, target, &s_fail, t3);
+#pragma unroll
+        for (int c = 0; c < 3; c++) v3[c] = ff_acc(v3[c], f[c]);
+        grid_total<3, kPcgThr>(v3, sc3, wsum, part3, wait, target, &s_fail, t3);
         it++;
         if (tid == 0) {
             const float over = (t3[2].hi - target_rr.hi) + (t3[2].lo - target_rr.lo);
@@ -359,7 +379,7 @@ __global__ void __launch_bounds__(kPcgThr, 1) k_pcg_grid(GridDev g, float* __res
 int chunk_of(const GridDev& g, int sms) { return ((g.nv + sms - 1) / sms + 31) / 32 * 32; }
 size_t sor_bytes(int chunk) { return 12 * (size_t)chunk; }
 size_t pcg_bytes(int chunk) { return 14 * (size_t)chunk; }
-using PcgKernel = void (*)(GridDev, float*, const float*, float*, const uint16_t*, FF, int, int, int*, GridSync*,
+using PcgKernel = void (*)(GridDev, float*, const float*, float*, const uint16_t*, SumScales, FF, int, int, int*, GridSync*,
                            GridWait);
 PcgKernel pcg_kernel(int chunk) {
     if (chunk <= 4 * kPcgThr) return k_pcg_grid<1>;
@@ -400,7 +420,7 @@ void launch_sor_grid(const GridDev& g, SolveWork& w, float omega, int sweeps, in
     cudaLaunchCooperativeKernel((const void*)k_sor_grid, dim3((g.nv + chunk - 1) / chunk), dim3(kThr), args,
                                 sor_bytes(chunk), s);
 }
-void launch_pcg_grid(const GridDev& g, SolveWork& w, double target_rr, int cap, int chunk, cudaStream_t s) {
+void launch_pcg_grid(const GridDev& g, SolveWork& w, double r2, double target_rr, int cap, int chunk, cudaStream_t s) {
     const uint16_t* kd = reinterpret_cast<const uint16_t*>(w.kind);
     const float* r = w.r;
     GridDev gg = g;
@@ -409,8 +429,9 @@ void launch_pcg_grid(const GridDev& g, SolveWork& w, double target_rr, int cap, 
     GridSync* sync = reinterpret_cast<GridSync*>(w.gpart);
     GridWait gw{&sync->arrived, w.wait_polls, w.err, w.flag + 2};
     cudaMemsetAsync(sync, 0, sizeof(unsigned), s);
-    FF t = ff_from_double(target_rr);
-    void* args[] = {&gg, &w.e, &r, &w.d, &kd, &t, &cap, &chunk, &w.flag, &sync, &gw};
+    SumScales sc = sum_scales(g, r2);
+    FF t = ff_from_double(target_rr * sc.rr);
+    void* args[] = {&gg, &w.e, &r, &w.d, &kd, &sc, &t, &cap, &chunk, &w.flag, &sync, &gw};
     cudaLaunchCooperativeKernel((const void*)pcg_kernel(chunk), dim3((g.nv + chunk - 1) / chunk), dim3(kPcgThr), args,
                                 pcg_bytes(chunk), s);
 }
