@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(256) k_rhs_update(GridDev g, float* __restrict
                                                     const uint16_t* __restrict__ kind, double* gpart, int gstride,
                                                     unsigned* ticket, double* out) {
     const float inv_eps0_f = (float)(1.0 / kEps0);
-    float acc_r = 0.f, acc_b = 0.f, acc_t = 0.f, acc_s = 0.f;
+    FF acc[4] = {FF{0.f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}};  // pairs over the groups of four nodes
     const int ng = g.nv >> 2;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ng; q += gridDim.x * blockDim.x) {
         const float4 r4 = reinterpret_cast<const float4*>(r)[q];
@@ -524,6 +524,7 @@ __global__ void __launch_bounds__(256) k_rhs_update(GridDev g, float* __restrict
         float rv[4] = {r4.x, r4.y, r4.z, r4.w}, hv[4] = {h4.x, h4.y, h4.z, h4.w};
         const float pv[4] = {p4.x, p4.y, p4.z, p4.w}, fv[4] = {f4.x, f4.y, f4.z, f4.w};
         const unsigned short kv[4] = {k4.x, k4.y, k4.z, k4.w};
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             if ((kv[c] & 3) != kFree) continue;
@@ -531,11 +532,13 @@ __global__ void __launch_bounds__(256) k_rhs_update(GridDev g, float* __restrict
             rv[c] += t;
             const float sc = hv[c] * inv_eps0_f;
             const float b = sc + fv[c];
-            acc_r += rv[c] * rv[c];
-            acc_b += b * b;
-            acc_t += t * t;
-            acc_s += sc * sc;
+            f[0] += rv[c] * rv[c];
+            f[1] += b * b;
+            f[2] += t * t;
+            f[3] += sc * sc;
         }
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[c] = ff_acc(acc[c], f[c]);
         reinterpret_cast<float4*>(r)[q] = make_float4(rv[0], rv[1], rv[2], rv[3]);
         reinterpret_cast<float4*>(rho_prev)[q] = h4;
     }
@@ -549,15 +552,14 @@ __global__ void __launch_bounds__(256) k_rhs_update(GridDev g, float* __restrict
             r[n] = rn;
             const float sc = rh * inv_eps0_f;
             const float b = sc + bfix[n];
-            acc_r += rn * rn;
-            acc_b += b * b;
-            acc_t += t * t;
-            acc_s += sc * sc;
+            acc[0] = ff_acc(acc[0], rn * rn);
+            acc[1] = ff_acc(acc[1], b * b);
+            acc[2] = ff_acc(acc[2], t * t);
+            acc[3] = ff_acc(acc[3], sc * sc);
         }
         rho_prev[n] = rho[n];
     }
-    const float v[4] = {acc_r, acc_b, acc_t, acc_s};
-    grid_sum<4>(v, gpart, gstride, ticket, out);
+    grid_sum<4>(acc, gpart, gstride, ticket, out);
 }
 void launch_rhs_update(const GridDev& g, SolveWork& w, float* rho_prev, const float* bfix, cudaStream_t s) {
     k_rhs_update<<<stream_blocks(g, kResPerSM), 256, 0, s>>>(g, w.r, w.rho, rho_prev, bfix,
@@ -665,7 +667,7 @@ __global__ void __launch_bounds__(256) k_pcg_init(GridDev g, const float* __rest
                                                   unsigned* ticket, double* scal, int* flag) {
     if (blockIdx.x == 0 && threadIdx.x == 0) flag[0] = 0;
     const float c3[3] = {g.inv_dx[0] * g.inv_dx[0], g.inv_dx[1] * g.inv_dx[1], g.inv_dx[2] * g.inv_dx[2]};
-    float acc = 0.f;
+    FF acc[1] = {FF{0.f, 0.f}};
     const int ng = g.nv >> 2;
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ng; q += gridDim.x * blockDim.x) {
@@ -673,12 +675,13 @@ __global__ void __launch_bounds__(256) k_pcg_init(GridDev g, const float* __rest
         const ushort4 k4 = reinterpret_cast<const ushort4*>(kind)[q];
         const float rv[4] = {r4.x, r4.y, r4.z, r4.w};
         const unsigned short kv[4] = {k4.x, k4.y, k4.z, k4.w};
-        float zv[4];
+        float zv[4], f = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             zv[c] = (kv[c] & 3) == kFree ? rv[c] * inv_diag_of(kv[c], c3) : 0.f;
-            acc += rv[c] * zv[c];
+            f += rv[c] * zv[c];
         }
+        acc[0] = ff_acc(acc[0], f);
         reinterpret_cast<float4*>(z)[q] = make_float4(zv[0], zv[1], zv[2], zv[3]);
         reinterpret_cast<float4*>(e)[q] = zero4;
         reinterpret_cast<float4*>(d)[q] = zero4;
@@ -690,12 +693,11 @@ __global__ void __launch_bounds__(256) k_pcg_init(GridDev g, const float* __rest
         z[n] = zz;
         e[n] = 0.f;
         d[n] = 0.f;
-        acc += r[n] * zz;
+        acc[0] = ff_acc(acc[0], r[n] * zz);
     }
-    const float v[1] = {acc};
-    grid_sum<1>(v, gpart, gstride, ticket, scal + kS_RZN);  // r.z
+    grid_sum<1>(acc, gpart, gstride, ticket, scal + kS_RZN);  // r.z
 }
-__global__ void __launch_bounds__(256) k_pcg_k1(GridDev g, const float* __restrict__ z,
+__global__ void __launch_bounds__(256, kPcgPerSM) k_pcg_k1(GridDev g, const float* __restrict__ z,
                                                          const float* __restrict__ d_in, float* __restrict__ d_out,
                                                          float* __restrict__ q, const uint16_t* __restrict__ kind,
                                                          double* gpart, int gstride, unsigned* ticket, double* scal,
@@ -726,14 +728,16 @@ __global__ void __launch_bounds__(256) k_pcg_k1(GridDev g, const float* __restri
     __syncthreads();
     if (s_stop) return;
     const float fb = s_beta;
-    float facc = 0.f;
+    FF acc[1] = {FF{0.f, 0.f}};
     const int ngroups = (g.nv + 3) >> 2;
-    for (int qg = blockIdx.x * blockDim.x + threadIdx.x; qg < ngroups; qg += gridDim.x * blockDim.x)
-        spmv_group(g, qg << 2, z, d_in, d_out, q, kind, fb, facc);
-    const float v[1] = {facc};
-    grid_sum<1>(v, gpart, gstride, ticket, scal + kS_DQ);
+    for (int qg = blockIdx.x * blockDim.x + threadIdx.x; qg < ngroups; qg += gridDim.x * blockDim.x) {
+        float f = 0.f;
+        spmv_group(g, qg << 2, z, d_in, d_out, q, kind, fb, f);
+        acc[0] = ff_acc(acc[0], f);
+    }
+    grid_sum<1>(acc, gpart, gstride, ticket, scal + kS_DQ);
 }
-__global__ void __launch_bounds__(256) k_pcg_k2(GridDev g, const float* __restrict__ d, const float* __restrict__ q,
+__global__ void __launch_bounds__(256, kPcgPerSM) k_pcg_k2(GridDev g, const float* __restrict__ d, const float* __restrict__ q,
                                                 float* __restrict__ e, float* __restrict__ r, float* __restrict__ z,
                                                 const uint16_t* __restrict__ kind, double* gpart, int gstride,
                                                 unsigned* ticket, double* scal, int* flag, int it) {
@@ -746,7 +750,7 @@ __global__ void __launch_bounds__(256) k_pcg_k2(GridDev g, const float* __restri
     __syncthreads();
     const float alpha = s_alpha;
     const float c3[3] = {g.inv_dx[0] * g.inv_dx[0], g.inv_dx[1] * g.inv_dx[1], g.inv_dx[2] * g.inv_dx[2]};
-    float f0 = 0.f, f1 = 0.f, f2 = 0.f;
+    FF acc[3] = {FF{0.f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}};
     const int ng = g.nv >> 2;
     for (int qq = blockIdx.x * blockDim.x + threadIdx.x; qq < ng; qq += gridDim.x * blockDim.x) {
         const float4 d4 = reinterpret_cast<const float4*>(d)[qq];
@@ -758,18 +762,21 @@ __global__ void __launch_bounds__(256) k_pcg_k2(GridDev g, const float* __restri
         const float dv[4] = {d4.x, d4.y, d4.z, d4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
         float ev[4] = {e4.x, e4.y, e4.z, e4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w}, zv[4] = {z4.x, z4.y, z4.z, z4.w};
         const unsigned short kv[4] = {k4.x, k4.y, k4.z, k4.w};
+        float f[3] = {0.f, 0.f, 0.f};
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             if ((kv[c] & 3) != kFree) continue;
             ev[c] += alpha * dv[c];
             const float rn = rv[c] - alpha * qv[c];
             const float zn = rn * inv_diag_of(kv[c], c3);
-            f0 += rn * zn;
-            f1 += rn * zv[c];
-            f2 += rn * rn;
+            f[0] += rn * zn;
+            f[1] += rn * zv[c];
+            f[2] += rn * rn;
             rv[c] = rn;
             zv[c] = zn;
         }
+#pragma unroll
+        for (int c = 0; c < 3; c++) acc[c] = ff_acc(acc[c], f[c]);
         reinterpret_cast<float4*>(e)[qq] = make_float4(ev[0], ev[1], ev[2], ev[3]);
         reinterpret_cast<float4*>(r)[qq] = make_float4(rv[0], rv[1], rv[2], rv[3]);
         reinterpret_cast<float4*>(z)[qq] = make_float4(zv[0], zv[1], zv[2], zv[3]);
@@ -781,15 +788,14 @@ __global__ void __launch_bounds__(256) k_pcg_k2(GridDev g, const float* __restri
             e[n] += alpha * d[n];
             const float rn = r[n] - alpha * q[n];
             const float zn = rn * inv_diag_of(kd, c3);
-            f0 += rn * zn;
-            f1 += rn * z[n];
-            f2 += rn * rn;
+            acc[0] = ff_acc(acc[0], rn * zn);
+            acc[1] = ff_acc(acc[1], rn * z[n]);
+            acc[2] = ff_acc(acc[2], rn * rn);
             r[n] = rn;
             z[n] = zn;
         }
     }
-    const float v[3] = {f0, f1, f2};
-    grid_sum<3>(v, gpart, gstride, ticket, scal + kS_RZN);  // r.z', r.z, r.r
+    grid_sum<3>(acc, gpart, gstride, ticket, scal + kS_RZN);  // r.z', r.z, r.r
 }
 void launch_pcg_init(const GridDev& g, SolveWork& w, cudaStream_t s) {
     k_pcg_init<<<stream_blocks(g, kPcgPerSM), 256, 0, s>>>(g, w.r, w.z, w.e, w.d,

@@ -243,6 +243,9 @@ inline int node_blocks(int nv) { return (nv + kNodeTile - 1) / kNodeTile; }
 // CTAs of a kernel that fits three an SM, 2.7 waves, the last wave leaves a third of the SMs idle: 12 learned
 // iterations of 256 x 256 x 512 nodes 7.90 ms, one wave 7.67 (304 CTAs 8.23, 532 8.46); of 32 x 32 x 2048
 // 1.53 -> 1.43; 300 Jacobi-PCG iterations of 144^3, five an SM, 12.5 -> 9.6 ms (456 CTAs 10.2, 912 13.0).
+// A thread has more nodes than with 1216 CTAs, so the CG kernels sum in pairs of FP32 over its groups of four and
+// its warp: a sum of |r|^2 over 33 M nodes is off FP64 by 1e-9 (FP32 over a thread and a warp: 1.3e-8 with 456
+// CTAs, 4e-9 with 1216); 300 Jacobi-PCG iterations of 144^3 9.9 -> 10.5 ms, of 256^3 49 -> 46.
 constexpr int kSms = 152;
 constexpr int kResPerSM = 3;  // residual and learned-CG kernels (80 registers; the others' sums stay short)
 constexpr int kPcgPerSM = 5;  // Jacobi-PCG kernels (48 registers)

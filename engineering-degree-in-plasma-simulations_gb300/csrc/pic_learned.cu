@@ -1607,7 +1607,7 @@ __global__ void __launch_bounds__(256, kResPerSM) k_lpcg_k1(GridDev g, const flo
     }
     __syncthreads();
     if (s_stop) return;
-    float facc = 0.f;
+    FF acc[1] = {FF{0.f, 0.f}};
     const float fb = s_beta;
     if ((g.ni & 3) == 0) {
         // pairs of rows (j0 even, j0 + 1) of a plane; an odd last row, or a pair across the seam
@@ -1620,20 +1620,24 @@ __global__ void __launch_bounds__(256, kResPerSM) k_lpcg_k1(GridDev g, const flo
             const int i0 = 4 * gx;
             const int n0 = (k * g.nj + j0) * g.ni + i0;
             const bool pair = j0 + 1 < g.nj && (g.periodic[1] ? wrap_p(j0, g.nj, 1) : j0 + 1) == j0 + 1;
+            float f = 0.f;
             if (pair) {
-                cg_pair(g, i0, j0, k, z, d_in, d_out, q, kind, fb, facc);
+                cg_pair(g, i0, j0, k, z, d_in, d_out, q, kind, fb, f);
             } else {
-                spmv_group(g, n0, z, d_in, d_out, q, kind, fb, facc);
-                if (j0 + 1 < g.nj) spmv_group(g, n0 + g.ni, z, d_in, d_out, q, kind, fb, facc);
+                spmv_group(g, n0, z, d_in, d_out, q, kind, fb, f);
+                if (j0 + 1 < g.nj) spmv_group(g, n0 + g.ni, z, d_in, d_out, q, kind, fb, f);
             }
+            acc[0] = ff_acc(acc[0], f);
         }
     } else {
         const int ngroups = (g.nv + 3) >> 2;
-        for (int qg = blockIdx.x * blockDim.x + threadIdx.x; qg < ngroups; qg += gridDim.x * blockDim.x)
-            spmv_group(g, qg << 2, z, d_in, d_out, q, kind, fb, facc);
+        for (int qg = blockIdx.x * blockDim.x + threadIdx.x; qg < ngroups; qg += gridDim.x * blockDim.x) {
+            float f = 0.f;
+            spmv_group(g, qg << 2, z, d_in, d_out, q, kind, fb, f);
+            acc[0] = ff_acc(acc[0], f);
+        }
     }
-    const float v[1] = {facc};
-    grid_sum<1>(v, gpart, gstride, ticket, scal + kS_DQ);
+    grid_sum<1>(acc, gpart, gstride, ticket, scal + kS_DQ);
 }
 __global__ void __launch_bounds__(256) k_lpcg_k2(GridDev g, const float* __restrict__ d, const float* __restrict__ q,
                                                  float* __restrict__ e, float* __restrict__ r,
@@ -1649,7 +1653,7 @@ __global__ void __launch_bounds__(256) k_lpcg_k2(GridDev g, const float* __restr
     }
     __syncthreads();
     const float alpha = s_alpha;
-    float frr = 0.f;
+    FF acc[1] = {FF{0.f, 0.f}};
     const int ng = g.nv >> 2;
     for (int qq = blockIdx.x * blockDim.x + threadIdx.x; qq < ng; qq += gridDim.x * blockDim.x) {
         const float4 d4 = reinterpret_cast<const float4*>(d)[qq];
@@ -1657,15 +1661,16 @@ __global__ void __launch_bounds__(256) k_lpcg_k2(GridDev g, const float* __restr
         const float4 e4 = reinterpret_cast<const float4*>(e)[qq];
         const float4 r4 = reinterpret_cast<const float4*>(r)[qq];
         const float dv[4] = {d4.x, d4.y, d4.z, d4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
-        float ev[4] = {e4.x, e4.y, e4.z, e4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
+        float ev[4] = {e4.x, e4.y, e4.z, e4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w}, f = 0.f;
         // no kind read: d and q are zero on non-FREE nodes (k_lpcg_k1 writes them so) and so is r,
         // which leaves e and r unchanged there
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             ev[c] += alpha * dv[c];
             rv[c] -= alpha * qv[c];
-            frr += rv[c] * rv[c];
+            f += rv[c] * rv[c];
         }
+        acc[0] = ff_acc(acc[0], f);
         reinterpret_cast<float4*>(e)[qq] = make_float4(ev[0], ev[1], ev[2], ev[3]);
         reinterpret_cast<float4*>(r)[qq] = make_float4(rv[0], rv[1], rv[2], rv[3]);
     }
@@ -1674,10 +1679,9 @@ __global__ void __launch_bounds__(256) k_lpcg_k2(GridDev g, const float* __restr
         e[n] += alpha * d[n];
         const float rn = r[n] - alpha * q[n];
         r[n] = rn;
-        frr += rn * rn;
+        acc[0] = ff_acc(acc[0], rn * rn);
     }
-    const float v[1] = {frr};
-    grid_sum<1>(v, gpart, gstride, ticket, scal + kS_RR);
+    grid_sum<1>(acc, gpart, gstride, ticket, scal + kS_RR);
 }
 // |a|^2 over n values into out[0] (deterministic: block partials, then one fixed-order sum)
 __global__ void k_lp_sq(const float* __restrict__ a, int n, double* part) {

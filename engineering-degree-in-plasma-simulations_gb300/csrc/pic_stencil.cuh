@@ -1,6 +1,7 @@
 // Node-index decoding, the 7-point stencil of the reduced Poisson system, and deterministic
 // block reductions, shared by the field kernels and the learned-preconditioner kernels.
 #pragma once
+#include "pic_ff.cuh"
 #include "pic_kernels.h"
 
 namespace pic {
@@ -85,23 +86,34 @@ __device__ __forceinline__ float diag_of(uint16_t kd, const Stencil& s) {
 
 namespace pic {
 
-// Deterministic grid-wide sums of N per-thread FP32 values: every block writes its FP64
+// one warp's sum in lane 0: FP32 (FP64 would occupy the narrow FP64 pipe with every thread of the grid), or pairs
+// of FP32 where a thread has summed many nodes
+__device__ __forceinline__ float warp_sum(float x) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    return x;
+}
+__device__ __forceinline__ FF warp_sum(FF x) {
+    for (int o = 16; o > 0; o >>= 1)
+        x = ff_gather(x, FF{__shfl_down_sync(0xffffffffu, x.hi, o), __shfl_down_sync(0xffffffffu, x.lo, o)});
+    return x;
+}
+__device__ __forceinline__ double wide(float x) { return (double)x; }
+__device__ __forceinline__ double wide(FF x) { return (double)x.hi + (double)x.lo; }
+// Deterministic grid-wide sums of N per-thread FP32 values or pairs: every block writes its FP64
 // partial sums to part[c * stride + block]; the last block to finish (an atomic ticket) adds the
 // partials in block order and writes out[c].  The order of the additions never depends on
 // timing, so the sums are bit-reproducible from run to run.
-template <int N>
-__device__ __forceinline__ void grid_sum(const float (&v)[N], double* part, int stride, unsigned* ticket,
+template <int N, class T>
+__device__ __forceinline__ void grid_sum(const T (&v)[N], double* part, int stride, unsigned* ticket,
                                          double* out) {
     __shared__ double s[N][32];
     __shared__ unsigned s_last;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // warp sums in FP32 (FP64 would occupy the narrow FP64 pipe with every thread of the grid),
     // block and grid sums in FP64
 #pragma unroll
     for (int c = 0; c < N; c++) {
-        float x = v[c];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) s[c][wp] = (double)x;
+        const T x = warp_sum(v[c]);
+        if (lane == 0) s[c][wp] = wide(x);
     }
     __syncthreads();
     if (threadIdx.x < N) {

@@ -1,7 +1,7 @@
 """The dot products of the persistent CG kernels, emulated exactly in FP32 on the CPU: FP32 over the 16 nodes that a
 thread adds first, pairs of FP32 (48 bits) over everything above, scaled by a power of two.  Against FP64 they are no
-further off than the sums of the launch-per-pass kernels (FP32 over a thread and a warp, FP64 above), for as many
-nodes as either form takes, and sums beyond FP32's range stay finite."""
+further off than sums in FP32 over a thread and a warp of 1216 CTAs and FP64 above, and sums beyond FP32's range stay
+finite.  Nor are those of the launch-per-pass kernels, whose threads sum more nodes in fewer CTAs."""
 import numpy as np
 import pytest
 
@@ -49,6 +49,21 @@ def launches(p, ctas=1216):
     return s.astype(np.float64).sum()
 
 
+def launches_in_one_wave(p, ctas):
+    """k_lpcg_k2 (456 CTAs), k_pcg_k2 (760): a thread's groups of four and its warp as pairs, FP64."""
+    threads = 256 * min(ctas, max(1, -(-(len(p) // 4) // 256)))
+    g = serial(pad(p, 4 * threads).reshape(-1, threads, 4).transpose(2, 0, 1))
+    h, l = np.zeros(threads, f32), np.zeros(threads, f32)
+    for t in g:
+        h, e = two_sum(h, t)
+        l = (l + e).astype(f32)
+    h, l = h.reshape(-1, 32), l.reshape(-1, 32)
+    while h.shape[1] > 1:
+        m = h.shape[1] // 2
+        h, l = gather(h[:, :m], l[:, :m], h[:, m:], l[:, m:])
+    return h.astype(np.float64).sum() + l.astype(np.float64).sum()
+
+
 def persistent(p, sms=152, threads=512):
     """k_pcg_grid: a thread's groups of four in turn in FP32, 16 nodes at a time; those, its warp, the warps of its CTA
     and the CTAs as pairs."""
@@ -85,6 +100,20 @@ def test_no_further_from_fp64_than_the_launches(n):
         exact = p.astype(np.float64).sum()
         a.append(launches(p) / exact - 1)
         b.append(persistent(p) / exact - 1)
+    assert np.sqrt(np.mean(np.square(b))) <= np.sqrt(np.mean(np.square(a)))
+
+
+@pytest.mark.parametrize("ctas", [456, 760])
+@pytest.mark.parametrize("n", [1_000_003, 2_146_689, 8_000_000])
+def test_one_wave_of_launches_is_no_further_from_fp64(n, ctas):
+    rng = np.random.default_rng(n)
+    a, b = [], []
+    for _ in range(3):
+        r = (rng.normal(size=n) * np.exp(rng.normal(size=n))).astype(f32)
+        p = (r * r).astype(f32)
+        exact = p.astype(np.float64).sum()
+        a.append(launches(p) / exact - 1)
+        b.append(launches_in_one_wave(p, ctas) / exact - 1)
     assert np.sqrt(np.mean(np.square(b))) <= np.sqrt(np.mean(np.square(a)))
 
 
