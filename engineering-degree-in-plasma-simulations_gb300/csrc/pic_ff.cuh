@@ -42,6 +42,7 @@ __device__ __forceinline__ FF ff_add_f(FF a, float b) {
     FF s = two_sum(a.hi, b);
     return two_sum(s.hi, s.lo + a.lo);
 }
+constexpr int kFp32Nodes = 16;  // nodes at most that a thread sums in FP32 before they join such a sum
 // a + t and a + b for running sums: the high parts by TwoSum, the low parts collected (normalised once at the end)
 __device__ __forceinline__ FF ff_acc(FF a, float t) {
     const FF s = two_sum(a.hi, t);

@@ -355,6 +355,7 @@ __device__ __forceinline__ void row_neighbours(const GridDev& g, int j, int k, i
 // Other grids go node by node, a node a thread (four in turn a thread: 14 us for 21^3 nodes, latency).
 // Capped at 80 registers (three CTAs per SM; a few bytes spill): measured faster than two CTAs at
 // 116 registers or four at 64.
+template <bool ROWS4>
 __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __restrict__ phi_in,
                                                   float2* __restrict__ phi_out, const float* __restrict__ e,
                                                   const float* __restrict__ rho, const uint16_t* __restrict__ kind,
@@ -371,16 +372,18 @@ __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __
     }
     K.ie = FF{kIeHi, kIeLo};
     const bool ae = apply_e != 0;
-    const bool rows4 = (g.ni & 3) == 0;
     const int nij = g.ni * g.nj;
     const float ie_f = kIeHi;
-    float acc_r = 0.f, acc_b = 0.f, acc_s = 0.f;  // per-thread sums in FP32, block and grid sums in FP64
-    const int ngroups = rows4 ? g.nv >> 2 : g.nv;
+    // |r|^2, |b|^2, |rho / eps0|^2: FP32 over a thread's groups, or pairs over its nodes where it has registers left for
+    // them (with groups of four they spill: 281 -> 305 us on 256 x 256 x 512 nodes; in shared memory 342)
+    float f_r = 0.f, f_b = 0.f, f_s = 0.f;
+    FF acc[4] = {FF{0.f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}, FF{0.f, 0.f}};
+    const int ngroups = ROWS4 ? g.nv >> 2 : g.nv;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ngroups; q += gridDim.x * blockDim.x) {
-        const int n0 = rows4 ? q << 2 : q;
+        const int n0 = ROWS4 ? q << 2 : q;
         int i0, j, k;
         node_ijk(g, n0, i0, j, k);
-        if (rows4) {
+        if constexpr (ROWS4) {
             // every group of a row, its ends included: see spmv_group for the x neighbours at the ends
             const bool xend = i0 + 4 == g.ni, wrapx = g.periodic[0] != 0;
             const int ixm = i0 > 0 ? n0 - 1 : (wrapx ? n0 + g.ni - 2 : n0);
@@ -439,10 +442,10 @@ __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __
                 const float en[6] = {c == 0 ? exm : E[c - 1], wr ? exp_ : E[c + 1], EYm[c], EYp[c], EZm[c], EZp[c]};
                 float b;
                 residual_node(K, kv[c], P[c], pn, E[c], en, hv[c], ae, rv[c], b, bf[c], pv[c]);
-                acc_r += rv[c] * rv[c];
-                acc_b += b * b;
+                f_r += rv[c] * rv[c];
+                f_b += b * b;
                 const float sc = hv[c] * ie_f;
-                acc_s += sc * sc;
+                f_s += sc * sc;
             }
             *reinterpret_cast<float4*>(r + n0) = make_float4(rv[0], rv[1], rv[2], rv[3]);
             if (ae) {
@@ -451,10 +454,7 @@ __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __
             }
             if (rho_prev) *reinterpret_cast<float4*>(rho_prev + n0) = h4;
             if (bfix_out) *reinterpret_cast<float4*>(bfix_out + n0) = make_float4(bf[0], bf[1], bf[2], bf[3]);
-            continue;
-        }
-        // node by node
-        {
+        } else {  // node by node
             const int n = n0;
             const uint16_t kd = kind[n];
             if ((kd & 3) != kFree) {
@@ -477,26 +477,38 @@ __global__ void __launch_bounds__(256, 3) k_residual(GridDev g, const float2* __
             residual_node(K, kd, phi_in[n], pn, ae ? e[n] : 0.f, en, rh, ae, rf, b, bfix, np);
             r[n] = rf;
             if (ae) phi_out[n] = np;
-            acc_r += rf * rf;
-            acc_b += b * b;
             const float sc = rh * ie_f;
-            acc_s += sc * sc;
+            acc[0] = ff_acc(acc[0], rf * rf);
+            acc[1] = ff_acc(acc[1], b * b);
+            acc[3] = ff_acc(acc[3], sc * sc);
             if (rho_prev) rho_prev[n] = rh;
             if (bfix_out) bfix_out[n] = bfix;
         }
     }
-    const float v[4] = {acc_r, acc_b, 0.f, acc_s};
-    grid_sum<4>(v, gpart, gstride, ticket, out);
+    if (ROWS4) {
+        acc[0].hi = f_r;
+        acc[1].hi = f_b;
+        acc[3].hi = f_s;
+    }
+    grid_sum<4>(acc, gpart, gstride, ticket, out);
 }
+// One wave where a thread then has kFp32Nodes nodes at most (64 x 64 x 256 nodes 44 -> 35 us with the call's
+// synchronisation) and on rows that go node by node; beyond, as many CTAs as keep a thread's FP32 sums short
+// (256 x 256 x 512 nodes 280 us either way, 300 with the two forms in one kernel, whose registers spill more)
+constexpr int kResidualMost = 1216;
 void launch_residual(const GridDev& g, SolveWork& w, int apply_e, cudaStream_t s, float* rho_prev, float* bfix_out) {
     const float2* in = w.phi;
     float2* out = apply_e ? w.phi_alt : w.phi;
-    const int blocks = (g.ni & 3) && g.node_grid <= 0 ? std::min(kResPerSM * kSms, (g.nv + 255) / 256)
-                                                     : stream_blocks(g, kResPerSM);
-    k_residual<<<blocks, 256, 0, s>>>(g, in, out, w.e, w.rho,
-                                                          reinterpret_cast<const uint16_t*>(w.kind), w.r, w.gpart,
-                                                          w.gstride, w.ticket, w.scal + kS_R2, apply_e, rho_prev,
-                                                          bfix_out);
+    int blocks = stream_blocks(g, kResPerSM);
+    if (g.node_grid <= 0) {
+        if (g.ni & 3)
+            blocks = std::min(kResPerSM * kSms, (g.nv + 255) / 256);
+        else if (g.nv > kFp32Nodes * 256 * blocks)
+            blocks = stream_blocks(g.nv, kResidualMost);
+    }
+    auto kernel = (g.ni & 3) ? k_residual<false> : k_residual<true>;
+    kernel<<<blocks, 256, 0, s>>>(g, in, out, w.e, w.rho, reinterpret_cast<const uint16_t*>(w.kind), w.r, w.gpart,
+                                  w.gstride, w.ticket, w.scal + kS_R2, apply_e, rho_prev, bfix_out);
     if (apply_e) {
         float2* t = w.phi;
         w.phi = w.phi_alt;

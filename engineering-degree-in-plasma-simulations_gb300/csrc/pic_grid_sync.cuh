@@ -89,7 +89,6 @@ __device__ __forceinline__ FF warp_halved(const FF (&x)[N]) {
 // |r|^2 is off by 2.6e-9 at 40 000 nodes and 7.3e-10 at 2.1 million (5.5e-9 and 8.5e-10 with FP32 over a thread and
 // a warp and FP64 above, as in the launch-per-pass kernels).  scale is a power of two that brings the sum near 1: a
 // warp's sum lies in FP32's range, the grid's need not.
-constexpr int kFp32Nodes = 16;
 template <int N, int NT>
 __device__ __forceinline__ bool grid_total(const FF (&v)[N], const float (&scale)[N], float2 (*wsum)[NT / 32],
                                            float2 (*part)[kMostCtas], const GridWait& w, unsigned& target, int* s_fail,
