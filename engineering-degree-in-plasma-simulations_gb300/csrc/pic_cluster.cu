@@ -7,11 +7,12 @@
 // of the grid are split over the CTAs of a cluster, every CTA keeps its planes in shared memory, and
 // the two boundary planes go into the neighbours' halo planes through distributed shared memory as
 // they are computed (st.async: the data and its completion on the receiver's mbarrier in one message, so
-// a CTA waits for its neighbours' planes only, never for a cluster-wide barrier).  Every wait is bounded; a CTA whose wait runs out leaves its loop and joins the others
-// at the closing cluster barrier, so that no CTA's shared memory goes away under a message.
+// a CTA waits for its neighbours' planes only, never for a cluster-wide barrier).  Every wait is bounded; a CTA
+// whose wait runs out leaves its loop and joins the others at the closing cluster barrier, so that no CTA's
+// shared memory goes away under a message.
 //
-// Measured: 25 sweeps of 21^3 nodes 37 us on 16 CTAs (60 on 4, 112 on 1; about 190 as 50 launches), of
-// 60^3 nodes 177 us; a CG iteration of 21^3 nodes 2.7 us, of 31 x 31 x 51 nodes 4.9 us (21 us as two
+// Measured: 25 sweeps of 21^3 nodes 34 us on 16 CTAs (60 on 4, 112 on 1; about 190 as 50 launches), of
+// 31 x 31 x 51 nodes 71 us; a CG iteration of 21^3 nodes 2.8 us, of 31 x 31 x 51 nodes 4.6 us (21 us as two
 // launches).  More CTAs are faster at every size, so the cluster is as large as the GPU allows.
 //
 // The arithmetic of a node is that of k_rbsor and k_pcg_* (pic_fields.cu), in the same order.
@@ -506,9 +507,9 @@ void fill_config(int ctas, int threads, size_t smem, cudaStream_t s, cudaLaunchC
     cfg.numAttrs = 1;
 }
 constexpr size_t kSmemMost = 216 * 1024;  // with the static arrays below the 227 KB of a CTA
-// nodes per CTA up to which one cluster is the faster form: at 45^3 (6075 a CTA) 25 sweeps take 107 us here
-// and 108 us on the whole GPU (pic_persist.cu), a CG iteration 6.7 and 7.4 us; at 31 x 31 x 51 (3844) 75
-// and 104 us, 4.9 and 7.3 us; sweeps of 60^3 (14 400) 161 and 120 us
+// nodes per CTA up to which one cluster is the faster form: at 45^3 (6075 a CTA) 25 sweeps take 101 us here
+// and 108 us on the whole GPU (pic_persist.cu), a CG iteration 6.0 and 7.4 us; at 31 x 31 x 51 (3844) 71
+// and 104 us, 4.6 and 7.3 us; sweeps of 60^3 (14 400) 161 and 116 us
 constexpr long kOwnMost = 6144;
 int stack_planes(const GridDev& g) { return g.periodic[2] ? g.nk - 1 : g.nk; }
 // whether a cluster of the kernel can be resident (its attributes are set here, before any launch)

@@ -247,7 +247,7 @@ inline int node_blocks(int nv) { return (nv + kNodeTile - 1) / kNodeTile; }
 // its warp: a sum of |r|^2 over 33 M nodes is off FP64 by 1e-9 (FP32 over a thread and a warp: 1.3e-8 with 456
 // CTAs, 4e-9 with 1216); 300 Jacobi-PCG iterations of 144^3 9.9 -> 10.5 ms, of 256^3 49 -> 46.
 constexpr int kSms = 152;
-constexpr int kResPerSM = 3;  // residual and learned-CG kernels (80 registers; the others' sums stay short)
+constexpr int kResPerSM = 3;  // residual (up to a size) and learned-CG kernels (80 registers), right-hand-side update
 constexpr int kPcgPerSM = 5;  // Jacobi-PCG kernels (48 registers)
 inline int stream_blocks(int nv, int cap) {
     const int want = (nv / 4 + 255) / 256;

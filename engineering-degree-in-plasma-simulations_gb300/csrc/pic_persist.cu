@@ -11,10 +11,10 @@
 // publication of the writes before it.  (Measured beside it: a flag per CTA that only the neighbours poll
 // 1.5 us at best and 4 us with the flags in one cache line; all CTAs polling all partial sums 2.3 us.)
 //
-// Measured: 25 sweeps of 65 x 65 x 97 nodes 172 us (325 us as 50 launches); a CG iteration of 65 x 65 x 97
-// nodes 7.9 us, of 129^3 nodes 14.4 us (52 us as two launches), of which the three barriers and sums are 6 us.
+// Measured: 25 sweeps of 65 x 65 x 97 nodes 168 us (325 us as 50 launches); a CG iteration of 65 x 65 x 97
+// nodes 8.1 us, of 129^3 nodes 14.7 us (52 us as two launches), of which the three barriers and sums are 6 us.
 //
-// The arithmetic of a node is that of k_rbsor and k_pcg_* (pic_fields.cu), in the same order.
+// The arithmetic of a node is that of k_rbsor and k_pcg_* (pic_fields.cu), in the same order; sums: grid_total.
 #include <algorithm>
 #include "pic_ff.cuh"
 #include "pic_grid_sync.cuh"

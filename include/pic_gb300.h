@@ -347,8 +347,9 @@ int pic_number_density_noalloc(int ni, int nj, int nk, const double* x0, const d
 /* ---- runtime ------------------------------------------------------------------------- */
 int pic_synchronize(pic_world* w);
 /* Test hook, no reference counterpart: how many times a kernel's first wait for a bulk copy
- * (the push) or for tensor-core MMAs (training) polls its mbarrier before it gives up, records
- * the fault and returns (pic_synchronize then returns PIC_ERR_DEVICE).  polls < 0 restores the
+ * (the push) or for tensor-core MMAs (training) polls its mbarrier, or a wait of the Poisson solvers and of
+ * the compaction for their other blocks polls, before it gives up, records the fault and returns
+ * (pic_synchronize, or the call itself, then returns PIC_ERR_DEVICE).  polls < 0 restores the
  * default 2^24; 0 makes every such wait give up at once.  The wait for the copies or MMAs still
  * in flight after a timeout always keeps the full limit, so no copy outlives its block.  The
  * tensor-core setting applies to the current device. */
